@@ -233,14 +233,12 @@ int pmb_stencil_stats(pmb_stencil* s, int image, int* iters, int* status, double
 int64_t pmb_stencil_launch_count(const pmb_stencil* s);
 int pmb_stencil_destroy(pmb_stencil* s);
 /* Launch-shape knobs of the solver, for the autotuner (no counterpart in the
- * reference): 0 vector width of the CG apply (2 or 4 pixels per thread, 4
- * only for the FP32 inner solve), 1 the same for the prolongation, 2/3/4
- * resident CTAs per SM of the level-0 tile kernels / prolongation /
- * restriction (up to the shared-memory limit), 5 CTAs per SM of the
- * element-wise kernels, 6 CG iterations per graph replay, 7 buffers of the
- * CG apply, restriction and prolongation kernels (1, the default: half the
- * shared memory, so twice the CTAs per SM; 2: a tile in flight per CTA;
- * setting it resets knobs 2, 3 and 4 to the new residency limit). Returns
+ * reference): 0 columns per lane of the CG apply (2 or 4, 4 only for the
+ * FP32 inner solve), 1 the same for restriction and prolongation, 2/3/4 CTAs
+ * per SM that the rows of the CG apply / prolongation / restriction are cut
+ * for (up to their residency), 5 CTAs per SM of the element-wise kernels, 6 CG
+ * iterations per graph replay, 7 buffers of the tile kernels (1 is the only
+ * setting; setting it resets knobs 2, 3 and 4 to their limits). Returns
  * the value applied (after clamping) or a negative status. */
 int pmb_stencil_tune(pmb_stencil* s, int knob, int value);
 int pmb_stencil_tuning(const pmb_stencil* s, int knob);

@@ -2,20 +2,17 @@
 
 The knobs (``pmb_stencil_tune`` in the C ABI):
 
-* ``vec_apply`` / ``vec_up`` — pixels per thread of the CG apply and of the
-  prolongation kernel (2 or 4; 4 halves the threads per CTA and the shared
-  loads per pixel, FP32 only);
-* ``ctas_fine`` / ``ctas_up`` / ``ctas_down`` — resident CTAs per SM of the
-  level-0 tile kernels, the prolongation and the restriction (bounded by
-  their shared memory);
+* ``vec_apply`` / ``vec_up`` — columns per lane of the CG apply and of the
+  V-cycle's restriction and prolongation (2 or 4; 4 in FP32 only);
+* ``ctas_fine`` / ``ctas_up`` / ``ctas_down`` — CTAs per SM that the rows of
+  the CG apply, the prolongation and the restriction are cut for (bounded by
+  their registers and shared memory);
 * ``ctas_flat`` — CTAs per SM of the element-wise kernels;
 * ``chunk`` — CG iterations per CUDA-graph replay (the host reads the
   per-image status once per replay);
-* ``stages`` — buffers of the CG apply, restriction and prolongation
-  kernels: 1 (the default: half the shared memory, so twice the CTAs per SM)
-  or 2 (one tile in flight per CTA while another is computed). Setting it
-  resets ``ctas_fine`` / ``ctas_up`` / ``ctas_down`` to the new residency
-  limit, so it is walked first.
+* ``stages`` — buffers of the tile kernels: 1 is the only setting left.
+  Setting it resets ``ctas_fine`` / ``ctas_up`` / ``ctas_down`` to their
+  limits, so it is walked first.
 
 ``autotune(batch)`` times full solves of the batch's own system with CUDA
 events and walks the knobs one at a time (coordinate descent, two passes),
@@ -37,7 +34,7 @@ __all__ = ["KNOBS", "tuning", "apply_tuning", "autotune", "cache_key", "cached"]
 
 KNOBS = {"stages": 7, "vec_apply": 0, "vec_up": 1, "ctas_fine": 2, "ctas_up": 3,
          "ctas_down": 4, "ctas_flat": 5, "chunk": 6}
-CANDIDATES = {"stages": [1, 2], "vec_apply": [2, 4], "vec_up": [2, 4], "ctas_fine": [1, 2, 3, 4],
+CANDIDATES = {"stages": [1], "vec_apply": [2, 4], "vec_up": [2, 4], "ctas_fine": [1, 2, 3, 4],
               "ctas_up": [1, 2, 3, 4], "ctas_down": [1, 2, 3, 4], "ctas_flat": [2, 4, 8, 16],
               "chunk": [2, 4, 8]}
 _MARGIN = 0.02          # a change must win by 2 %

@@ -22,6 +22,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hi
 SOURCES = {
     "cf_assemble.cu": ["-fmad=false"],
     "stencil.cu": [],
+    "stencil_rows.cu": [],
     "csr.cu": [],
     "lkm.cu": [],
     "foreground.cu": [],

@@ -134,6 +134,12 @@ struct HostList {
     WorkList wl{};                   // device view, filled at bind
     const GridDesc* partner_dev = nullptr;
     int per_sm = 8;                  // resident CTAs per SM of the kernels using it
+    // Unit table of the row-streaming kernel that walks this list (-1: none).
+    int rows = -1;
+    std::vector<int4> cta;
+    int64_t cta_cap = 0;             // entries the workspace holds
+    size_t d_cta = 0;
+    RowList R{};                     // device view
 };
 
 struct Level {
@@ -156,17 +162,12 @@ struct Stencil {
     std::vector<int> h, w;
     int precision = 0;   // 0: FP64, 1: FP32 inner + FP64 refinement
     int precond = 0;     // kPrecNone / kPrecJacobi / kPrecVcycle
-    // Launch shapes (pmb_stencil_tune): vector width of the CG apply and of
-    // the prolongation, resident CTAs per SM of each list family (limit:
-    // shared memory), CG iterations per graph replay.
+    // Launch shapes (pmb_stencil_tune): columns per lane of the CG apply and
+    // of the V-cycle kernels, CTAs per SM that each list is cut for, CG
+    // iterations per graph replay.
     int vec_apply = 2, vec_up = 2, chunk = 4;
     int max_fine = 1, max_up = 1, max_down = 1;
     int pre = 1, post = 1;
-    // Buffers of the CG apply, restriction and prolongation kernels: 1 (the
-    // default: half the shared memory, twice the CTAs per SM, measured 14-20 %
-    // faster per solve than 2 on the 64-image batch) or 2 (a tile in flight
-    // per CTA while another is computed).
-    int stages = 1;
     double omega = 0.8;
     int direct = 64;
     int cy = 3;                      // restriction tile height (inner precision)
@@ -210,6 +211,7 @@ struct Stencil {
     double delta = 1e-4;            // mixed: FP32 phase reduction before a residual replacement
     int max_outer = 50;             // mixed: most residual replacements
     int64_t graph_kernels = 0;      // kernel nodes of one graph replay
+    int pass = 0;                   // level-0 passes queued: every other one runs backwards
     bool bound = false, setup_done = false;
     // last solve
     int64_t launches = 0;
@@ -264,7 +266,64 @@ static void build_flat(HostList& L, const std::vector<GridDesc>& grids) {
     }
 }
 
+// Columns per lane of the row-streaming kernel that walks list L.
+static int rows_vec(const Stencil& S, const HostList& L) {
+    return L.rows == kRowsApply ? S.vec_apply : S.vec_up;
+}
+
+// Resident CTAs per SM that a list of this kind may be cut for.
+static int rows_limit(const Stencil& S, int kind, int vec) {
+    stencil_prepare();
+    const int n = S.precision == 1 ? rows_resident_of<float>(kind, vec)
+                                   : rows_resident_of<double>(kind, vec);
+    return std::max(1, std::min(4, n));
+}
+
+// Unit table of list L: the rows of every strip cut into segments, a warp
+// each. A list that fits the resident warps is cut so that it fills one wave
+// of them and no more (a second, thin wave would double its time); a longer
+// one into segments of 32 rows (16 coarse rows), whose two rows of halo cost
+// about 5 % (they come from L2) while the scheduler still balances the waves.
+static void build_rows(HostList& L, int vec) {
+    const int cols = rows_strip(L.rows, vec);
+    const int longest = L.rows == kRowsDown ? 16 : 32;
+    auto units = [&](int seg, bool ctas) {
+        int64_t n = 0;
+        for (const GridDesc& g : L.grids) {
+            const int64_t u = (int64_t)((g.w + cols - 1) / cols) * ((g.h + seg - 1) / seg);
+            n += ctas ? (u + kUnitWarps - 1) / kUnitWarps : u;
+        }
+        return n;
+    };
+    const int64_t slots = (int64_t)148 * L.per_sm;
+    int seg = 1;
+    while (seg < longest && units(seg, true) > slots) ++seg;
+    L.R.seg = seg;
+    L.cta.clear();
+    for (size_t gi = 0; gi < L.grids.size(); ++gi) {
+        const GridDesc& g = L.grids[gi];
+        const int strips = (g.w + cols - 1) / cols;
+        const int n = strips * ((g.h + seg - 1) / seg);
+        for (int u = 0; u < n; u += kUnitWarps) L.cta.push_back(make_int4((int)gi, u, strips, n));
+    }
+    L.R.total = (int)L.cta.size();
+}
+
+// The largest table that any knob setting gives list L.
+static void plan_rows(Stencil& S, HostList& L, int kind) {
+    L.rows = kind;
+    const int per_sm = L.per_sm;
+    for (L.per_sm = 1; L.per_sm <= 4; ++L.per_sm)
+        for (int vec = 2; vec <= (S.precision == 1 ? 4 : 2); vec += 2) {
+            build_rows(L, vec);
+            L.cta_cap = std::max<int64_t>(L.cta_cap, L.R.total);
+        }
+    L.per_sm = per_sm;
+    build_rows(L, rows_vec(S, L));
+}
+
 static void carve_list(Carve& c, HostList& L) {
+    if (L.rows >= 0) L.d_cta = c.take<int4>(L.cta_cap);
     L.d_grids = c.take<GridDesc>((int64_t)L.grids.size());
     L.d_partner = c.take<GridDesc>((int64_t)L.partner.size());
     L.d_starts = c.take<int>((int64_t)L.starts.size());
@@ -346,22 +405,25 @@ static int plan_stencil(Stencil& S) {
         lv.plane_elems = poff;
     }
     S.nmaps = map_base;
+    // Four columns per lane in FP32 once the strips of 120 columns fill the
+    // GPU: measured per iteration, 2 against 4 columns, 139 and 147 us at
+    // 320x240, 155 and 160 at 512x512, 295 and 291 at 1920x1080, 666 and 637
+    // at 3840x2160, 4214 and 3908 on the 73 Mpix of 64 images.
+    if (mixed && S.user_total >= 2000000) S.vec_apply = S.vec_up = 4;
     // Work lists and the residency of the kernels that walk them.
-    const bool vec_up = S.pre == 1 && S.post == 1, vec_down = S.pre == 1;
-    const int per_fine = mixed ? resident_cg_apply<float>(S.vec_apply, S.stages)
-                               : resident_cg_apply<double>(S.vec_apply, S.stages);
-    const int per_up =
-        vec_up ? (mixed ? resident_up<float>(S.vec_up, S.stages)
-                        : resident_up<double>(S.vec_up, S.stages))
-               : blocks_per_sm(mixed ? smem_up<float>(S.pre) : smem_up<double>(S.pre));
+    const bool rows_up = S.pre == 1 && S.post >= 1, rows_down = S.pre == 1;
+    const int per_fine = rows_limit(S, kRowsApply, S.vec_apply);
+    const int per_up = rows_up ? rows_limit(S, kRowsUp, S.vec_up)
+                               : blocks_per_sm(mixed ? smem_up<float>(S.pre) : smem_up<double>(S.pre));
     const int per_down =
-        vec_down ? (mixed ? resident_down<float>(S.stages) : resident_down<double>(S.stages))
-                 : blocks_per_sm(mixed ? smem_down<float>(S.pre) : smem_down<double>(S.pre));
+        rows_down ? rows_limit(S, kRowsDown, S.vec_up)
+                  : blocks_per_sm(mixed ? smem_down<float>(S.pre) : smem_down<double>(S.pre));
     S.max_fine = per_fine;
     S.max_up = per_up;
     S.max_down = per_down;
     build_list(S.fine0, S.levels[0].grids, {}, kTY, kTX);
     S.fine0.per_sm = per_fine;
+    plan_rows(S, S.fine0, kRowsApply);
     build_flat(S.flat0, S.levels[0].grids);
     S.flat0.per_sm = 8;
     for (int l = 0; l + 1 < L; ++l) {
@@ -381,8 +443,10 @@ static int plan_stencil(Stencil& S) {
         build_list(lv.gal, gc, gf, kGalerkinTileY, kGalerkinTileX);   // coarse tiles
         build_list(lv.fine, f, c, kTY, kTX);
         lv.fine.per_sm = per_up;
+        if (rows_up) plan_rows(S, lv.fine, kRowsUp);
         build_list(lv.coarse, c, f, S.cy, kCX);
         lv.coarse.per_sm = per_down;
+        if (rows_down) plan_rows(S, lv.coarse, kRowsDown);
         build_flat(lv.flat, f);
         lv.flat.per_sm = 8;
     }
@@ -409,9 +473,11 @@ static int plan_stencil(Stencil& S) {
     const int64_t v0 = S.levels[0].vec_elems;
     S.o_state = c.take<InstState>(n);
     S.o_outer = c.take<InstState>(n);
-    int64_t maxt = std::max(S.fine0.starts.back(), S.flat0.starts.back());
+    int64_t maxt = std::max<int64_t>(std::max(S.fine0.starts.back(), S.flat0.starts.back()),
+                                     S.fine0.cta_cap);
     for (auto& lv : S.levels) {
         if (!lv.fine.starts.empty()) maxt = std::max<int64_t>(maxt, lv.fine.starts.back());
+        maxt = std::max(maxt, lv.fine.cta_cap);
         if (!lv.flat.starts.empty()) maxt = std::max<int64_t>(maxt, lv.flat.starts.back());
     }
     // Per-CTA partial sums: partials[(image * 3 + q) * G + cta] for the
@@ -492,6 +558,25 @@ static void list_view(Stencil& S, HostList& L) {
     L.wl.ngrids = (int)L.grids.size();
     L.wl.total = L.starts.empty() ? 0 : L.starts.back();
     L.partner_dev = S.at<GridDesc>(L.d_partner);
+    L.R.cta = S.at<int4>(L.d_cta);
+    L.R.grids = L.wl.grids;
+}
+
+static int upload_rows(Stencil& S, HostList& L) {
+    if (!L.cta.empty())
+        PMB_CUDA(cudaMemcpyAsync(S.ws + L.d_cta, L.cta.data(), sizeof(int4) * L.cta.size(),
+                                 cudaMemcpyHostToDevice, S.stream));
+    return 0;
+}
+
+// After a knob of list L changed: its table again.
+static int retune_rows(Stencil& S, HostList& L) {
+    if (L.rows < 0) return 0;
+    build_rows(L, rows_vec(S, L));
+    if (!S.bound) return 0;
+    if (int rc = upload_rows(S, L)) return rc;
+    PMB_CUDA(cudaStreamSynchronize(S.stream));
+    return 0;
 }
 
 static int upload_list(Stencil& S, HostList& L) {
@@ -504,7 +589,7 @@ static int upload_list(Stencil& S, HostList& L) {
     PMB_CUDA(cudaMemcpyAsync(S.ws + L.d_starts, L.starts.data(), sizeof(int) * L.starts.size(),
                              cudaMemcpyHostToDevice, S.stream));
     list_view(S, L);
-    return 0;
+    return upload_rows(S, L);
 }
 
 // Run `fn` on the solver's own stream, ordered after everything already
@@ -553,7 +638,6 @@ static int encode_map(CUtensorMap* out, const void* base, const GridDesc& g, boo
 static int encode_grid_maps(Stencil& S, int l, const GridDesc& g, CUtensorMap* m) {
     const bool mixed = S.precision == 1;
     const int DH = 2 * S.cy + 5;
-    const int DWV = mixed ? down_box_width<float>() : down_box_width<double>();
     Level& lv = S.levels[l];
     const void* P = mixed ? (const void*)planes32(S, l) : (const void*)planes64(S, l);
     const void* B; const void* X; const void* XA = nullptr; const void* XB = nullptr;
@@ -575,14 +659,7 @@ static int encode_grid_maps(Stencil& S, int l, const GridDesc& g, CUtensorMap* m
     rc |= encode_map(m + kMapBD, B, g, false, mixed, kBW, DH);
     rc |= encode_map(m + kMapXC, X, g, false, mixed, kCBW, kCBH);
     rc |= encode_map(m + kMapXF, X, g, false, mixed, kBW, kBH);
-    rc |= encode_map(m + kMapPlS, P, g, true, mixed, kBW, kPH);
-    rc |= encode_map(m + kMapPlDV, P, g, true, mixed, DWV, DH);
-    rc |= encode_map(m + kMapBDV, B, g, false, mixed, DWV, DH);
     rc |= encode_map(m + kMapPlG, planes64(S, l), g, true, false, kGCols, kGRows);
-    rc |= encode_map(m + kMapPlD0, P, g, true, mixed, DWV, DH, 1);
-    rc |= encode_map(m + kMapPlD1, P, g, true, mixed, DWV, DH - 2, kNH - 1);
-    rc |= encode_map(m + kMapPlU0, P, g, true, mixed, kBW, kBH, 1);
-    rc |= encode_map(m + kMapPlU1, P, g, true, mixed, kBW, kPH, kNH - 1);
     if (XA) {
         rc |= encode_map(m + kMapXAF, XA, g, false, mixed, kBW, kBH);
         rc |= encode_map(m + kMapXAD, XA, g, false, mixed, kBW, DH);
@@ -863,8 +940,12 @@ static void run_vcycle(Stencil& S, const T* b0, T* z0, InstState* st, const T* d
             xs_slot_f[l] = in_a ? kMapXAF : kMapXBF;
             xs_slot_d[l] = in_a ? kMapXAD : kMapXBD;
         }
-        launch_vc_down<T>(pre, S.stages, LaunchCfg{persistent_grid(c)}, c.wl, c.partner_dev, S.maps(),
-                          xs_slot_d[l], B(l + 1), om, st, S.err(), s);
+        if (c.rows >= 0)
+            launch_rows_down<T>(rows_vec(S, c), c.R, l == 0 ? S.pass++ & 1 : 0, c.partner_dev,
+                                lvl_P<T>(S, l), B(l), B(l + 1), om, st, s);
+        else
+            launch_vc_down<T>(pre, LaunchCfg{persistent_grid(c)}, c.wl, c.partner_dev, S.maps(),
+                              xs_slot_d[l], B(l + 1), om, st, S.err(), s);
         ++S.launches;
         prof_mark(S, l == 0 ? kPkDown0 : kPkDown);
     }
@@ -894,9 +975,14 @@ static void run_vcycle(Stencil& S, const T* b0, T* z0, InstState* st, const T* d
         const bool first_in_x = (extra % 2 == 0);
         T* first_out = first_in_x ? X(l) : lvl_xa<T>(S, l);
         const bool reduce_here = (l == 0) && st && extra == 0;
-        launch_vc_up<T>(S.vec_up, S.stages, pre, post, Lf, f.wl, f.partner_dev, S.maps(), xs_slot_f[l], B(l),
-                        first_out, om, st, reduce_here ? 1 : 0, dr, reorth, S.partials(), S.err(),
-                        s);
+        if (f.rows >= 0)
+            launch_rows_up<T>(rows_vec(S, f), f.R, l == 0 ? S.pass++ & 1 : 0, f.partner_dev,
+                              lvl_P<T>(S, l), B(l), X(l + 1), first_out, om, st,
+                              reduce_here ? 1 : 0, dr, reorth, S.partials(), s);
+        else
+            launch_vc_up<T>(pre, post, Lf, f.wl, f.partner_dev, S.maps(), xs_slot_f[l], B(l),
+                            first_out, om, st, reduce_here ? 1 : 0, dr, reorth, S.partials(),
+                            S.err(), s);
         ++S.launches;
         prof_mark(S, l == 0 ? kPkUp0 : kPkUp);
         bool cur_x = first_in_x;
@@ -926,10 +1012,8 @@ static void cg_iteration(Stencil& S, int reorth) {
     CgVecs<T> v = cg_vecs<T>(S);
     InstState* st = S.state();
     // Without a preconditioner z is r itself (cg.py:53-55).
-    const int zslot = S.precond == kPrecNone ? kMapBF : kMapZF;
-    launch_cg_apply<T>(S.vec_apply, S.stages, LaunchCfg{persistent_grid(S.fine0)}, S.fine0.wl,
-                       S.maps(), zslot,
-                       v.p0, v.p1, v.ap, st, S.partials(), S.err(), s);
+    launch_rows_apply<T>(S.vec_apply, S.fine0.R, S.pass++ & 1, v.P,
+                         S.precond == kPrecNone ? v.r : v.z, v.p0, v.p1, v.ap, st, S.partials(), s);
     prof_mark(S, kPkApply);
     const bool mixed = S.precision == 1;
     const int upd_grid = std::min(persistent_grid(S.flat0), 148 * resident_cg_update<T>(S.precond));
@@ -985,6 +1069,7 @@ static int iterate(Stencil& S, int reorth, int maxiter) {
         }
         cudaGraph_t g;
         PMB_CUDA(cudaStreamBeginCapture(S.stream, cudaStreamCaptureModeThreadLocal));
+        S.pass = 0;
         for (int i = 0; i < chunk; ++i) cg_iteration<T>(S, reorth);
         PMB_CUDA(cudaStreamEndCapture(S.stream, &g));
         size_t nodes = 0;
@@ -1558,12 +1643,12 @@ PMB_API int pmb_stencil_apply(pmb_stencil* p, const double* x, double* y, void* 
     return on_stream(S, (cudaStream_t)stream, [&]() -> int {
         HostList& a = S.fine0;
         cudaStream_t s = S.stream;
-        double* tx = S.at<double>(S.o_r64);   // level-0 b buffer: map slot kMapBF
+        double* tx = S.at<double>(S.o_r64);
         double* ty = S.at<double>(S.o_ap64);
         launch_pack<double, double>(a.wl.grids, a.wl.ngrids, S.at<int64_t>(S.o_uoff), x, tx,
                                     S.user_total, s);
-        launch_apply<double>(LaunchCfg{grid_for(a, smem_apply_v<double>(2))}, a.wl, S.maps(), ty,
-                             S.err(), s);
+        launch_rows_apply<double>(S.vec_apply, a.R, 0, S.P0, tx, nullptr, nullptr, ty, nullptr,
+                                  nullptr, s);
         launch_unpack<double, double>(a.wl.grids, a.wl.ngrids, S.at<int64_t>(S.o_uoff), ty, y,
                                       S.user_total, s);
         PMB_CUDA(cudaGetLastError());
@@ -1600,32 +1685,46 @@ PMB_API int pmb_stencil_tune(pmb_stencil* p, int knob, int value) {
     const int wide = S.precision == 1 ? 4 : 2;
     auto clampi = [](int v, int lo, int hi) { return std::max(lo, std::min(hi, v)); };
     int applied;
+    auto each = [&](HostList Level::*list) {
+        for (auto& lv : S.levels)
+            if (int rc = retune_rows(S, lv.*list)) return rc;
+        return 0;
+    };
+    int rc = 0;
     switch (knob) {
     case 0:
         applied = S.vec_apply = (value >= 4 ? wide : 2);
-        S.max_fine = S.precision == 1 ? resident_cg_apply<float>(S.vec_apply, S.stages)
-                                      : resident_cg_apply<double>(S.vec_apply, S.stages);
+        S.max_fine = rows_limit(S, kRowsApply, S.vec_apply);
         S.fine0.per_sm = std::min(S.fine0.per_sm, S.max_fine);
+        rc = retune_rows(S, S.fine0);
         break;
     case 1:
         applied = S.vec_up = (value >= 4 ? wide : 2);
-        if (S.pre == 1 && S.post == 1) {
-            S.max_up = S.precision == 1 ? resident_up<float>(S.vec_up, S.stages)
-                                        : resident_up<double>(S.vec_up, S.stages);
+        if (S.pre == 1) {
+            S.max_down = rows_limit(S, kRowsDown, S.vec_up);
+            for (auto& lv : S.levels) lv.coarse.per_sm = std::min(lv.coarse.per_sm, S.max_down);
+            rc = each(&Level::coarse);
+        }
+        if (S.pre == 1 && S.post >= 1) {
+            S.max_up = rows_limit(S, kRowsUp, S.vec_up);
             for (auto& lv : S.levels) lv.fine.per_sm = std::min(lv.fine.per_sm, S.max_up);
+            if (!rc) rc = each(&Level::fine);
         }
         break;
     case 2:
         applied = clampi(value, 1, S.max_fine);
         S.fine0.per_sm = applied;
+        rc = retune_rows(S, S.fine0);
         break;
     case 3:
         applied = clampi(value, 1, S.max_up);
         for (auto& lv : S.levels) lv.fine.per_sm = applied;
+        rc = each(&Level::fine);
         break;
     case 4:
         applied = clampi(value, 1, S.max_down);
         for (auto& lv : S.levels) lv.coarse.per_sm = applied;
+        rc = each(&Level::coarse);
         break;
     case 5:
         applied = clampi(value, 1, kMaxCtasPerSm);
@@ -1633,27 +1732,22 @@ PMB_API int pmb_stencil_tune(pmb_stencil* p, int knob, int value) {
         for (auto& lv : S.levels) lv.flat.per_sm = applied;
         break;
     case 6: applied = S.chunk = clampi(value, 1, 16); break;
-    case 7: {
-        // Buffers of the restriction / prolongation kernels; their CTAs per
-        // SM follow the shared memory of the choice.
-        applied = S.stages = value <= 1 ? 1 : 2;
-        const bool mixed = S.precision == 1;
-        S.max_fine = mixed ? resident_cg_apply<float>(S.vec_apply, S.stages)
-                           : resident_cg_apply<double>(S.vec_apply, S.stages);
+    case 7:
+        // Buffers of the tile kernels: one setting is left; it resets the
+        // CTAs per SM to their limits.
+        applied = 1;
         S.fine0.per_sm = S.max_fine;
-        if (S.pre == 1 && S.post == 1) {
-            S.max_up = mixed ? resident_up<float>(S.vec_up, S.stages)
-                             : resident_up<double>(S.vec_up, S.stages);
-            S.max_down = mixed ? resident_down<float>(S.stages) : resident_down<double>(S.stages);
-            for (auto& lv : S.levels) {
-                lv.fine.per_sm = S.max_up;
-                lv.coarse.per_sm = S.max_down;
-            }
+        rc = retune_rows(S, S.fine0);
+        for (auto& lv : S.levels) {
+            lv.fine.per_sm = S.max_up;
+            lv.coarse.per_sm = S.max_down;
         }
+        if (!rc) rc = each(&Level::fine);
+        if (!rc) rc = each(&Level::coarse);
         break;
-    }
     default: return fail(kErrArg, "pmb_stencil_tune: unknown knob");
     }
+    if (rc) return rc;
     if (S.graph) {
         cudaGraphExecDestroy(S.graph);
         S.graph = nullptr;
@@ -1672,7 +1766,7 @@ PMB_API int pmb_stencil_tuning(const pmb_stencil* p, int knob) {
     case 4: return S.levels.empty() ? 0 : S.levels[0].coarse.per_sm;
     case 5: return S.flat0.per_sm;
     case 6: return S.chunk;
-    case 7: return S.stages;
+    case 7: return 1;
     default: return fail(kErrArg, "pmb_stencil_tuning: unknown knob");
     }
 }
@@ -2533,13 +2627,14 @@ PMB_API int pmb_stencil_time_apply(pmb_stencil* p, int iters, double* ms, void* 
         PMB_CUDA(cudaEventCreate(&e0));
         PMB_CUDA(cudaEventCreate(&e1));
         HostList& a = S.fine0;
-        const LaunchCfg L{grid_for(a, S.precision == 0 ? smem_apply_v<double>(2)
-                                                      : smem_apply_v<float>(2))};
         auto launch = [&]() {
             if (S.precision == 0)
-                launch_apply<double>(L, a.wl, S.maps(), S.at<double>(S.o_ap64), S.err(), S.stream);
+                launch_rows_apply<double>(S.vec_apply, a.R, 0, S.P0, S.at<double>(S.o_r64), nullptr,
+                                          nullptr, S.at<double>(S.o_ap64), nullptr, nullptr, S.stream);
             else
-                launch_apply<float>(L, a.wl, S.maps(), S.at<float>(S.o_ap32), S.err(), S.stream);
+                launch_rows_apply<float>(S.vec_apply, a.R, 0, S.at<float>(S.o_P032),
+                                         S.at<float>(S.o_r32), nullptr, nullptr,
+                                         S.at<float>(S.o_ap32), nullptr, nullptr, S.stream);
         };
         launch();
         PMB_CUDA(cudaEventRecord(e0, S.stream));

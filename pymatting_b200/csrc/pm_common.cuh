@@ -40,9 +40,6 @@ constexpr int kFlat = 8192;
 constexpr int kBOX = 4;
 constexpr int kBW = kTX + 2 * kBOX;   // 72
 constexpr int kBH = kTY + 4;          // 12
-// Plane rows of the register-blocked apply kernels: y0 - 2 .. y0 + 7 (the
-// backward entries reach two rows up; no plane is read below the tile).
-constexpr int kPH = kTY + 2;          // 10
 // Restriction tiles: kCX x CY coarse pixels; the fine box starts at
 // (2 X0 - 4, 2 Y0 - 3) and is kBW x (2 CY + 5).
 constexpr int kCX = 32;
@@ -77,14 +74,7 @@ enum : int {
     kMapP1F,       // CG p parity 1, fine box
     kMapX64F,      // FP64 refinement iterate, fine box
     kMapP64F,      // FP64 planes, fine box (refinement residual)
-    kMapPlS,       // planes, apply box (kPH rows)
-    kMapPlDV,      // planes, register-blocked restriction box
-    kMapBDV,       // b, register-blocked restriction box
     kMapPlG,       // FP64 planes, Galerkin box (42 x 21 x 13)
-    kMapPlD0,      // plane 0, register-blocked restriction box (1 plane)
-    kMapPlD1,      // planes 1..12, restriction box two rows shorter (loaded at plane 1)
-    kMapPlU0,      // plane 0, prolongation box kBW x kBH (1 plane)
-    kMapPlU1,      // planes 1..12, kBW x kPH (loaded at plane 1)
     kMapsPerGrid
 };
 
@@ -267,6 +257,64 @@ __device__ __forceinline__ void cta_flush(double (&v)[NQ], double* partials, int
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < NQ; ++q) v[q] = 0.0;
+}
+
+// V-element vector load / store (8 or 16 bytes, aligned).
+template <typename T, int V>
+__device__ __forceinline__ void ldv(const T* p, T* o) {
+    if constexpr (sizeof(T) == 4 && V == 4) {
+        const float4 q = *reinterpret_cast<const float4*>(p);
+        o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
+    } else if constexpr (sizeof(T) == 4 && V == 2) {
+        const float2 q = *reinterpret_cast<const float2*>(p);
+        o[0] = q.x; o[1] = q.y;
+    } else {
+        static_assert(sizeof(T) == 8 && V == 2, "unsupported vector");
+        const double2 q = *reinterpret_cast<const double2*>(p);
+        o[0] = q.x; o[1] = q.y;
+    }
+}
+
+template <typename T, int V>
+__device__ __forceinline__ void stv(T* p, const T* o) {
+    if constexpr (sizeof(T) == 4 && V == 4) {
+        *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
+    } else if constexpr (sizeof(T) == 4 && V == 2) {
+        *reinterpret_cast<float2*>(p) = make_float2(o[0], o[1]);
+    } else {
+        *reinterpret_cast<double2*>(p) = make_double2(o[0], o[1]);
+    }
+}
+
+__device__ __forceinline__ void finish_beta(InstState* st, double rz_new) {
+    // First pass after the initial residual: only record r.z (cg.py:78-80).
+    if (st->flags & kFirst) {
+        st->rz = rz_new;
+        return;
+    }
+    // beta = (1 / rz) * r.z  (cg.py:105-108)
+    double beta = 1.0 / st->rz;
+    beta *= rz_new;
+    st->beta = beta;
+    st->rz = rz_new;
+}
+
+// beta = ((r - r_old) . z) / rz when reorthogonalising (cg.py:102-104).
+__device__ __forceinline__ void finish_beta_reorth(InstState* st, double rz_new, double dz) {
+    if (st->flags & kFirst) {
+        st->rz = rz_new;
+        return;
+    }
+    st->beta = dz / st->rz;
+    st->rz = rz_new;
+}
+
+// Division in the smoothing sweeps: IEEE in FP64; __fdividef in FP32, where
+// the V-cycle is the inner preconditioner of the mixed solve (convergence is
+// judged on the FP64 residual).
+template <typename T> __device__ __forceinline__ T smooth_div(T a, T b) { return a / b; }
+template <> __device__ __forceinline__ float smooth_div<float>(float a, float b) {
+    return __fdividef(a, b);
 }
 
 }  // namespace pmb

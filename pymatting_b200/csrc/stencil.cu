@@ -53,34 +53,6 @@ struct Buf2 {
     __device__ __forceinline__ T* operator[](int b) const { return p0 + b * d; }
 };
 
-// V-element vector load / store (8 or 16 bytes, aligned).
-template <typename T, int V>
-__device__ __forceinline__ void ldv(const T* p, T* o) {
-    if constexpr (sizeof(T) == 4 && V == 4) {
-        const float4 q = *reinterpret_cast<const float4*>(p);
-        o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
-    } else if constexpr (sizeof(T) == 4 && V == 2) {
-        const float2 q = *reinterpret_cast<const float2*>(p);
-        o[0] = q.x; o[1] = q.y;
-    } else {
-        static_assert(sizeof(T) == 8 && V == 2, "unsupported vector");
-        const double2 q = *reinterpret_cast<const double2*>(p);
-        o[0] = q.x; o[1] = q.y;
-    }
-}
-
-template <typename T, int V>
-__device__ __forceinline__ void stv(T* p, const T* o) {
-    if constexpr (sizeof(T) == 4 && V == 4) {
-        *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
-    } else if constexpr (sizeof(T) == 4 && V == 2) {
-        *reinterpret_cast<float2*>(p) = make_float2(o[0], o[1]);
-    } else {
-        *reinterpret_cast<double2*>(p) = make_double2(o[0], o[1]);
-    }
-}
-
-
 // Description of one tile, prepared by thread 0 for the whole CTA.
 struct Meta {
     int t, g, y0, x0;     // tile, grid index in the list, tile origin
@@ -338,55 +310,6 @@ __device__ __forceinline__ void tile_loop(const WorkList& wl, const InstState* s
     }
 }
 
-// Single-buffer variant of tile_loop: the tile's loads are issued when the
-// previous tile is done, so a CTA has at most one tile in flight and needs
-// half the shared memory; several CTAs per SM then overlap each other's
-// loads and compute.
-template <int H, int W, int GATE = kGateRunning, typename Issue, typename Body, typename Flush>
-__device__ __forceinline__ void tile_loop1(const WorkList& wl, const InstState* st, Pipe& pipe,
-                                           Meta* s_m, GridDesc* s_g, Issue issue, Body body,
-                                           Flush flush) {
-    __shared__ TileDir D;
-    __shared__ int s_tn, s_gn, s_ninst, s_abort;   // the tile after the current one
-    if (threadIdx.x == 0) s_abort = 0;
-    dir_load<GATE>(D, wl, st);
-    unsigned int mine = 0;
-    if (threadIdx.x == 0) s_tn = next_running_tile<GATE>(D, wl, st, blockIdx.x, &s_gn);
-    __syncthreads();
-    int t = s_tn;
-    int g = s_gn;
-    __syncthreads();
-    while (t < wl.total) {
-        if (threadIdx.x == 0) {
-            dir_meta<H, W>(D, wl, st, t, g, s_m[0], s_g[0]);
-            fence_proxy_async();
-            issue(s_m[0], s_g[0], 0);
-            int gn;
-            const int tn = next_running_tile<GATE>(D, wl, st, t + (int)gridDim.x, &gn);
-            s_tn = tn;
-            s_gn = gn;
-            s_ninst = tn < wl.total ? (D.n ? D.g[gn].inst : wl.grids[gn].inst) : -1;
-        }
-        __syncthreads();
-        const Meta m = s_m[0];
-        const int tn = s_tn, gn = s_gn, ninst = s_ninst;
-        if (!pipe.wait(0)) s_abort = 1;
-        body(m, s_g[0], 0);
-        ++mine;
-        if (ninst != m.inst) {
-            flush(m, mine);
-            mine = 0;
-        }
-        __syncthreads();
-        if (s_abort) {
-            pipe.drain(0, false);
-            return;
-        }
-        t = tn;
-        g = gn;
-    }
-}
-
 struct NoFlush {
     __device__ void operator()(const Meta&, unsigned int) const {}
 };
@@ -394,29 +317,6 @@ struct NoFlush {
 // --------------------------------------------------------------------------
 // Conjugate gradient steps (cg.py:64-117)
 // --------------------------------------------------------------------------
-
-__device__ __forceinline__ void finish_beta(InstState* st, double rz_new) {
-    // First pass after the initial residual: only record r.z (cg.py:78-80).
-    if (st->flags & kFirst) {
-        st->rz = rz_new;
-        return;
-    }
-    // beta = (1 / rz) * r.z  (cg.py:105-108)
-    double beta = 1.0 / st->rz;
-    beta *= rz_new;
-    st->beta = beta;
-    st->rz = rz_new;
-}
-
-// beta = ((r - r_old) . z) / rz when reorthogonalising (cg.py:102-104).
-__device__ __forceinline__ void finish_beta_reorth(InstState* st, double rz_new, double dz) {
-    if (st->flags & kFirst) {
-        st->rz = rz_new;
-        return;
-    }
-    st->beta = dz / st->rz;
-    st->rz = rz_new;
-}
 
 // r = b - A x0 (or r = b), |b|, |r|, and for Jacobi / no preconditioner also
 // z and r.z. Finaliser sets norm_b, tol, status (cg.py:64-80). x0 arrives in
@@ -502,75 +402,6 @@ k_cg_init(WorkList wl, const CUtensorMap* maps, const T* __restrict__ P, const T
     };
     // Every image starts from scratch: its tiles run whatever its status.
     tile_loop<kTY, kTX>(wl, nullptr, pipe, s_m, s_g, issue, body, flush);
-}
-
-// p_new = z + beta p_old (p_new = z on the first pass), Ap = A p_new and
-// p_new . Ap; finaliser: alpha = rz / (p . Ap)   (cg.py:85-90, 111-113).
-// p is double-buffered by iteration parity: neighbouring tiles still read
-// p_old while this tile writes p_new. zslot selects z (r without a
-// preconditioner).
-template <typename T>
-__global__ void __launch_bounds__(kTileThreads)
-k_cg_apply(WorkList wl, const CUtensorMap* maps, int zslot, T* p0, T* p1, T* Ap, InstState* st,
-           double* partials, int* err) {
-    __shared__ double s_red[32];
-    __shared__ __align__(8) uint64_t s_bar[2];
-    __shared__ Meta s_m[2];
-    __shared__ GridDesc s_g[2];
-    SmemCarve sc(g_smem);
-    T* sP_[2];
-    T* sZ_[2];
-    T* sQ_[2];
-    for (int k = 0; k < 2; ++k) {
-        sP_[k] = sc.take<T>(kNH * kBH * kBW);
-        sZ_[k] = sc.take<T>(kBH * kBW);
-        sQ_[k] = sc.take<T>(kBH * kBW);
-    }
-    const Buf2<T> sP{sP_[0], sP_[1] - sP_[0]};
-    const Buf2<T> sZ{sZ_[0], sZ_[1] - sZ_[0]};
-    const Buf2<T> sQ{sQ_[0], sQ_[1] - sQ_[0]};
-    Pipe pipe;
-    pipe.init(s_bar, err);
-    double v[1] = {0.0};
-    auto issue = [&](const Meta& m, const GridDesc& g, int bb) {
-        mbar_expect_tx(&pipe.bar[bb], (kNH + (m.first ? 1 : 2)) * kBH * kBW * sizeof(T));
-        tma_load_3d(sP[bb], map_of(maps, g, kMapPlF), m.x0 - kBOX, m.y0 - 2, 0, &pipe.bar[bb]);
-        tma_load_2d(sZ[bb], map_of(maps, g, zslot), m.x0 - kBOX, m.y0 - 2, &pipe.bar[bb]);
-        if (!m.first)
-            tma_load_2d(sQ[bb], map_of(maps, g, m.par ? kMapP1F : kMapP0F), m.x0 - kBOX, m.y0 - 2,
-                        &pipe.bar[bb]);
-    };
-    auto body = [&](const Meta& m, const GridDesc& g, int bb) {
-        T* Z = sZ[bb];
-        if (!m.first) {
-            const T beta = (T)m.beta;
-            const T* Q = sQ[bb];
-            for (int q = threadIdx.x; q < kBH * kBW; q += blockDim.x) Z[q] = Z[q] + beta * Q[q];
-            __syncthreads();
-        }
-        T* pnew = m.par ? p0 : p1;
-        {
-            const int lx = threadIdx.x & 63, ly = threadIdx.x >> 6;
-            const int y = m.y0 + ly, x = m.x0 + lx;
-            if (y < g.h && x < g.w) {
-                const int64_t i = g.voff + (int64_t)y * g.pitch + x;
-                const T pi = Z[(ly + 2) * kBW + lx + kBOX];
-                const T api = stencil_at<T>(sP[bb], kBH, Z, ly + 2, lx + kBOX);
-                pnew[i] = pi;
-                Ap[i] = api;
-                v[0] += (double)pi * (double)api;
-            }
-        }
-    };
-    auto flush = [&](const Meta& m, unsigned int mine) {
-        InstState* s = st + m.inst;
-        cta_flush<1>(v, partials, m.inst, m.t0, m.t1, mine, s, s_red, [&](double* sum) {
-            s->pap = sum[0];
-            s->alpha = s->rz / sum[0];
-            s->flags &= ~kFirst;
-        });
-    };
-    tile_loop<kTY, kTX>(wl, st, pipe, s_m, s_g, issue, body, flush);
 }
 
 // Element-wise loop over a flat work list (kFlat-element chunks) with the same
@@ -772,7 +603,6 @@ k_vc_down(WorkList wl /* coarse tiles */, const GridDesc* fine, const CUtensorMa
     const Buf2<T> sP{sP_[0], sP_[1] - sP_[0]};
     const Buf2<T> sB{sB_[0], sB_[1] - sB_[0]};
     const Buf2<T> sS{sS_[0], sS_[1] - sS_[0]};
-    T* sX = PRE == 1 ? sc.take<T>(DH * kBW) : nullptr;
     T* sR = sc.take<T>(RH * RW);
     Pipe pipe;
     pipe.init(s_bar, err);
@@ -789,18 +619,7 @@ k_vc_down(WorkList wl /* coarse tiles */, const GridDesc* fine, const CUtensorMa
         const GridDesc gf = fine[m.g];
         const int bx = 2 * m.x0 - 4, by = 2 * m.y0 - 3;
         const T* B = sB[bb];
-        const T* X1 = PRE > 1 ? sS[bb] : sX;
-        if (PRE == 1) {
-            // x1 = omega b / d inside the image, 0 outside.
-            for (int q = threadIdx.x; q < DH * kBW; q += blockDim.x) {
-                const int rr = q / kBW, cc = q - rr * kBW;
-                const int fy = by + rr, fx = bx + cc;
-                T v = T(0);
-                if (fy >= 0 && fy < gf.h && fx >= 0 && fx < gf.w) v = (T)omega * B[q] / sP[bb][q];
-                sX[q] = v;
-            }
-            __syncthreads();
-        }
+        const T* X1 = sS[bb];
         for (int q = threadIdx.x; q < RH * RW; q += blockDim.x) {
             const int rr = q / RW, cc = q - rr * RW;
             const int br = rr + 2, bcol = cc + 3;           // box coordinates
@@ -1028,42 +847,6 @@ __global__ void k_vc_direct(const DirectDesc* dd, int count, const T* __restrict
         block_sum<1>(v, s_red);
         if (threadIdx.x == 0) finish_beta(s, v[0]);
     }
-}
-
-// y = A x on pitched vectors (no reductions): used by A.dot(x) and by the
-// benchmark's apply timing. x is the level-0 b buffer (map slot kMapBF).
-template <typename T>
-__global__ void __launch_bounds__(kTileThreads)
-k_apply(WorkList wl, const CUtensorMap* maps, T* y, int* err) {
-    __shared__ __align__(8) uint64_t s_bar[2];
-    __shared__ Meta s_m[2];
-    __shared__ GridDesc s_g[2];
-    SmemCarve sc(g_smem);
-    T* sP_[2];
-    T* sX_[2];
-    for (int k = 0; k < 2; ++k) {
-        sP_[k] = sc.take<T>(kNH * kBH * kBW);
-        sX_[k] = sc.take<T>(kBH * kBW);
-    }
-    const Buf2<T> sP{sP_[0], sP_[1] - sP_[0]};
-    const Buf2<T> sX{sX_[0], sX_[1] - sX_[0]};
-    Pipe pipe;
-    pipe.init(s_bar, err);
-    auto issue = [&](const Meta& m, const GridDesc& g, int bb) {
-        mbar_expect_tx(&pipe.bar[bb], (kNH + 1) * kBH * kBW * sizeof(T));
-        tma_load_3d(sP[bb], map_of(maps, g, kMapPlF), m.x0 - kBOX, m.y0 - 2, 0, &pipe.bar[bb]);
-        tma_load_2d(sX[bb], map_of(maps, g, kMapBF), m.x0 - kBOX, m.y0 - 2, &pipe.bar[bb]);
-    };
-    auto body = [&](const Meta& m, const GridDesc& g, int bb) {
-        {
-            const int lx = threadIdx.x & 63, ly = threadIdx.x >> 6;
-            const int yy = m.y0 + ly, xx = m.x0 + lx;
-            if (yy < g.h && xx < g.w)
-                y[g.voff + (int64_t)yy * g.pitch + xx] =
-                    stencil_at<T>(sP[bb], kBH, sX[bb], ly + 2, lx + kBOX);
-        }
-    };
-    tile_loop<kTY, kTX>(wl, nullptr, pipe, s_m, s_g, issue, body, NoFlush());
 }
 
 // --------------------------------------------------------------------------
@@ -1494,465 +1277,6 @@ k_refine_correct(WorkList wl, double* x64, float* x32, const InstState* st, cons
 
 
 // --------------------------------------------------------------------------
-// Register-blocked kernels
-// --------------------------------------------------------------------------
-//
-// Each thread computes V adjacent pixels of a row (V = 2 or 4 in FP32, 2 in
-// FP64: one 8- or 16-byte shared-memory vector). The operand window of the 25-point
-// stencil is held in registers (5 rows x 3 vectors) and every plane is read
-// with vector loads, so a pixel costs ~12 (FP32) or ~25 (FP64) shared loads
-// instead of 50. The accumulation order per pixel is that of stencil_at, so
-// the results are bit-identical to the one-pixel-per-thread kernels.
-
-// Threads of the 64x8-tile kernels: one V-pixel group each.
-template <int V> __host__ __device__ constexpr int tile_threads_v() { return kTX / V * kTY; }
-// Threads of the restriction kernel (grid-stride over its work items).
-constexpr int kDownThreads = 256;
-
-// (A x) for the V pixels at box row r, box columns c0 .. c0 + V - 1 (c0 a
-// multiple of V, c0 >= V). P: 13 planes of BW-wide rows, `ps` elements apart,
-// row 0 = two rows above the first output row of the tile; loadx(row, col, o)
-// loads V operand values at an aligned box position. Needs rows r-2 .. r+2 of
-// the operand, r-2 .. r of the planes, columns c0 - V .. c0 + 2V - 1.
-// Plane 0 and planes 1..12 may lie in separate boxes with the same first
-// row: plane 0 at P0, plane p >= 1 at P1 + (p - 1) ps1 (BW-wide rows).
-template <typename T, int V, int BW, typename LoadX>
-__device__ __forceinline__ void stencil_split(const T* P0, const T* P1, int ps1, LoadX loadx,
-                                              int r, int c0, T (&acc)[V]) {
-    T xr[5][3 * V];
-#pragma unroll
-    for (int k = 0; k < 5; ++k)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) loadx(r - 2 + k, c0 - V + j * V, &xr[k][j * V]);
-    T pc[V];
-    ldv<T, V>(P0 + r * BW + c0, pc);
-    // FP32: forward and backward terms in two independent chains (half the
-    // dependent-FMA latency per pixel). FP64 keeps one chain in the original
-    // order, which its iteration-count parity with the reference rests on.
-    constexpr bool kSplit = sizeof(T) == 4;
-    T accb[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-        acc[v] = pc[v] * xr[2][V + v];
-        accb[v] = T(0);
-    }
-#pragma unroll
-    for (int p = 1; p < kNH; ++p) {
-        const int dy = half_dy(p), dx = half_dx(p);
-        const T* Pp = P1 + (p - 1) * ps1;
-        T pf[V];
-        ldv<T, V>(Pp + r * BW + c0, pf);
-        // Backward entries A[i, i - d] = plane p at (r - dy, c - dx): an
-        // aligned window of one or two vectors around c0 - dx.
-        T pb[2 * V];
-        const int cb = dx > 0 ? c0 - V : c0;
-        ldv<T, V>(Pp + (r - dy) * BW + cb, pb);
-        if (dx != 0) ldv<T, V>(Pp + (r - dy) * BW + cb + V, pb + V);
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            acc[v] += pf[v] * xr[2 + dy][V + v + dx];
-            if (kSplit) accb[v] += pb[(dx > 0 ? V : 0) + v - dx] * xr[2 - dy][V + v - dx];
-            else acc[v] += pb[(dx > 0 ? V : 0) + v - dx] * xr[2 - dy][V + v - dx];
-        }
-    }
-    if (kSplit) {
-#pragma unroll
-        for (int v = 0; v < V; ++v) acc[v] += accb[v];
-    }
-}
-
-template <typename T, int V, int BW, typename LoadX>
-__device__ __forceinline__ void stencil_vec(const T* P, int ps, LoadX loadx, int r, int c0,
-                                            T (&acc)[V]) {
-    stencil_split<T, V, BW>(P, P + ps, ps, loadx, r, c0, acc);
-}
-
-// Division in the smoothing sweeps: IEEE in FP64; __fdividef in FP32, where
-// the V-cycle is the inner preconditioner of the mixed solve (convergence is
-// judged on the FP64 residual).
-template <typename T> __device__ __forceinline__ T smooth_div(T a, T b) { return a / b; }
-template <> __device__ __forceinline__ float smooth_div<float>(float a, float b) {
-    return __fdividef(a, b);
-}
-
-// y = A x (pitched vectors, no reductions). Plane box: rows y0-2 .. y0+7
-// (kMapPlS), operand box 72 x 12 (kMapBF).
-template <typename T, int V>
-__global__ void __launch_bounds__(tile_threads_v<V>())
-k_apply_v(WorkList wl, const CUtensorMap* maps, T* y, int* err) {
-    constexpr int TPR = kTX / V;
-    __shared__ __align__(8) uint64_t s_bar[2];
-    __shared__ Meta s_m[2];
-    __shared__ GridDesc s_g[2];
-    SmemCarve sc(g_smem);
-    T* sP_[2];
-    T* sX_[2];
-    for (int k = 0; k < 2; ++k) {
-        sP_[k] = sc.take<T>(kNH * kPH * kBW);
-        sX_[k] = sc.take<T>(kBH * kBW);
-    }
-    const Buf2<T> sP{sP_[0], sP_[1] - sP_[0]};
-    const Buf2<T> sX{sX_[0], sX_[1] - sX_[0]};
-    Pipe pipe;
-    pipe.init(s_bar, err);
-    auto issue = [&](const Meta& m, const GridDesc& g, int bb) {
-        mbar_expect_tx(&pipe.bar[bb], (kNH * kPH + kBH) * kBW * sizeof(T));
-        tma_load_3d(sP[bb], map_of(maps, g, kMapPlS), m.x0 - kBOX, m.y0 - 2, 0, &pipe.bar[bb]);
-        tma_load_2d(sX[bb], map_of(maps, g, kMapBF), m.x0 - kBOX, m.y0 - 2, &pipe.bar[bb]);
-    };
-    auto body = [&](const Meta& m, const GridDesc& g, int bb) {
-        const int tx = threadIdx.x % TPR, ty = threadIdx.x / TPR;
-        const int yy = m.y0 + ty, xx = m.x0 + V * tx;
-        if (yy < g.h && xx < g.w) {
-            const T* X = sX[bb];
-            T acc[V];
-            stencil_vec<T, V, kBW>(sP[bb], kPH * kBW,
-                                [&](int rr, int cc, T* o) { ldv<T, V>(X + rr * kBW + cc, o); },
-                                ty + 2, kBOX + V * tx, acc);
-#pragma unroll
-            for (int v = 0; v < V; ++v)
-                if (xx + v >= g.w) acc[v] = T(0);
-            stv<T, V>(y + g.voff + (int64_t)yy * g.pitch + xx, acc);
-        }
-    };
-    tile_loop<kTY, kTX>(wl, nullptr, pipe, s_m, s_g, issue, body, NoFlush());
-}
-
-// p_new = z + beta p_old (z on the first pass), Ap = A p_new, p_new . Ap;
-// finaliser alpha = rz / (p . Ap) (cg.py:85-90, 111-113). p_new is formed
-// in registers from the z and p_old boxes.
-template <typename T, int V, int NST>
-__global__ void __launch_bounds__(tile_threads_v<V>())
-k_cg_apply_v(WorkList wl, const CUtensorMap* maps, int zslot, T* p0, T* p1, T* Ap, InstState* st,
-             double* partials, int* err) {
-    constexpr int TPR = kTX / V;
-    __shared__ double s_red[32];
-    __shared__ __align__(8) uint64_t s_bar[2];
-    __shared__ Meta s_m[2];
-    __shared__ GridDesc s_g[2];
-    SmemCarve sc(g_smem);
-    T* sP_[2];
-    T* sZ_[2];
-    T* sQ_[2];
-    for (int k = 0; k < NST; ++k) {
-        sP_[k] = sc.take<T>(kNH * kPH * kBW);
-        sZ_[k] = sc.take<T>(kBH * kBW);
-        sQ_[k] = sc.take<T>(kBH * kBW);
-    }
-    if (NST == 1) {
-        sP_[1] = sP_[0];
-        sZ_[1] = sZ_[0];
-        sQ_[1] = sQ_[0];
-    }
-    const Buf2<T> sP{sP_[0], sP_[1] - sP_[0]};
-    const Buf2<T> sZ{sZ_[0], sZ_[1] - sZ_[0]};
-    const Buf2<T> sQ{sQ_[0], sQ_[1] - sQ_[0]};
-    Pipe pipe;
-    pipe.init(s_bar, err);
-    double v0[1] = {0.0};
-    auto issue = [&](const Meta& m, const GridDesc& g, int bb) {
-        mbar_expect_tx(&pipe.bar[bb], (kNH * kPH + (m.first ? 1 : 2) * kBH) * kBW * sizeof(T));
-        tma_load_3d(sP[bb], map_of(maps, g, kMapPlS), m.x0 - kBOX, m.y0 - 2, 0, &pipe.bar[bb]);
-        tma_load_2d(sZ[bb], map_of(maps, g, zslot), m.x0 - kBOX, m.y0 - 2, &pipe.bar[bb]);
-        if (!m.first)
-            tma_load_2d(sQ[bb], map_of(maps, g, m.par ? kMapP1F : kMapP0F), m.x0 - kBOX, m.y0 - 2,
-                        &pipe.bar[bb]);
-    };
-    auto body = [&](const Meta& m, const GridDesc& g, int bb) {
-        const int tx = threadIdx.x % TPR, ty = threadIdx.x / TPR;
-        const int yy = m.y0 + ty, xx = m.x0 + V * tx;
-        if (yy < g.h && xx < g.w) {
-            const T* Z = sZ[bb];
-            const T* Q = sQ[bb];
-            const bool first = m.first != 0;
-            const T beta = (T)m.beta;
-            auto loadp = [&](int rr, int cc, T* o) {
-                ldv<T, V>(Z + rr * kBW + cc, o);
-                if (!first) {
-                    T q[V];
-                    ldv<T, V>(Q + rr * kBW + cc, q);
-#pragma unroll
-                    for (int v = 0; v < V; ++v) o[v] = o[v] + beta * q[v];
-                }
-            };
-            T acc[V], pv[V];
-            stencil_vec<T, V, kBW>(sP[bb], kPH * kBW, loadp, ty + 2, kBOX + V * tx, acc);
-            loadp(ty + 2, kBOX + V * tx, pv);
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                if (xx + v >= g.w) {
-                    acc[v] = T(0);
-                    pv[v] = T(0);
-                }
-                v0[0] += (double)pv[v] * (double)acc[v];
-            }
-            const int64_t i = g.voff + (int64_t)yy * g.pitch + xx;
-            stv<T, V>((m.par ? p0 : p1) + i, pv);
-            stv<T, V>(Ap + i, acc);
-        }
-    };
-    auto flush = [&](const Meta& m, unsigned int mine) {
-        InstState* s = st + m.inst;
-        cta_flush<1>(v0, partials, m.inst, m.t0, m.t1, mine, s, s_red, [&](double* sum) {
-            s->pap = sum[0];
-            s->alpha = s->rz / sum[0];
-            s->flags &= ~kFirst;
-        });
-    };
-    if (NST == 2) tile_loop<kTY, kTX>(wl, st, pipe, s_m, s_g, issue, body, flush);
-    else tile_loop1<kTY, kTX>(wl, st, pipe, s_m, s_g, issue, body, flush);
-}
-
-// Restriction box of the register-blocked restriction kernel: fine columns
-// from 2 X0 - DOFF, DW wide; rows 2 Y0 - 3 .. 2 Y0 + 2 CY + 1.
-template <typename T, int VV> struct DownBox {
-    static constexpr int V = VV;
-    static constexpr int CY = Coarse<T>::CY;
-    static constexpr int DH = 2 * CY + 5;
-    static constexpr int DOFF = 2 * V;
-    static constexpr int DW = kTX + DOFF + 4;      // 76 (FP32), 72 (FP64)
-    static constexpr int RH = 2 * CY + 1;          // residual rows
-    static constexpr int RW = kTX + V;             // residual columns from 2 X0 - V
-};
-
-// One pre-smoothing sweep from zero, residual and full-weighting restriction
-// (vcycle.py:33-36, 77-80; same arithmetic as k_vc_down<T, 1>):
-//   x1 = omega b / d on the box, res = b - A x1 on the fine rows
-//   2 Y0 - 1 .. 2 Y0 + 2 CY - 1, b_coarse = R res.
-// NST: 2 buffers (a tile in flight while the previous one is computed) or 1
-// (half the shared memory, twice the CTAs per SM). Plane 0 (the diagonal of
-// the sweep over the whole box) is loaded on DH rows, planes 1..12 (only
-// the residual rows' backward entries) on DH - 2.
-template <typename T, int V, int NST>
-__global__ void __launch_bounds__(kDownThreads)
-k_vc_down_v(WorkList wl /* coarse tiles */, const GridDesc* fine, const CUtensorMap* maps, T* bc,
-            double omega, const InstState* st, int* err) {
-    using D = DownBox<T, V>;
-    constexpr int DH = D::DH, DW = D::DW, RH = D::RH, RW = D::RW, CY = D::CY;
-    constexpr int RV = RW / V, XV = DW / V;
-    __shared__ __align__(8) uint64_t s_bar[2];
-    __shared__ Meta s_m[2];
-    __shared__ GridDesc s_g[2];
-    SmemCarve sc(g_smem);
-    T* sP0_[2];
-    T* sP1_[2];
-    T* sB_[2];
-    for (int k = 0; k < NST; ++k) {
-        sP0_[k] = sc.take<T>(DH * DW);
-        sP1_[k] = sc.take<T>((kNH - 1) * (DH - 2) * DW);
-        sB_[k] = sc.take<T>(DH * DW);
-    }
-    if (NST == 1) {
-        sP0_[1] = sP0_[0];
-        sP1_[1] = sP1_[0];
-        sB_[1] = sB_[0];
-    }
-    const Buf2<T> sP0{sP0_[0], sP0_[1] - sP0_[0]};
-    const Buf2<T> sP1{sP1_[0], sP1_[1] - sP1_[0]};
-    const Buf2<T> sB{sB_[0], sB_[1] - sB_[0]};
-    T* sX = sc.take<T>(DH * DW);
-    T* sR = sc.take<T>(RH * RW);
-    Pipe pipe;
-    pipe.init(s_bar, err);
-    auto issue = [&](const Meta& m, const GridDesc& gc, int bb) {
-        const GridDesc gf = fine[m.g];
-        const int bx = 2 * m.x0 - D::DOFF, by = 2 * m.y0 - 3;
-        mbar_expect_tx(&pipe.bar[bb], (2 * DH + (kNH - 1) * (DH - 2)) * DW * sizeof(T));
-        tma_load_3d(sP0[bb], map_of(maps, gf, kMapPlD0), bx, by, 0, &pipe.bar[bb]);
-        tma_load_3d(sP1[bb], map_of(maps, gf, kMapPlD1), bx, by, 1, &pipe.bar[bb]);
-        tma_load_2d(sB[bb], map_of(maps, gf, kMapBDV), bx, by, &pipe.bar[bb]);
-    };
-    auto body = [&](const Meta& m, const GridDesc& gc, int bb) {
-        const GridDesc gf = fine[m.g];
-        const int bx = 2 * m.x0 - D::DOFF, by = 2 * m.y0 - 3;
-        const T* B = sB[bb];
-        const T* P = sP0[bb];
-        const T* P1 = sP1[bb];
-        for (int q = threadIdx.x; q < DH * XV; q += kDownThreads) {
-            const int rr = q / XV, col = (q - rr * XV) * V;
-            const int fy = by + rr;
-            T bv[V], dv[V], o[V];
-            ldv<T, V>(B + rr * DW + col, bv);
-            ldv<T, V>(P + rr * DW + col, dv);
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                const int fx = bx + col + v;
-                o[v] = (fy >= 0 && fy < gf.h && fx >= 0 && fx < gf.w)
-                           ? smooth_div<T>((T)omega * bv[v], dv[v]) : T(0);
-            }
-            stv<T, V>(sX + rr * DW + col, o);
-        }
-        __syncthreads();
-        for (int q = threadIdx.x; q < RH * RV; q += kDownThreads) {
-            const int rr = q / RV, cv = q - rr * RV;
-            const int br = rr + 2, bcol = D::DOFF - V + cv * V;
-            const int fy = by + br;
-            T acc[V], bv[V], o[V];
-            stencil_split<T, V, DW>(P, P1, (DH - 2) * DW,
-                                    [&](int r2, int c2, T* out) { ldv<T, V>(sX + r2 * DW + c2, out); },
-                                    br, bcol, acc);
-            ldv<T, V>(B + br * DW + bcol, bv);
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                const int fx = bx + bcol + v;
-                o[v] = (fy >= 0 && fy < gf.h && fx >= 0 && fx < gf.w) ? bv[v] - acc[v] : T(0);
-            }
-            stv<T, V>(sR + rr * RW + cv * V, o);
-        }
-        __syncthreads();
-        for (int q = threadIdx.x; q < kCX * CY; q += kDownThreads) {
-            const int ly = q / kCX, lx = q - ly * kCX;
-            const int Y = m.y0 + ly, X = m.x0 + lx;
-            if (Y < gc.h && X < gc.w) {
-                T sum = T(0);
-#pragma unroll
-                for (int ay = -1; ay <= 1; ++ay)
-#pragma unroll
-                    for (int ax = -1; ax <= 1; ++ax)
-                        sum += (T)(pw(ax) * pw(ay) / 16.0) *
-                               sR[(2 * ly + 1 + ay) * RW + (2 * lx + ax + V)];
-                bc[gc.voff + (int64_t)Y * gc.pitch + X] = sum;
-            }
-        }
-    };
-    if (NST == 2) tile_loop<CY, kCX>(wl, st, pipe, s_m, s_g, issue, body, NoFlush());
-    else tile_loop1<CY, kCX>(wl, st, pipe, s_m, s_g, issue, body, NoFlush());
-}
-
-// Prolongation and one post-smoothing sweep (same arithmetic as
-// k_vc_up<T, 1, 1>): x2 = x1 + P xc on the 72 x 12 box into shared memory,
-// then x3 = x2 + omega (b - A x2) / d for the tile; at level 0 also r . z
-// (and (r - r_old) . z) with beta.
-// NST as in k_vc_down_v. Plane 0 (the diagonal of the first sweep over the
-// whole box) is loaded on kBH rows, planes 1..12 (the post sweep's backward
-// entries) on kPH.
-template <typename T, int V, int NST>
-__global__ void __launch_bounds__(tile_threads_v<V>())
-k_vc_up_v(WorkList wl /* fine tiles */, const GridDesc* coarse, const CUtensorMap* maps,
-          const T* __restrict__ b, T* xout, double omega, InstState* st, int level0,
-          const T* __restrict__ dr, int reorth, double* partials, int* err) {
-    constexpr int TPR = kTX / V, NT = tile_threads_v<V>(), XV = kBW / V;
-    __shared__ double s_red[2 * 32];
-    __shared__ __align__(8) uint64_t s_bar[2];
-    __shared__ Meta s_m[2];
-    __shared__ GridDesc s_g[2];
-    SmemCarve sc(g_smem);
-    T* sP0_[2];
-    T* sP1_[2];
-    T* sB_[2];
-    T* sC_[2];
-    for (int k = 0; k < NST; ++k) {
-        sP0_[k] = sc.take<T>(kBH * kBW);
-        sP1_[k] = sc.take<T>((kNH - 1) * kPH * kBW);
-        sB_[k] = sc.take<T>(kBH * kBW);
-        sC_[k] = sc.take<T>(kCBH * kCBW);
-    }
-    if (NST == 1) {
-        sP0_[1] = sP0_[0];
-        sP1_[1] = sP1_[0];
-        sB_[1] = sB_[0];
-        sC_[1] = sC_[0];
-    }
-    const Buf2<T> sP0{sP0_[0], sP0_[1] - sP0_[0]};
-    const Buf2<T> sP1{sP1_[0], sP1_[1] - sP1_[0]};
-    const Buf2<T> sB{sB_[0], sB_[1] - sB_[0]};
-    const Buf2<T> sC{sC_[0], sC_[1] - sC_[0]};
-    T* sX = sc.take<T>(kBH * kBW);
-    Pipe pipe;
-    pipe.init(s_bar, err);
-    double acc2[2] = {0.0, 0.0};
-    auto issue = [&](const Meta& m, const GridDesc& gf, int bb) {
-        const GridDesc gc = coarse[m.g];
-        mbar_expect_tx(&pipe.bar[bb],
-                       ((2 * kBH + (kNH - 1) * kPH) * kBW + kCBH * kCBW) * sizeof(T));
-        tma_load_3d(sP0[bb], map_of(maps, gf, kMapPlU0), m.x0 - kBOX, m.y0 - 2, 0, &pipe.bar[bb]);
-        tma_load_3d(sP1[bb], map_of(maps, gf, kMapPlU1), m.x0 - kBOX, m.y0 - 2, 1, &pipe.bar[bb]);
-        tma_load_2d(sB[bb], map_of(maps, gf, kMapBF), m.x0 - kBOX, m.y0 - 2, &pipe.bar[bb]);
-        tma_load_2d(sC[bb], map_of(maps, gc, kMapXC), (m.x0 >> 1) - 4, (m.y0 >> 1) - 2,
-                    &pipe.bar[bb]);
-    };
-    auto body = [&](const Meta& m, const GridDesc& gf, int bb) {
-        const int bx = m.x0 - kBOX, by = m.y0 - 2;
-        const int cx0 = (m.x0 >> 1) - 4, cy0 = (m.y0 >> 1) - 2;
-        const T* P = sP0[bb];
-        const T* P1 = sP1[bb];
-        const T* B = sB[bb];
-        const T* C = sC[bb];
-        for (int q = threadIdx.x; q < kBH * XV; q += NT) {
-            const int rr = q / XV, col = (q - rr * XV) * V;
-            const int y = by + rr;
-            T bv[V], dv[V], o[V];
-            ldv<T, V>(B + rr * kBW + col, bv);
-            ldv<T, V>(P + rr * kBW + col, dv);
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                const int x = bx + col + v;
-                T val = T(0);
-                if (y >= 0 && y < gf.h && x >= 0 && x < gf.w) {
-                    const T x1 = smooth_div<T>((T)omega * bv[v], dv[v]);
-                    // Coarse pixels whose 3x3 support holds (y, x), in raster
-                    // order: an even coordinate has one parent (weight 2), an
-                    // odd one two (weight 1). Written without branches: the
-                    // second parent of an even coordinate gets weight 0, and
-                    // parents outside the coarse grid read the zeros the TMA
-                    // box is filled with there, so both add exactly nothing.
-                    const int oy = y & 1, ox = x & 1;
-                    const T* c00 = C + (((y - oy) >> 1) - cy0) * kCBW + (((x - ox) >> 1) - cx0);
-                    const T wy0 = T(2 - oy), wy1 = T(oy), wx0 = T(2 - ox), wx1 = T(ox);
-                    const T s16 = T(0.0625);
-                    T sum = T(0);
-                    sum += (wx0 * wy0 * s16) * c00[0];
-                    sum += (wx1 * wy0 * s16) * c00[ox];
-                    sum += (wx0 * wy1 * s16) * c00[oy * kCBW];
-                    sum += (wx1 * wy1 * s16) * c00[oy * kCBW + ox];
-                    val = x1 + sum;
-                }
-                o[v] = val;
-            }
-            stv<T, V>(sX + rr * kBW + col, o);
-        }
-        __syncthreads();
-        const int tx = threadIdx.x % TPR, ty = threadIdx.x / TPR;
-        const int yy = m.y0 + ty, xx = m.x0 + V * tx;
-        if (yy < gf.h && xx < gf.w) {
-            const int r = ty + 2, c0 = kBOX + V * tx;
-            T ax[V], x2[V], bv[V], dv[V], x3[V];
-            stencil_split<T, V, kBW>(P, P1, kPH * kBW,
-                                     [&](int r2, int c2, T* out) { ldv<T, V>(sX + r2 * kBW + c2, out); },
-                                     r, c0, ax);
-            ldv<T, V>(sX + r * kBW + c0, x2);
-            ldv<T, V>(B + r * kBW + c0, bv);
-            ldv<T, V>(P + r * kBW + c0, dv);
-            const int64_t i = gf.voff + (int64_t)yy * gf.pitch + xx;
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                if (xx + v < gf.w) {
-                    x3[v] = x2[v] + smooth_div<T>((T)omega * (bv[v] - ax[v]), dv[v]);
-                    if (level0) {
-                        acc2[0] += (double)bv[v] * (double)x3[v];
-                        if (reorth) acc2[1] += (double)dr[i + v] * (double)x3[v];
-                    }
-                } else {
-                    x3[v] = T(0);
-                }
-            }
-            stv<T, V>(xout + i, x3);
-        }
-    };
-    auto flush = [&](const Meta& m, unsigned int mine) {
-        if (!level0 || !st) return;
-        InstState* s = st + m.inst;
-        cta_flush<2>(acc2, partials, m.inst, m.t0, m.t1, mine, s, s_red, [&](double* sum) {
-            if (reorth) finish_beta_reorth(s, sum[0], sum[1]);
-            else finish_beta(s, sum[0]);
-        });
-    };
-    if (NST == 2) tile_loop<kTY, kTX>(wl, st, pipe, s_m, s_g, issue, body, flush);
-    else tile_loop1<kTY, kTX>(wl, st, pipe, s_m, s_g, issue, body, flush);
-}
-
-
-// --------------------------------------------------------------------------
 // Self-test of the bounded mbarrier wait
 // --------------------------------------------------------------------------
 //
@@ -2193,9 +1517,6 @@ void launch_vc_tail(const TailDesc<T>* descs, int count, size_t smem, const Inst
 // Shared-memory sizes; they follow the SmemCarve layout of each kernel (two
 // pipeline buffers, every piece rounded up to 128 bytes).
 static inline size_t rup(size_t b) { return (b + 127) & ~size_t(127); }
-template <typename T> size_t smem_apply() {
-    return 2 * (rup(kNH * kBH * kBW * sizeof(T)) + 2 * rup(kBH * kBW * sizeof(T))) + 128;
-}
 template <typename T> size_t smem_init() {
     return 2 * (rup(kNH * kBH * kBW * sizeof(T)) + rup(kBH * kBW * sizeof(T))) + 128;
 }
@@ -2203,11 +1524,8 @@ template <typename T> size_t smem_down(int pre) {
     constexpr int CY = Coarse<T>::CY;
     constexpr int DH = 2 * CY + 5;
     size_t per = rup(DH * kBW * sizeof(T));
-    if (pre != 0) per += rup(kNH * DH * kBW * sizeof(T));
-    if (pre > 1) per += rup(DH * kBW * sizeof(T));
-    size_t s = 2 * per + rup((size_t)(2 * CY + 1) * (2 * kCX + 1) * sizeof(T));
-    if (pre == 1) s += rup(DH * kBW * sizeof(T));
-    return s + 128;
+    if (pre != 0) per += rup(kNH * DH * kBW * sizeof(T)) + rup(DH * kBW * sizeof(T));
+    return 2 * per + rup((size_t)(2 * CY + 1) * (2 * kCX + 1) * sizeof(T)) + 128;
 }
 template <typename T> size_t smem_up(int pre) {
     size_t per = rup(kNH * kBH * kBW * sizeof(T)) + rup(kBH * kBW * sizeof(T)) +
@@ -2215,33 +1533,6 @@ template <typename T> size_t smem_up(int pre) {
     if (pre > 1) per += rup(kBH * kBW * sizeof(T));
     return 2 * per + 128;
 }
-
-template <typename T> size_t smem_apply_v(int nst) {
-    return nst * (rup(kNH * kPH * kBW * sizeof(T)) + 2 * rup(kBH * kBW * sizeof(T))) + 128;
-}
-// Vector widths of the register-blocked kernels, measured on B200 at
-// 1920x1080 and 4096x4096: the plain apply is fastest with 4 FP32 pixels per
-// thread (128 threads), the solver kernels (more work per tile) with 2
-// (256 threads); FP64 uses 2 (one 16-byte vector).
-template <typename T> constexpr int kVApply = sizeof(T) == 8 ? 2 : 4;
-template <typename T> constexpr int kVSolve = 2;
-// Widest vector of the element type (the tuner may pick it for the CG apply
-// and the prolongation): 4 in FP32, 2 in FP64.
-template <typename T> constexpr int kVWide = sizeof(T) == 8 ? 2 : 4;
-
-template <typename T, int V> static size_t smem_down_vv(int nst) {
-    using D = DownBox<T, V>;
-    return nst * (rup(D::DH * D::DW * sizeof(T)) +
-                  rup((kNH - 1) * (D::DH - 2) * D::DW * sizeof(T)) + rup(D::DH * D::DW * sizeof(T))) +
-           rup(D::DH * D::DW * sizeof(T)) + rup(D::RH * D::RW * sizeof(T)) + 128;
-}
-template <typename T> size_t smem_up_v(int nst) {
-    return nst * (rup(kBH * kBW * sizeof(T)) + rup((kNH - 1) * kPH * kBW * sizeof(T)) +
-                  rup(kBH * kBW * sizeof(T)) + rup(kCBH * kCBW * sizeof(T))) +
-           rup(kBH * kBW * sizeof(T)) + 128;
-}
-template <typename T> size_t smem_down_v(int nst) { return smem_down_vv<T, kVSolve<T>>(nst); }
-template <typename T> int down_box_width() { return DownBox<T, kVSolve<T>>::DW; }
 
 // Raise the dynamic shared-memory limit of a kernel. Done once for every
 // instantiation by stencil_prepare(), before any stream capture.
@@ -2274,26 +1565,6 @@ void launch_cg_init(int prec, const LaunchCfg& L, const WorkList& wl, const CUte
 }
 
 template <typename T>
-void launch_cg_apply(int vec, int stages, const LaunchCfg& L, const WorkList& wl,
-                     const CUtensorMap* maps, int zslot, T* p0, T* p1, T* Ap, InstState* st,
-                     double* part, int* err, cudaStream_t s) {
-    const int ns = stages <= 1 ? 1 : 2;
-    const size_t sm = smem_apply_v<T>(ns);
-    constexpr int V4 = kVWide<T>;
-#define PMB_CGA(VV, NS)                                                                       \
-    k_cg_apply_v<T, VV, NS><<<L.grid, tile_threads_v<VV>(), sm, s>>>(wl, maps, zslot, p0, p1, Ap, \
-                                                                     st, part, err)
-    if (vec == 4 && V4 == 4) {
-        if (ns == 1) PMB_CGA(V4, 1);
-        else PMB_CGA(V4, 2);
-    } else {
-        if (ns == 1) PMB_CGA(2, 1);
-        else PMB_CGA(2, 2);
-    }
-#undef PMB_CGA
-}
-
-template <typename T>
 void launch_cg_update(int prec, const LaunchCfg& L, const WorkList& wl, const T* P, T* x, T* r,
                       T* z, const T* p0, const T* p1, const T* Ap, T* dr, int reorth, int reliable,
                       int* pending, InstState* st, double* part, cudaStream_t s) {
@@ -2311,54 +1582,24 @@ void launch_cg_rz(const LaunchCfg& L, const WorkList& wl, const T* r, const T* z
 }
 
 template <typename T>
-void launch_vc_down(int pre, int stages, const LaunchCfg& L, const WorkList& wl,
-                    const GridDesc* fine, const CUtensorMap* maps, int xs_slot, T* bc,
-                    double omega, const InstState* st, int* err, cudaStream_t s) {
-    const int pk = pre > 1 ? 2 : pre;
-    if (pk == 1) {
-        constexpr int V = kVSolve<T>;
-        if (stages == 1)
-            k_vc_down_v<T, V, 1><<<L.grid, kDownThreads, smem_down_v<T>(1), s>>>(
-                wl, fine, maps, bc, omega, st, err);
-        else
-            k_vc_down_v<T, V, 2><<<L.grid, kDownThreads, smem_down_v<T>(2), s>>>(
-                wl, fine, maps, bc, omega, st, err);
-        return;
-    }
+void launch_vc_down(int pre, const LaunchCfg& L, const WorkList& wl, const GridDesc* fine,
+                    const CUtensorMap* maps, int xs_slot, T* bc, double omega, const InstState* st,
+                    int* err, cudaStream_t s) {
+    const int pk = pre > 1 ? 2 : 0;
     const size_t sm = smem_down<T>(pk);
-#define PMB_DOWN(PK)                                                                         \
-    do {                                                                                     \
-                                                                                    \
-        k_vc_down<T, PK><<<L.grid, kTileThreads, sm, s>>>(wl, fine, maps, xs_slot, bc, omega, st, err); \
-    } while (0)
-    if (pk == 0) PMB_DOWN(0);
-    else if (pk == 1) PMB_DOWN(1);
-    else PMB_DOWN(2);
-#undef PMB_DOWN
+    if (pk == 0)
+        k_vc_down<T, 0><<<L.grid, kTileThreads, sm, s>>>(wl, fine, maps, xs_slot, bc, omega, st, err);
+    else
+        k_vc_down<T, 2><<<L.grid, kTileThreads, sm, s>>>(wl, fine, maps, xs_slot, bc, omega, st, err);
 }
 
 template <typename T>
-void launch_vc_up(int vec, int stages, int pre, int post, const LaunchCfg& L, const WorkList& wl,
+void launch_vc_up(int pre, int post, const LaunchCfg& L, const WorkList& wl,
                   const GridDesc* coarse, const CUtensorMap* maps, int xs_slot, const T* b,
                   T* xout, double omega, InstState* st, int level0, const T* dr, int reorth,
                   double* part, int* err, cudaStream_t s) {
     const int pk = pre > 1 ? 2 : pre;
     const int qk = post > 0 ? 1 : 0;
-    if (pk == 1 && qk == 1) {
-        constexpr int V4 = kVWide<T>;
-#define PMB_UPV(VV, NS)                                                                       \
-    k_vc_up_v<T, VV, NS><<<L.grid, tile_threads_v<VV>(), smem_up_v<T>(NS), s>>>(               \
-        wl, coarse, maps, b, xout, omega, st, level0, dr, reorth, part, err)
-        if (vec == 4 && V4 == 4) {
-            if (stages == 1) PMB_UPV(V4, 1);
-            else PMB_UPV(V4, 2);
-        } else {
-            if (stages == 1) PMB_UPV(2, 1);
-            else PMB_UPV(2, 2);
-        }
-#undef PMB_UPV
-        return;
-    }
     const size_t sm = smem_up<T>(pk);
 #define PMB_UP(PK, QK)                                                                       \
     do {                                                                                     \
@@ -2368,8 +1609,7 @@ void launch_vc_up(int vec, int stages, int pre, int post, const LaunchCfg& L, co
     } while (0)
     if (pk == 0 && qk == 0) PMB_UP(0, 0);
     else if (pk == 0) PMB_UP(0, 1);
-    else if (pk == 1 && qk == 0) PMB_UP(1, 0);
-    else if (pk == 1) PMB_UP(1, 1);
+    else if (pk == 1) PMB_UP(1, 0);
     else if (qk == 0) PMB_UP(2, 0);
     else PMB_UP(2, 1);
 #undef PMB_UP
@@ -2387,14 +1627,6 @@ template <typename T>
 void launch_vc_direct(const DirectDesc* dd, int count, const T* b, T* x, InstState* st,
                       int rz_level0, cudaStream_t s) {
     if (count > 0) k_vc_direct<T><<<count, 256, 0, s>>>(dd, count, b, x, st, rz_level0);
-}
-
-template <typename T>
-void launch_apply(const LaunchCfg& L, const WorkList& wl, const CUtensorMap* maps, T* y, int* err,
-                  cudaStream_t s) {
-    const size_t sm = smem_apply_v<T>(2);
-    constexpr int V = kVApply<T>;
-    k_apply_v<T, V><<<L.grid, tile_threads_v<V>(), sm, s>>>(wl, maps, y, err);
 }
 
 template <typename TS, typename TD>
@@ -2475,36 +1707,19 @@ static void prepare_type() {
     allow_smem(k_cg_init<T, kPrecNone, true>, smem_init<T>());
     allow_smem(k_cg_init<T, kPrecJacobi, true>, smem_init<T>());
     allow_smem(k_cg_init<T, kPrecVcycle, true>, smem_init<T>());
-    allow_smem(k_cg_apply<T>, smem_apply<T>());
     allow_smem(k_vc_down<T, 0>, smem_down<T>(0));
-    allow_smem(k_vc_down<T, 1>, smem_down<T>(1));
     allow_smem(k_vc_down<T, 2>, smem_down<T>(2));
     allow_smem(k_vc_up<T, 0, 0>, smem_up<T>(0));
     allow_smem(k_vc_up<T, 0, 1>, smem_up<T>(0));
     allow_smem(k_vc_up<T, 1, 0>, smem_up<T>(1));
-    allow_smem(k_vc_up<T, 1, 1>, smem_up<T>(1));
     allow_smem(k_vc_up<T, 2, 0>, smem_up<T>(2));
     allow_smem(k_vc_up<T, 2, 1>, smem_up<T>(2));
     allow_smem(k_vc_smooth<T>, smem_init<T>());
-    allow_smem(k_apply<T>, smem_init<T>());
-    allow_smem(k_apply_v<T, kVApply<T>>, smem_apply_v<T>(2));
     allow_smem(k_vc_tail<T>, kTailSmem);
-    allow_smem(k_cg_apply_v<T, 2, 2>, smem_apply_v<T>(2));
-    allow_smem(k_cg_apply_v<T, 2, 1>, smem_apply_v<T>(1));
-    allow_smem(k_cg_apply_v<T, kVWide<T>, 2>, smem_apply_v<T>(2));
-    allow_smem(k_cg_apply_v<T, kVWide<T>, 1>, smem_apply_v<T>(1));
-    allow_smem(k_vc_up_v<T, kVWide<T>, 2>, smem_up_v<T>(2));
-    allow_smem(k_vc_up_v<T, kVWide<T>, 1>, smem_up_v<T>(1));
-    allow_smem(k_vc_down_v<T, kVSolve<T>, 2>, smem_down_v<T>(2));
-    allow_smem(k_vc_down_v<T, kVSolve<T>, 1>, smem_down_v<T>(1));
-    allow_smem(k_vc_up_v<T, kVSolve<T>, 2>, smem_up_v<T>(2));
-    allow_smem(k_vc_up_v<T, kVSolve<T>, 1>, smem_up_v<T>(1));
 }
 
-// Resident CTAs per SM of the register-blocked kernels as the occupancy
-// calculator gives them (registers, static and dynamic shared memory,
-// threads), at least 1. The shared-memory limits must be raised first
-// (stencil_prepare).
+// Resident CTAs per SM of a kernel as the occupancy calculator gives them, at
+// least 1.
 template <typename K>
 static int occupancy_of(K kernel, int threads, size_t smem) {
     int n = 0;
@@ -2515,17 +1730,6 @@ static int occupancy_of(K kernel, int threads, size_t smem) {
     return n > 0 ? n : 1;
 }
 
-template <typename T> int resident_cg_apply(int vec, int stages) {
-    stencil_prepare();
-    constexpr int V4 = kVWide<T>;
-    const int ns = stages <= 1 ? 1 : 2;
-    const size_t sm = smem_apply_v<T>(ns);
-    if (vec == 4 && V4 == 4)
-        return ns == 1 ? occupancy_of(k_cg_apply_v<T, V4, 1>, tile_threads_v<V4>(), sm)
-                       : occupancy_of(k_cg_apply_v<T, V4, 2>, tile_threads_v<V4>(), sm);
-    return ns == 1 ? occupancy_of(k_cg_apply_v<T, 2, 1>, tile_threads_v<2>(), sm)
-                   : occupancy_of(k_cg_apply_v<T, 2, 2>, tile_threads_v<2>(), sm);
-}
 // Resident CTAs per SM of k_cg_update (a register limit, below the flat
 // lists' default of 8: a persistent grid beyond it would run a second, thin
 // wave of CTAs after the first).
@@ -2539,28 +1743,12 @@ template <typename T> int resident_cg_update(int prec) {
     }
     return cached[k];
 }
-template <typename T> int resident_down(int stages) {
-    stencil_prepare();
-    constexpr int V = kVSolve<T>;
-    return stages <= 1 ? occupancy_of(k_vc_down_v<T, V, 1>, kDownThreads, smem_down_v<T>(1))
-                       : occupancy_of(k_vc_down_v<T, V, 2>, kDownThreads, smem_down_v<T>(2));
-}
-template <typename T> int resident_up(int vec, int stages) {
-    stencil_prepare();
-    constexpr int V4 = kVWide<T>;
-    const int ns = stages <= 1 ? 1 : 2;
-    if (vec == 4 && V4 == 4)
-        return ns == 1 ? occupancy_of(k_vc_up_v<T, V4, 1>, tile_threads_v<V4>(), smem_up_v<T>(1))
-                       : occupancy_of(k_vc_up_v<T, V4, 2>, tile_threads_v<V4>(), smem_up_v<T>(2));
-    return ns == 1 ? occupancy_of(k_vc_up_v<T, 2, 1>, tile_threads_v<2>(), smem_up_v<T>(1))
-                   : occupancy_of(k_vc_up_v<T, 2, 2>, tile_threads_v<2>(), smem_up_v<T>(2));
-}
-
 void stencil_prepare() {
     static bool done = false;
     if (done) return;
     prepare_type<double>();
     prepare_type<float>();
+    prepare_rows();
     allow_smem(k_galerkin_t, kNH * kGRows * kGCols * sizeof(double));
     allow_smem(k_refine_residual<kPrecNone, true>, smem_init<double>());
     allow_smem(k_refine_residual<kPrecJacobi, true>, smem_init<double>());
@@ -2575,18 +1763,15 @@ void stencil_prepare() {
     template void launch_cg_init<T>(int, const LaunchCfg&, const WorkList&, const CUtensorMap*,   \
                                     const T*, const T*, T*, bool, T*, T*, InstState*, double*,    \
                                     double, double, int, int*, cudaStream_t);                     \
-    template void launch_cg_apply<T>(int, int, const LaunchCfg&, const WorkList&,                 \
-                                     const CUtensorMap*, int, T*, T*, T*, InstState*, double*,    \
-                                     int*, cudaStream_t);                                         \
     template void launch_cg_update<T>(int, const LaunchCfg&, const WorkList&, const T*, T*, T*,   \
                                       T*, const T*, const T*, const T*, T*, int, int, int*,      \
                                       InstState*, double*, cudaStream_t);                        \
     template void launch_cg_rz<T>(const LaunchCfg&, const WorkList&, const T*, const T*,          \
                                   const T*, int, InstState*, double*, cudaStream_t);             \
-    template void launch_vc_down<T>(int, int, const LaunchCfg&, const WorkList&, const GridDesc*, \
+    template void launch_vc_down<T>(int, const LaunchCfg&, const WorkList&, const GridDesc*,      \
                                     const CUtensorMap*, int, T*, double, const InstState*, int*, \
                                     cudaStream_t);                                               \
-    template void launch_vc_up<T>(int, int, int, int, const LaunchCfg&, const WorkList&,         \
+    template void launch_vc_up<T>(int, int, const LaunchCfg&, const WorkList&,                   \
                                   const GridDesc*, const CUtensorMap*, int, const T*, T*, double, \
                                   InstState*, int, const T*, int, double*, int*, cudaStream_t);  \
     template void launch_vc_smooth<T>(const LaunchCfg&, const WorkList&, const CUtensorMap*, int, \
@@ -2594,20 +1779,10 @@ void stencil_prepare() {
                                       cudaStream_t);                                             \
     template void launch_vc_direct<T>(const DirectDesc*, int, const T*, T*, InstState*, int,      \
                                       cudaStream_t);                                             \
-    template void launch_apply<T>(const LaunchCfg&, const WorkList&, const CUtensorMap*, T*, int*, \
-                                  cudaStream_t);                                                 \
-    template size_t smem_apply<T>();                                                              \
     template size_t smem_init<T>();                                                               \
     template size_t smem_down<T>(int);                                                            \
     template size_t smem_up<T>(int);                                                              \
-    template size_t smem_apply_v<T>(int);                                                         \
-    template int resident_cg_apply<T>(int, int);                                                  \
-    template int resident_down<T>(int);                                                           \
-    template int resident_cg_update<T>(int);                                                      \
-    template int resident_up<T>(int, int);                                                        \
-    template size_t smem_down_v<T>(int);                                                          \
-    template size_t smem_up_v<T>(int);                                                            \
-    template int down_box_width<T>();
+    template int resident_cg_update<T>(int);
 
 PMB_INST(double)
 PMB_INST(float)

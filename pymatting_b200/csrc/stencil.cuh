@@ -48,23 +48,44 @@ void launch_vc_tail(const TailDesc<T>* descs, int count, size_t smem, const Inst
                     double omega, int* err, cudaStream_t s);
 
 // Shared memory (bytes) of the TMA-tiled kernels, for launch sizing.
-template <typename T> size_t smem_apply();
 template <typename T> size_t smem_init();
 template <typename T> size_t smem_down(int pre);
 template <typename T> size_t smem_up(int pre);
-// ... of the register-blocked kernels (default one pre- and one post-sweep).
-template <typename T> size_t smem_apply_v(int nst);
-// nst: 2 buffers (a tile in flight while one is computed) or 1.
-template <typename T> size_t smem_down_v(int nst);
-template <typename T> size_t smem_up_v(int nst);
-// Resident CTAs per SM of the register-blocked CG apply, restriction and
-// prolongation kernels for a vector width and buffer count (occupancy API).
-template <typename T> int resident_cg_apply(int vec, int stages);
-template <typename T> int resident_down(int stages);
+// Resident CTAs per SM of k_cg_update (occupancy API).
 template <typename T> int resident_cg_update(int prec);
-template <typename T> int resident_up(int vec, int stages);
-// Width of the register-blocked restriction box (its TMA maps).
-template <typename T> int down_box_width();
+
+// --- Row-streaming kernels (stencil_rows.cu) -------------------------------
+
+constexpr int kUnitWarps = 4;      // units (warps) of one CTA
+
+// Unit table of a row-streaming launch: one int4 per CTA {grid, first unit of
+// the CTA in the grid, strips of the grid, units of the grid}. Units of a grid
+// are numbered strip by strip, segment by segment (`seg` rows each).
+struct RowList {
+    const int4* cta;
+    const GridDesc* grids;
+    int total;                     // CTAs
+    int seg;
+};
+
+enum : int { kRowsApply = 0, kRowsDown = 1, kRowsUp = 2 };
+// Useful columns of a strip (coarse columns for kRowsDown); vec = 2 or 4.
+int rows_strip(int kind, int vec);
+template <typename T> int rows_resident_of(int kind, int vec);
+void prepare_rows();
+
+// rev: CTAs take the table from its end, so that a pass starts with what the
+// pass before it left in L2. st == nullptr: every image, no reduction.
+template <typename T>
+void launch_rows_apply(int vec, const RowList& R, int rev, const T* P, const T* z, T* p0, T* p1,
+                       T* Ap, InstState* st, double* part, cudaStream_t s);
+template <typename T>
+void launch_rows_down(int vec, const RowList& R, int rev, const GridDesc* fine, const T* P, const T* b,
+                      T* bc, double omega, const InstState* st, cudaStream_t s);
+template <typename T>
+void launch_rows_up(int vec, const RowList& R, int rev, const GridDesc* coarse, const T* P, const T* b,
+                    const T* xc, T* xout, double omega, InstState* st, int level0, const T* dr,
+                    int reorth, double* part, cudaStream_t s);
 
 // Raise the dynamic shared-memory limits once (before any graph capture).
 void stencil_prepare();
@@ -78,10 +99,6 @@ void launch_cg_init(int prec, const LaunchCfg& L, const WorkList& wl, const CUte
                     const T* P, const T* b, T* x, bool have_x0, T* r, T* z, InstState* st,
                     double* part, double atol, double rtol, int maxiter, int* err, cudaStream_t s);
 template <typename T>
-void launch_cg_apply(int vec, int stages, const LaunchCfg& L, const WorkList& wl,
-                     const CUtensorMap* maps, int zslot, T* p0, T* p1, T* Ap, InstState* st,
-                     double* part, int* err, cudaStream_t s);
-template <typename T>
 void launch_cg_update(int prec, const LaunchCfg& L, const WorkList& wl, const T* P, T* x, T* r,
                       T* z, const T* p0, const T* p1, const T* Ap, T* dr, int reorth, int reliable,
                       int* pending, InstState* st, double* part, cudaStream_t s);
@@ -89,11 +106,11 @@ template <typename T>
 void launch_cg_rz(const LaunchCfg& L, const WorkList& wl, const T* r, const T* z, const T* dr,
                   int reorth, InstState* st, double* part, cudaStream_t s);
 template <typename T>
-void launch_vc_down(int pre, int stages, const LaunchCfg& L, const WorkList& wl,
-                    const GridDesc* fine, const CUtensorMap* maps, int xs_slot, T* bc,
-                    double omega, const InstState* st, int* err, cudaStream_t s);
+void launch_vc_down(int pre, const LaunchCfg& L, const WorkList& wl, const GridDesc* fine,
+                    const CUtensorMap* maps, int xs_slot, T* bc, double omega, const InstState* st,
+                    int* err, cudaStream_t s);
 template <typename T>
-void launch_vc_up(int vec, int stages, int pre, int post, const LaunchCfg& L, const WorkList& wl,
+void launch_vc_up(int pre, int post, const LaunchCfg& L, const WorkList& wl,
                   const GridDesc* coarse, const CUtensorMap* maps, int xs_slot, const T* b,
                   T* xout, double omega, InstState* st, int level0, const T* dr, int reorth,
                   double* part, int* err, cudaStream_t s);
@@ -104,9 +121,6 @@ void launch_vc_smooth(const LaunchCfg& L, const WorkList& wl, const CUtensorMap*
 template <typename T>
 void launch_vc_direct(const DirectDesc* dd, int count, const T* b, T* x, InstState* st,
                       int rz_level0, cudaStream_t s);
-template <typename T>
-void launch_apply(const LaunchCfg& L, const WorkList& wl, const CUtensorMap* maps, T* y, int* err,
-                  cudaStream_t s);
 template <typename TS, typename TD>
 void launch_pack(const GridDesc* grids, int ngrids, const int64_t* uoff, const TS* src, TD* dst,
                  int64_t total, cudaStream_t s);
