@@ -233,8 +233,9 @@ int pmb_stencil_stats(pmb_stencil* s, int image, int* iters, int* status, double
 int64_t pmb_stencil_launch_count(const pmb_stencil* s);
 int pmb_stencil_destroy(pmb_stencil* s);
 /* Launch-shape knobs of the solver, for the autotuner (no counterpart in the
- * reference): 0 columns per lane of the CG apply (2 or 4, 4 only for the
- * FP32 inner solve), 1 the same for restriction and prolongation, 2/3/4 CTAs
+ * reference): 0 columns per lane of the CG apply (one 16-byte vector: 4 for
+ * the FP32 inner solve, 2 for FP64), 1 the same for restriction and
+ * prolongation, 2/3/4 CTAs
  * per SM that the rows of the CG apply / prolongation / restriction are cut
  * for (up to their residency), 5 CTAs per SM of the element-wise kernels, 6 CG
  * iterations per graph replay, 7 buffers of the tile kernels (1 is the only

@@ -3,7 +3,8 @@
 The knobs (``pmb_stencil_tune`` in the C ABI):
 
 * ``vec_apply`` / ``vec_up`` — columns per lane of the CG apply and of the
-  V-cycle's restriction and prolongation (2 or 4; 4 in FP32 only);
+  V-cycle's restriction and prolongation: one 16-byte vector, 4 in FP32 and 2
+  in FP64;
 * ``ctas_fine`` / ``ctas_up`` / ``ctas_down`` — CTAs per SM that the rows of
   the CG apply, the prolongation and the restriction are cut for (bounded by
   their registers and shared memory);
@@ -34,7 +35,7 @@ __all__ = ["KNOBS", "tuning", "apply_tuning", "autotune", "cache_key", "cached"]
 
 KNOBS = {"stages": 7, "vec_apply": 0, "vec_up": 1, "ctas_fine": 2, "ctas_up": 3,
          "ctas_down": 4, "ctas_flat": 5, "chunk": 6}
-CANDIDATES = {"stages": [1], "vec_apply": [2, 4], "vec_up": [2, 4], "ctas_fine": [1, 2, 3, 4],
+CANDIDATES = {"stages": [1], "vec_apply": [2], "vec_up": [2], "ctas_fine": [1, 2, 3, 4],
               "ctas_up": [1, 2, 3, 4], "ctas_down": [1, 2, 3, 4], "ctas_flat": [2, 4, 8, 16],
               "chunk": [2, 4, 8]}
 _MARGIN = 0.02          # a change must win by 2 %

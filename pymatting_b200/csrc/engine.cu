@@ -162,10 +162,9 @@ struct Stencil {
     std::vector<int> h, w;
     int precision = 0;   // 0: FP64, 1: FP32 inner + FP64 refinement
     int precond = 0;     // kPrecNone / kPrecJacobi / kPrecVcycle
-    // Launch shapes (pmb_stencil_tune): columns per lane of the CG apply and
-    // of the V-cycle kernels, CTAs per SM that each list is cut for, CG
-    // iterations per graph replay.
-    int vec_apply = 2, vec_up = 2, chunk = 4;
+    // Launch shapes (pmb_stencil_tune): CTAs per SM that each list is cut for,
+    // CG iterations per graph replay.
+    int chunk = 4;
     int max_fine = 1, max_up = 1, max_down = 1;
     int pre = 1, post = 1;
     double omega = 0.8;
@@ -260,22 +259,22 @@ static void build_flat(HostList& L, const std::vector<GridDesc>& grids) {
     L.grids = grids;
     L.partner.clear();
     L.starts.assign(grids.size() + 1, 0);
+    int64_t total = 0;
+    for (const GridDesc& g : grids) total += (int64_t)g.h * g.pitch;
+    // A chunk is a CTA's serial work: as long as it can be while every
+    // resident CTA has one.
+    L.wl.chunk = kFlat;
+    while (L.wl.chunk > kFlatMin && total < (int64_t)L.wl.chunk * 148 * 6) L.wl.chunk /= 2;
     for (size_t g = 0; g < grids.size(); ++g) {
         const int64_t n = (int64_t)grids[g].h * grids[g].pitch;
-        L.starts[g + 1] = L.starts[g] + (int)((n + kFlat - 1) / kFlat);
+        L.starts[g + 1] = L.starts[g] + (int)((n + L.wl.chunk - 1) / L.wl.chunk);
     }
 }
 
-// Columns per lane of the row-streaming kernel that walks list L.
-static int rows_vec(const Stencil& S, const HostList& L) {
-    return L.rows == kRowsApply ? S.vec_apply : S.vec_up;
-}
-
 // Resident CTAs per SM that a list of this kind may be cut for.
-static int rows_limit(const Stencil& S, int kind, int vec) {
+static int rows_limit(const Stencil& S, int kind) {
     stencil_prepare();
-    const int n = S.precision == 1 ? rows_resident_of<float>(kind, vec)
-                                   : rows_resident_of<double>(kind, vec);
+    const int n = S.precision == 1 ? rows_resident_of<float>(kind) : rows_resident_of<double>(kind);
     return std::max(1, std::min(4, n));
 }
 
@@ -284,8 +283,8 @@ static int rows_limit(const Stencil& S, int kind, int vec) {
 // of them and no more (a second, thin wave would double its time); a longer
 // one into segments of 32 rows (16 coarse rows), whose two rows of halo cost
 // about 5 % (they come from L2) while the scheduler still balances the waves.
-static void build_rows(HostList& L, int vec) {
-    const int cols = rows_strip(L.rows, vec);
+static void build_rows(const Stencil& S, HostList& L) {
+    const int cols = S.precision == 1 ? rows_strip<float>(L.rows) : rows_strip<double>(L.rows);
     const int longest = L.rows == kRowsDown ? 16 : 32;
     auto units = [&](int seg, bool ctas) {
         int64_t n = 0;
@@ -313,13 +312,12 @@ static void build_rows(HostList& L, int vec) {
 static void plan_rows(Stencil& S, HostList& L, int kind) {
     L.rows = kind;
     const int per_sm = L.per_sm;
-    for (L.per_sm = 1; L.per_sm <= 4; ++L.per_sm)
-        for (int vec = 2; vec <= (S.precision == 1 ? 4 : 2); vec += 2) {
-            build_rows(L, vec);
-            L.cta_cap = std::max<int64_t>(L.cta_cap, L.R.total);
-        }
+    for (L.per_sm = 1; L.per_sm <= 4; ++L.per_sm) {
+        build_rows(S, L);
+        L.cta_cap = std::max<int64_t>(L.cta_cap, L.R.total);
+    }
     L.per_sm = per_sm;
-    build_rows(L, rows_vec(S, L));
+    build_rows(S, L);
 }
 
 static void carve_list(Carve& c, HostList& L) {
@@ -405,18 +403,13 @@ static int plan_stencil(Stencil& S) {
         lv.plane_elems = poff;
     }
     S.nmaps = map_base;
-    // Four columns per lane in FP32 once the strips of 120 columns fill the
-    // GPU: measured per iteration, 2 against 4 columns, 139 and 147 us at
-    // 320x240, 155 and 160 at 512x512, 295 and 291 at 1920x1080, 666 and 637
-    // at 3840x2160, 4214 and 3908 on the 73 Mpix of 64 images.
-    if (mixed && S.user_total >= 2000000) S.vec_apply = S.vec_up = 4;
     // Work lists and the residency of the kernels that walk them.
     const bool rows_up = S.pre == 1 && S.post >= 1, rows_down = S.pre == 1;
-    const int per_fine = rows_limit(S, kRowsApply, S.vec_apply);
-    const int per_up = rows_up ? rows_limit(S, kRowsUp, S.vec_up)
+    const int per_fine = rows_limit(S, kRowsApply);
+    const int per_up = rows_up ? rows_limit(S, kRowsUp)
                                : blocks_per_sm(mixed ? smem_up<float>(S.pre) : smem_up<double>(S.pre));
     const int per_down =
-        rows_down ? rows_limit(S, kRowsDown, S.vec_up)
+        rows_down ? rows_limit(S, kRowsDown)
                   : blocks_per_sm(mixed ? smem_down<float>(S.pre) : smem_down<double>(S.pre));
     S.max_fine = per_fine;
     S.max_up = per_up;
@@ -572,7 +565,7 @@ static int upload_rows(Stencil& S, HostList& L) {
 // After a knob of list L changed: its table again.
 static int retune_rows(Stencil& S, HostList& L) {
     if (L.rows < 0) return 0;
-    build_rows(L, rows_vec(S, L));
+    build_rows(S, L);
     if (!S.bound) return 0;
     if (int rc = upload_rows(S, L)) return rc;
     PMB_CUDA(cudaStreamSynchronize(S.stream));
@@ -941,7 +934,7 @@ static void run_vcycle(Stencil& S, const T* b0, T* z0, InstState* st, const T* d
             xs_slot_d[l] = in_a ? kMapXAD : kMapXBD;
         }
         if (c.rows >= 0)
-            launch_rows_down<T>(rows_vec(S, c), c.R, l == 0 ? S.pass++ & 1 : 0, c.partner_dev,
+            launch_rows_down<T>(c.R, l == 0 ? S.pass++ & 1 : 0, c.partner_dev,
                                 lvl_P<T>(S, l), B(l), B(l + 1), om, st, s);
         else
             launch_vc_down<T>(pre, LaunchCfg{persistent_grid(c)}, c.wl, c.partner_dev, S.maps(),
@@ -976,7 +969,7 @@ static void run_vcycle(Stencil& S, const T* b0, T* z0, InstState* st, const T* d
         T* first_out = first_in_x ? X(l) : lvl_xa<T>(S, l);
         const bool reduce_here = (l == 0) && st && extra == 0;
         if (f.rows >= 0)
-            launch_rows_up<T>(rows_vec(S, f), f.R, l == 0 ? S.pass++ & 1 : 0, f.partner_dev,
+            launch_rows_up<T>(f.R, l == 0 ? S.pass++ & 1 : 0, f.partner_dev,
                               lvl_P<T>(S, l), B(l), X(l + 1), first_out, om, st,
                               reduce_here ? 1 : 0, dr, reorth, S.partials(), s);
         else
@@ -1012,7 +1005,7 @@ static void cg_iteration(Stencil& S, int reorth) {
     CgVecs<T> v = cg_vecs<T>(S);
     InstState* st = S.state();
     // Without a preconditioner z is r itself (cg.py:53-55).
-    launch_rows_apply<T>(S.vec_apply, S.fine0.R, S.pass++ & 1, v.P,
+    launch_rows_apply<T>(S.fine0.R, S.pass++ & 1, v.P,
                          S.precond == kPrecNone ? v.r : v.z, v.p0, v.p1, v.ap, st, S.partials(), s);
     prof_mark(S, kPkApply);
     const bool mixed = S.precision == 1;
@@ -1647,7 +1640,7 @@ PMB_API int pmb_stencil_apply(pmb_stencil* p, const double* x, double* y, void* 
         double* ty = S.at<double>(S.o_ap64);
         launch_pack<double, double>(a.wl.grids, a.wl.ngrids, S.at<int64_t>(S.o_uoff), x, tx,
                                     S.user_total, s);
-        launch_rows_apply<double>(S.vec_apply, a.R, 0, S.P0, tx, nullptr, nullptr, ty, nullptr,
+        launch_rows_apply<double>(a.R, 0, S.P0, tx, nullptr, nullptr, ty, nullptr,
                                   nullptr, s);
         launch_unpack<double, double>(a.wl.grids, a.wl.ngrids, S.at<int64_t>(S.o_uoff), ty, y,
                                       S.user_total, s);
@@ -1682,7 +1675,6 @@ PMB_API int64_t pmb_stencil_launch_count(const pmb_stencil* p) { return p ? p->S
 PMB_API int pmb_stencil_tune(pmb_stencil* p, int knob, int value) {
     if (!p) return fail(kErrArg, "pmb_stencil_tune: null solver");
     Stencil& S = p->S;
-    const int wide = S.precision == 1 ? 4 : 2;
     auto clampi = [](int v, int lo, int hi) { return std::max(lo, std::min(hi, v)); };
     int applied;
     auto each = [&](HostList Level::*list) {
@@ -1693,24 +1685,7 @@ PMB_API int pmb_stencil_tune(pmb_stencil* p, int knob, int value) {
     int rc = 0;
     switch (knob) {
     case 0:
-        applied = S.vec_apply = (value >= 4 ? wide : 2);
-        S.max_fine = rows_limit(S, kRowsApply, S.vec_apply);
-        S.fine0.per_sm = std::min(S.fine0.per_sm, S.max_fine);
-        rc = retune_rows(S, S.fine0);
-        break;
-    case 1:
-        applied = S.vec_up = (value >= 4 ? wide : 2);
-        if (S.pre == 1) {
-            S.max_down = rows_limit(S, kRowsDown, S.vec_up);
-            for (auto& lv : S.levels) lv.coarse.per_sm = std::min(lv.coarse.per_sm, S.max_down);
-            rc = each(&Level::coarse);
-        }
-        if (S.pre == 1 && S.post >= 1) {
-            S.max_up = rows_limit(S, kRowsUp, S.vec_up);
-            for (auto& lv : S.levels) lv.fine.per_sm = std::min(lv.fine.per_sm, S.max_up);
-            if (!rc) rc = each(&Level::fine);
-        }
-        break;
+    case 1: applied = S.precision == 1 ? 4 : 2; break;    // one 16-byte vector per lane
     case 2:
         applied = clampi(value, 1, S.max_fine);
         S.fine0.per_sm = applied;
@@ -1759,8 +1734,8 @@ PMB_API int pmb_stencil_tuning(const pmb_stencil* p, int knob) {
     if (!p) return fail(kErrArg, "pmb_stencil_tuning: null solver");
     const Stencil& S = p->S;
     switch (knob) {
-    case 0: return S.vec_apply;
-    case 1: return S.vec_up;
+    case 0:
+    case 1: return S.precision == 1 ? 4 : 2;
     case 2: return S.fine0.per_sm;
     case 3: return S.levels.empty() ? 0 : S.levels[0].fine.per_sm;
     case 4: return S.levels.empty() ? 0 : S.levels[0].coarse.per_sm;
@@ -2629,10 +2604,10 @@ PMB_API int pmb_stencil_time_apply(pmb_stencil* p, int iters, double* ms, void* 
         HostList& a = S.fine0;
         auto launch = [&]() {
             if (S.precision == 0)
-                launch_rows_apply<double>(S.vec_apply, a.R, 0, S.P0, S.at<double>(S.o_r64), nullptr,
+                launch_rows_apply<double>(a.R, 0, S.P0, S.at<double>(S.o_r64), nullptr,
                                           nullptr, S.at<double>(S.o_ap64), nullptr, nullptr, S.stream);
             else
-                launch_rows_apply<float>(S.vec_apply, a.R, 0, S.at<float>(S.o_P032),
+                launch_rows_apply<float>(a.R, 0, S.at<float>(S.o_P032),
                                          S.at<float>(S.o_r32), nullptr, nullptr,
                                          S.at<float>(S.o_ap32), nullptr, nullptr, S.stream);
         };

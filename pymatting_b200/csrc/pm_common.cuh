@@ -29,10 +29,13 @@ constexpr int kTX = 64;      // fine tile width
 constexpr int kTY = 8;       // fine tile height
 constexpr int kThreads = 256;      // element-wise kernels
 constexpr int kTileThreads = 512;  // tiled stencil kernels: one pixel per thread
-// Elements per tile of the element-wise kernels. 8192 halves the per-chunk
-// barriers and directory lookups of the flat loops against 4096 (the FP32 CG
-// update: 0.38 -> 0.31 ms per iteration of the 64-image batch).
+// Most elements per tile of the element-wise kernels, and fewest (one pass of
+// 16-byte vectors over the CTA). 8192 halves the per-chunk barriers and
+// directory lookups of the flat loops against 4096 (the FP32 CG update: 0.38
+// -> 0.31 ms per iteration of the 64-image batch); lists that would give most
+// SMs nothing to do are cut finer (engine.cu, build_flat).
 constexpr int kFlat = 8192;
+constexpr int kFlatMin = 1024;
 
 // Shared-memory boxes loaded by TMA around a fine tile at (x0, y0): origin
 // (x0 - kBOX, y0 - 2), kBW x kBH elements. x0 - kBOX keeps the box start
@@ -104,6 +107,7 @@ struct WorkList {
     const int* tile_start;
     int ngrids;
     int total;
+    int chunk;          // elements per tile of a flat list
 };
 
 // Per-image solver state, kept on the device so a whole iteration can be
@@ -275,6 +279,19 @@ __device__ __forceinline__ void ldv(const T* p, T* o) {
     }
 }
 
+// The same from L2, for what earlier kernels of a chain write (grid_wait).
+template <typename T, int V>
+__device__ __forceinline__ void ldv_l2(const T* p, T* o) {
+    if constexpr (sizeof(T) == 4 && V == 4) {
+        const float4 q = __ldcg(reinterpret_cast<const float4*>(p));
+        o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
+    } else {
+        static_assert(sizeof(T) == 8 && V == 2, "unsupported vector");
+        const double2 q = __ldcg(reinterpret_cast<const double2*>(p));
+        o[0] = q.x; o[1] = q.y;
+    }
+}
+
 template <typename T, int V>
 __device__ __forceinline__ void stv(T* p, const T* o) {
     if constexpr (sizeof(T) == 4 && V == 4) {
@@ -286,7 +303,7 @@ __device__ __forceinline__ void stv(T* p, const T* o) {
     }
 }
 
-__device__ __forceinline__ void finish_beta(InstState* st, double rz_new) {
+__device__ __forceinline__ void finish_beta(volatile InstState* st, double rz_new) {
     // First pass after the initial residual: only record r.z (cg.py:78-80).
     if (st->flags & kFirst) {
         st->rz = rz_new;
@@ -300,7 +317,7 @@ __device__ __forceinline__ void finish_beta(InstState* st, double rz_new) {
 }
 
 // beta = ((r - r_old) . z) / rz when reorthogonalising (cg.py:102-104).
-__device__ __forceinline__ void finish_beta_reorth(InstState* st, double rz_new, double dz) {
+__device__ __forceinline__ void finish_beta_reorth(volatile InstState* st, double rz_new, double dz) {
     if (st->flags & kFirst) {
         st->rz = rz_new;
         return;
@@ -315,6 +332,43 @@ __device__ __forceinline__ void finish_beta_reorth(InstState* st, double rz_new,
 template <typename T> __device__ __forceinline__ T smooth_div(T a, T b) { return a / b; }
 template <> __device__ __forceinline__ float smooth_div<float>(float a, float b) {
     return __fdividef(a, b);
+}
+
+// --- Programmatic dependent launch ------------------------------------------
+//
+// The kernels of an iteration are launched with launch_chain: each may start
+// while its predecessor still runs (grid_trigger, called first by every CTA)
+// and does what depends on nothing that a solve writes (unit tables, grid
+// descriptors, operator planes) before grid_wait, which returns when the
+// predecessor has completed and its writes are visible. Every kernel of a
+// chain waits before it ends, so completion is transitive; the writers of
+// planes and tables are always followed by a kernel launched without the
+// attribute. Everything that a kernel of a chain writes is read from L2 by the
+// others (ldv_l2, __ldcg, volatile, bulk copies, cp.async.cg), so that nothing
+// rests on when an SM drops L1 lines that a kernel still running there fetched
+// after its successor had started.
+// It takes the launch gaps and the latency of the first rows' planes off every
+// kernel of an iteration: one FP64 V-cycle of 1920x1080 310 -> 251 us, a
+// forward and an adjoint FP64 solve of four 512x512 images 61 -> 53 ms.
+__device__ __forceinline__ void grid_trigger() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+inline void launch_chain(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s,
+                         Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
 }  // namespace pmb

@@ -7,7 +7,7 @@
 // operator planes (72 x 12 x 13), 2D boxes hold the vector operands; the
 // hardware zero-fills everything outside the image, which supplies the
 // stencil's border terms. The kernels then read operators and operands from
-// shared memory only. Element-wise kernels stream kFlat-element chunks.
+// shared memory only. Element-wise kernels stream chunks of elements.
 //
 // Every kernel walks a WorkList of tiles over a batch of grids (images of
 // different sizes, or the same multigrid level of several images) with a
@@ -127,7 +127,7 @@ __device__ __forceinline__ void dir_load(TileDir& D, const WorkList& wl, const I
             int run = 1, par = 0, first = 0;
             double beta = 0.0;
             if (st) {
-                const InstState& q = st[g.inst];
+                const volatile InstState& q = st[g.inst];
                 run = q.status == kRunning && (GATE == kGateRunning || (q.flags & kUpdate) != 0);
                 par = q.iters & 1;
                 first = (q.flags & kFirst) != 0;
@@ -201,7 +201,7 @@ __device__ __forceinline__ int next_running_tile(const TileDir& D, const WorkLis
             g = find_grid(wl, t);
             run = true;
             if (st) {
-                const InstState& q = st[wl.grids[g].inst];
+                const volatile InstState& q = st[wl.grids[g].inst];
                 run = q.status == kRunning && (GATE == kGateRunning || (q.flags & kUpdate) != 0);
             }
             nxt = wl.tile_start[g + 1];
@@ -238,7 +238,7 @@ __device__ __forceinline__ void dir_meta(const TileDir& D, const WorkList& wl, c
         m.first = 0;
         m.beta = 0.0;
         if (st) {
-            const InstState& q = st[gd.inst];
+            const volatile InstState& q = st[gd.inst];
             m.par = q.iters & 1;
             m.first = (q.flags & kFirst) != 0;
             m.beta = q.beta;
@@ -404,7 +404,7 @@ k_cg_init(WorkList wl, const CUtensorMap* maps, const T* __restrict__ P, const T
     tile_loop<kTY, kTX>(wl, nullptr, pipe, s_m, s_g, issue, body, flush);
 }
 
-// Element-wise loop over a flat work list (kFlat-element chunks) with the same
+// Element-wise loop over a flat work list (wl.chunk elements a tile) with the same
 // per-CTA, per-image flush as the tiled kernels. Chunks cover the pitched
 // rows; padding columns are skipped.
 template <int GATE = kGateRunning, typename Body, typename Flush>
@@ -436,8 +436,8 @@ __device__ __forceinline__ void flat_loop(const WorkList& wl, const InstState* s
         __syncthreads();
         const GridDesc g = s_gd;
         const int64_t n = (int64_t)g.h * g.pitch;
-        const int64_t e0 = (int64_t)(t - s_t0) * kFlat;
-        const int64_t e1 = min(e0 + kFlat, n);
+        const int64_t e0 = (int64_t)(t - s_t0) * wl.chunk;
+        const int64_t e1 = min(e0 + wl.chunk, n);
         body(g, e0, e1);
         ++mine;
         if (s_inst[1] != s_inst[0]) {
@@ -455,13 +455,15 @@ __device__ __forceinline__ void flat_loop(const WorkList& wl, const InstState* s
 template <typename T, int PREC>
 __global__ void __launch_bounds__(kThreads)
 k_cg_update(WorkList wl, const T* __restrict__ P, T* x, T* r, T* z, const T* p0, const T* p1,
-            const T* __restrict__ Ap, T* dr, int reorth, int reliable, int* pending, InstState* st,
+            const T* Ap, T* dr, int reorth, int reliable, int* pending, InstState* st,
             double* partials) {
     constexpr int VE = 16 / sizeof(T);          // elements per 16-byte vector
     __shared__ double s_red[3 * 32];
+    grid_trigger();
+    grid_wait();
     double v[3] = {0.0, 0.0, 0.0};
     auto body = [&](const GridDesc& g, int64_t e0, int64_t e1) {
-        const InstState& s = st[g.inst];
+        const volatile InstState& s = st[g.inst];
         const T a = (T)s.alpha;
         const T* p = (s.iters & 1) ? p0 : p1;   // the buffer k_cg_apply wrote
         // Vectors never straddle rows (the pitch is a multiple of 32); padding
@@ -474,16 +476,16 @@ k_cg_update(WorkList wl, const T* __restrict__ P, T* x, T* r, T* z, const T* p0,
             if (col0 >= g.w) continue;
             const int64_t i = g.voff + e;
             T xv[VE], rv[VE], pv[VE], av[VE], zv[VE], dv[VE], drv[VE];
-            ldv<T, VE>(x + i, xv);
-            ldv<T, VE>(r + i, rv);
-            ldv<T, VE>(p + i, pv);
-            ldv<T, VE>(Ap + i, av);
+            ldv_l2<T, VE>(x + i, xv);
+            ldv_l2<T, VE>(r + i, rv);
+            ldv_l2<T, VE>(p + i, pv);
+            ldv_l2<T, VE>(Ap + i, av);
             if (PREC == kPrecJacobi) {
                 const int row = (int)(e / g.pitch);
                 ldv<T, VE>(P + g.poff + (int64_t)row * g.pitch + col0, dv);
-                ldv<T, VE>(z + i, zv);
+                ldv_l2<T, VE>(z + i, zv);
             }
-            if (PREC == kPrecVcycle && reorth) ldv<T, VE>(dr + i, drv);
+            if (PREC == kPrecVcycle && reorth) ldv_l2<T, VE>(dr + i, drv);
 #pragma unroll
             for (int u = 0; u < VE; ++u) {
                 if (col0 + u >= g.w) continue;
@@ -511,18 +513,18 @@ k_cg_update(WorkList wl, const T* __restrict__ P, T* x, T* r, T* z, const T* p0,
         }
     };
     auto flush = [&](int inst, int t0, int t1, unsigned int mine) {
-        InstState* s = st + inst;
-        cta_flush<3>(v, partials, inst, t0, t1, mine, s, s_red, [&](double* sum) {
+        volatile InstState* s = st + inst;
+        cta_flush<3>(v, partials, inst, t0, t1, mine, st + inst, s_red, [&](double* sum) {
             const double nr = sqrt(sum[0]);
             s->norm_r = nr;
-            s->iters += 1;
+            s->iters = s->iters + 1;
             if (!isfinite(nr)) s->status = kNonFinite;
             else if (nr < s->tol) {
                 // Mixed precision: the phase ends with an FP64 residual
                 // replacement (k_refine_residual, same iteration), which also
                 // finishes beta; otherwise the solve has converged.
                 if (reliable) {
-                    s->flags |= kUpdate;
+                    s->flags = s->flags | kUpdate;
                     atomicAdd(pending, 1);
                 } else {
                     s->status = kConverged;
@@ -1162,6 +1164,8 @@ k_refine_residual(WorkList wl, const CUtensorMap* maps, const float* __restrict_
                   const double* __restrict__ b, float* r32, float* x32, float* z32,
                   InstState* outer, InstState* inner, double* partials, double atol, double rtol,
                   double delta, int maxiter, int max_outer, int* err) {
+    grid_trigger();
+    grid_wait();
     // Replacement launches with no image flagged (most iterations) end here:
     // err[kPendingSlot] counts the images k_cg_update flagged.
     if (!FIRST && *(volatile int*)(err + kPendingSlot) == 0) return;
@@ -1208,9 +1212,9 @@ k_refine_residual(WorkList wl, const CUtensorMap* maps, const float* __restrict_
         }
     };
     auto flush = [&](const Meta& m, unsigned int mine) {
-        InstState* so = outer + m.inst;
-        InstState* si = inner + m.inst;
-        cta_flush<3>(v, partials, m.inst, m.t0, m.t1, mine, so, s_red, [&](double* sum) {
+        volatile InstState* so = outer + m.inst;
+        volatile InstState* si = inner + m.inst;
+        cta_flush<3>(v, partials, m.inst, m.t0, m.t1, mine, outer + m.inst, s_red, [&](double* sum) {
             const double nr = sqrt(sum[1]);
             if (FIRST) {
                 const double nb = sqrt(sum[0]);
@@ -1222,8 +1226,8 @@ k_refine_residual(WorkList wl, const CUtensorMap* maps, const float* __restrict_
                 si->flags = kFirst;
                 si->beta = 0.0;
             } else {
-                so->iters += 1;
-                si->flags &= ~kUpdate;
+                so->iters = so->iters + 1;
+                si->flags = si->flags & ~kUpdate;
                 atomicSub(err + kPendingSlot, 1);
             }
             so->norm_r = nr;
@@ -1254,6 +1258,8 @@ k_refine_residual(WorkList wl, const CUtensorMap* maps, const float* __restrict_
 template <int GATE>
 __global__ void __launch_bounds__(kThreads)
 k_refine_correct(WorkList wl, double* x64, float* x32, const InstState* st, const int* pending) {
+    grid_trigger();
+    grid_wait();
     if (GATE == kGateUpdate && *(volatile const int*)pending == 0) return;
     auto body = [&](const GridDesc& g, int64_t e0, int64_t e1) {
 #pragma unroll
@@ -1262,7 +1268,7 @@ k_refine_correct(WorkList wl, double* x64, float* x32, const InstState* st, cons
             if (e >= e1) break;
             if ((int)(e % g.pitch) >= g.w) continue;
             const int64_t i = g.voff + e;
-            x64[i] += (double)x32[i];
+            x64[i] = __ldcg(x64 + i) + (double)__ldcg(x32 + i);
             x32[i] = 0.0f;
         }
     };
@@ -1363,9 +1369,17 @@ k_vc_tail(const TailDesc<T>* __restrict__ descs, const InstState* st, double ome
     __shared__ TailDesc<T> D;
     __shared__ int s_off[kMaxTailLevels + 1];
     __shared__ __align__(8) uint64_t s_bar;
+    grid_trigger();
     if (threadIdx.x == 0) D = descs[blockIdx.x];
     __syncthreads();
-    if (st && st[D.inst].status != kRunning) return;   // uniform over the CTA
+    // Planes are fetched before the wait for the kernel that writes b, unless
+    // the image looked finished already (it then still is, or its solve has
+    // only just begun: the loads follow the wait).
+    const bool early = !st || *(volatile const int*)&st[D.inst].status == kRunning;
+    if (!__syncthreads_or(early)) {
+        grid_wait();
+        if (__ldcg(&st[D.inst].status) != kRunning) return;   // uniform over the CTA
+    }
     const int nlev = D.nlev;
     T* sm = reinterpret_cast<T*>(g_smem);
     if (threadIdx.x == 0) {
@@ -1386,10 +1400,12 @@ k_vc_tail(const TailDesc<T>* __restrict__ descs, const InstState* st, double ome
             bulk_load(sm + s_off[l], D.lev[l].P + g.poff,
                       (uint32_t)(kNH * g.pstride * sizeof(T)), &s_bar);
         }
+        grid_wait();
         const GridDesc g0 = D.lev[0].g;
         bulk_load(sm + s_off[0] + kNH * g0.pstride, D.lev[0].b + g0.voff,
                   (uint32_t)(g0.pstride * sizeof(T)), &s_bar);
     }
+    grid_wait();
     __syncthreads();
     const bool ok = mbar_wait(&s_bar, 0);
     if (__syncthreads_or(!ok)) {
@@ -1400,6 +1416,7 @@ k_vc_tail(const TailDesc<T>* __restrict__ descs, const InstState* st, double ome
         }
         return;
     }
+    if (st && __ldcg(&st[D.inst].status) != kRunning) return;   // finished meanwhile
     auto planes = [&](int l) { return sm + s_off[l]; };
     auto vb = [&](int l) { return sm + s_off[l] + kNH * D.lev[l].g.pstride; };
     auto vx = [&](int l) { return vb(l) + D.lev[l].g.pstride; };
@@ -1511,7 +1528,7 @@ k_vc_tail(const TailDesc<T>* __restrict__ descs, const InstState* st, double ome
 template <typename T>
 void launch_vc_tail(const TailDesc<T>* descs, int count, size_t smem, const InstState* st,
                     double omega, int* err, cudaStream_t s) {
-    if (count > 0) k_vc_tail<T><<<count, kTailThreads, smem, s>>>(descs, st, omega, err);
+    if (count > 0) launch_chain(k_vc_tail<T>, count, kTailThreads, smem, s, descs, st, omega, err);
 }
 
 // Shared-memory sizes; they follow the SmemCarve layout of each kernel (two
@@ -1569,9 +1586,9 @@ void launch_cg_update(int prec, const LaunchCfg& L, const WorkList& wl, const T*
                       T* z, const T* p0, const T* p1, const T* Ap, T* dr, int reorth, int reliable,
                       int* pending, InstState* st, double* part, cudaStream_t s) {
     switch (prec) {
-    case kPrecNone: k_cg_update<T, kPrecNone><<<L.grid, kThreads, 0, s>>>(wl, P, x, r, z, p0, p1, Ap, dr, reorth, reliable, pending, st, part); break;
-    case kPrecJacobi: k_cg_update<T, kPrecJacobi><<<L.grid, kThreads, 0, s>>>(wl, P, x, r, z, p0, p1, Ap, dr, reorth, reliable, pending, st, part); break;
-    default: k_cg_update<T, kPrecVcycle><<<L.grid, kThreads, 0, s>>>(wl, P, x, r, z, p0, p1, Ap, dr, reorth, reliable, pending, st, part); break;
+    case kPrecNone: launch_chain(k_cg_update<T, kPrecNone>, L.grid, kThreads, 0, s, wl, P, x, r, z, p0, p1, Ap, dr, reorth, reliable, pending, st, part); break;
+    case kPrecJacobi: launch_chain(k_cg_update<T, kPrecJacobi>, L.grid, kThreads, 0, s, wl, P, x, r, z, p0, p1, Ap, dr, reorth, reliable, pending, st, part); break;
+    default: launch_chain(k_cg_update<T, kPrecVcycle>, L.grid, kThreads, 0, s, wl, P, x, r, z, p0, p1, Ap, dr, reorth, reliable, pending, st, part); break;
     }
 }
 
@@ -1679,25 +1696,24 @@ void launch_refine_residual(int prec, int first, const LaunchCfg& L, const WorkL
                             double delta, int maxiter, int max_outer, int* err,
                             cudaStream_t s) {
     const size_t sm = smem_init<double>();
-#define PMB_RR(PK, F)                                                                           \
-    k_refine_residual<PK, F><<<L.grid, kTileThreads, sm, s>>>(wl, maps, P32, b, r32, x32, z32,  \
-                                                              outer, inner, part, atol, rtol,   \
-                                                              delta, maxiter, max_outer, err)
-    if (first) {
-        if (prec == kPrecNone) PMB_RR(kPrecNone, true);
-        else if (prec == kPrecJacobi) PMB_RR(kPrecJacobi, true);
-        else PMB_RR(kPrecVcycle, true);
-    } else {
-        if (prec == kPrecNone) PMB_RR(kPrecNone, false);
-        else if (prec == kPrecJacobi) PMB_RR(kPrecJacobi, false);
-        else PMB_RR(kPrecVcycle, false);
-    }
+    // The first one follows the writers of the planes: a plain launch.
+#define PMB_RR_ARGS wl, maps, P32, b, r32, x32, z32, outer, inner, part, atol, rtol, delta,     \
+                    maxiter, max_outer, err
+#define PMB_RR(PK)                                                                              \
+    do {                                                                                        \
+        if (first) k_refine_residual<PK, true><<<L.grid, kTileThreads, sm, s>>>(PMB_RR_ARGS);   \
+        else launch_chain(k_refine_residual<PK, false>, L.grid, kTileThreads, sm, s, PMB_RR_ARGS); \
+    } while (0)
+    if (prec == kPrecNone) PMB_RR(kPrecNone);
+    else if (prec == kPrecJacobi) PMB_RR(kPrecJacobi);
+    else PMB_RR(kPrecVcycle);
 #undef PMB_RR
+#undef PMB_RR_ARGS
 }
 
 void launch_refine_correct(const LaunchCfg& L, const WorkList& wl, double* x64, float* x32,
                            const InstState* inner, const int* pending, cudaStream_t s) {
-    if (inner) k_refine_correct<kGateUpdate><<<L.grid, kThreads, 0, s>>>(wl, x64, x32, inner, pending);
+    if (inner) launch_chain(k_refine_correct<kGateUpdate>, L.grid, kThreads, 0, s, wl, x64, x32, inner, pending);
     else k_refine_correct<kGateRunning><<<L.grid, kThreads, 0, s>>>(wl, x64, x32, nullptr, pending);
 }
 

@@ -69,21 +69,21 @@ struct RowList {
 };
 
 enum : int { kRowsApply = 0, kRowsDown = 1, kRowsUp = 2 };
-// Useful columns of a strip (coarse columns for kRowsDown); vec = 2 or 4.
-int rows_strip(int kind, int vec);
-template <typename T> int rows_resident_of(int kind, int vec);
+// Useful columns of a strip (coarse columns for kRowsDown), resident CTAs.
+template <typename T> int rows_strip(int kind);
+template <typename T> int rows_resident_of(int kind);
 void prepare_rows();
 
 // rev: CTAs take the table from its end, so that a pass starts with what the
 // pass before it left in L2. st == nullptr: every image, no reduction.
 template <typename T>
-void launch_rows_apply(int vec, const RowList& R, int rev, const T* P, const T* z, T* p0, T* p1,
+void launch_rows_apply(const RowList& R, int rev, const T* P, const T* z, T* p0, T* p1,
                        T* Ap, InstState* st, double* part, cudaStream_t s);
 template <typename T>
-void launch_rows_down(int vec, const RowList& R, int rev, const GridDesc* fine, const T* P, const T* b,
+void launch_rows_down(const RowList& R, int rev, const GridDesc* fine, const T* P, const T* b,
                       T* bc, double omega, const InstState* st, cudaStream_t s);
 template <typename T>
-void launch_rows_up(int vec, const RowList& R, int rev, const GridDesc* coarse, const T* P, const T* b,
+void launch_rows_up(const RowList& R, int rev, const GridDesc* coarse, const T* P, const T* b,
                     const T* xc, T* xout, double omega, InstState* st, int level0, const T* dr,
                     int reorth, double* part, cudaStream_t s);
 

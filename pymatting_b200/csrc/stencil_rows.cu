@@ -9,7 +9,7 @@
 // their dx once and kept. So every plane value is read from memory once per
 // strip, no operand or plane is read back from shared memory at another
 // lane's address, and no barrier stands between rows. The outer lanes (one on
-// each side, V >= 2) only feed their neighbours: a strip yields 30 V columns.
+// each side) only feed their neighbours: a strip yields 30 V columns.
 //
 // Rows come through a private ring: every lane copies its own V elements of
 // the 13 planes and the operand rows with cp.async, kAhead rows before it
@@ -25,7 +25,7 @@
 // barriers of each tile. Level 0 of 64 images (73 Mpix, FP32), tile kernels
 // and these: apply 0.70 and 0.87 of the measured copy bandwidth, restriction
 // 0.56 and 0.90, prolongation 0.58 and 0.75; one V-cycle of 1920x1080 in FP64
-// 352 and 310 us.
+// 352 and 310 us (251 us with the programmatic launches of pm_common.cuh).
 //
 // Work is cut into units of `seg` rows of one strip, kUnitWarps units per
 // CTA; one CTA per entry of the unit table, so that the hardware scheduler
@@ -41,27 +41,21 @@ namespace {
 constexpr int kAhead = 2;              // rows in flight ahead of the current one
 constexpr int kRing = kAhead + 1;
 
-// Resident CTAs that the registers must allow: the ring's shared memory
-// allows as many.
-template <typename T, int V> constexpr int kRowCtas = sizeof(T) * V == 8 ? 4 : 2;
+constexpr int kRowCtas = 2;            // resident CTAs; the ring's shared memory allows as many
+// Columns per lane: one 16-byte vector.
+template <typename T> constexpr int kVec = 16 / sizeof(T);
 
 template <typename T, int V>
 __device__ __forceinline__ void copy_async(T* dst, const T* src, int n) {
     // n bytes of the V elements are read, the others are zero-filled.
     constexpr int B = sizeof(T) * V;
     const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    if constexpr (B == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n)
-                     : "memory");
-    else if constexpr (B == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n)
-                     : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n)
-                     : "memory");
+    static_assert(B == 16, "cp.async.cg copies 16 bytes");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
 
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -97,7 +91,7 @@ struct Unit {
 
 template <int V, int SW, int LEAD>
 __device__ __forceinline__ Unit unit_of(const RowList& R, const int4& d, int cta, const GridDesc& g,
-                                        int scale, int rows) {
+                                        int rows) {
     Unit u;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = d.y + warp;
@@ -115,14 +109,16 @@ __device__ __forceinline__ Unit unit_of(const RowList& R, const int4& d, int cta
     return u;
 }
 
-// V elements of row y of a pitched array (zero outside the image).
-template <typename T, int V>
+// V elements of row y of a pitched array (zero outside the image). MUT: the
+// array is written by other kernels of the chain.
+template <typename T, int V, bool MUT>
 __device__ __forceinline__ void load_row(const T* base, int pitch, int y, int h, const Unit& u,
                                          T (&o)[V]) {
 #pragma unroll
     for (int v = 0; v < V; ++v) o[v] = T(0);
     if (u.nv > 0 && y >= 0 && y < h) {
-        ldv<T, V>(base + (int64_t)y * pitch + u.col, o);
+        if (MUT) ldv_l2<T, V>(base + (int64_t)y * pitch + u.col, o);
+        else ldv<T, V>(base + (int64_t)y * pitch + u.col, o);
 #pragma unroll
         for (int v = 1; v < V; ++v)
             if (v >= u.nv) o[v] = T(0);
@@ -149,11 +145,11 @@ __device__ __forceinline__ void back_init(Back<T, V>& B, const T* P, const GridD
     T c[V];
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
-        load_row<T, V>(P + (8 + k) * g.pstride, g.pitch, y - 2, g.h, u, c);
+        load_row<T, V, false>(P + (8 + k) * g.pstride, g.pitch, y - 2, g.h, u, c);
         shift_plane<T, V>(c, k - 2, B.b2[k]);
-        load_row<T, V>(P + (8 + k) * g.pstride, g.pitch, y - 1, g.h, u, c);
+        load_row<T, V, false>(P + (8 + k) * g.pstride, g.pitch, y - 1, g.h, u, c);
         shift_plane<T, V>(c, k - 2, B.b2n[k]);
-        load_row<T, V>(P + (3 + k) * g.pstride, g.pitch, y - 1, g.h, u, c);
+        load_row<T, V, false>(P + (3 + k) * g.pstride, g.pitch, y - 1, g.h, u, c);
         shift_plane<T, V>(c, k - 2, B.b1[k]);
     }
 }
@@ -207,6 +203,12 @@ __device__ __forceinline__ void roll(T (&W)[5][N]) {
         for (int j = 0; j < N; ++j) W[k][j] = W[k + 1][j];
 }
 
+// Whether an image is running, as far as can be told before grid_wait (it may
+// finish, or its solve may begin, while this kernel waits); warp-uniform.
+__device__ __forceinline__ bool looks_running(const InstState* s) {
+    return __any_sync(0xffffffffu, *(volatile const int*)&s->status == kRunning);
+}
+
 extern __shared__ __align__(128) char r_smem[];
 
 // The lane's slot of ring row `r`, array `k` (NA arrays of 32 V elements).
@@ -228,56 +230,73 @@ template <int V> __host__ __device__ constexpr int strip_coarse() { return 29 * 
 // alpha = rz / (p . Ap) (cg.py:85-90, 111-113). CG = false: y = A x alone.
 // --------------------------------------------------------------------------
 
-template <typename T, int V, bool CG>
-__global__ void __launch_bounds__(kUnitWarps * 32, kRowCtas<T, V>)
-k_rows_apply(RowList R, int rev, const T* __restrict__ Pl, const T* __restrict__ z, T* p0, T* p1,
+template <typename T, bool CG>
+__global__ void __launch_bounds__(kUnitWarps * 32, kRowCtas)
+k_rows_apply(RowList R, int rev, const T* __restrict__ Pl, const T* z, T* p0, T* p1,
              T* Ap, InstState* st, double* partials) {
-    constexpr int NA = kNH + (CG ? 2 : 1);
+    constexpr int V = kVec<T>, NA = kNH + (CG ? 2 : 1);
     __shared__ double s_red[32];
+    grid_trigger();
     const int cta = rev ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
     const int4 d = R.cta[cta];
     const GridDesc g = R.grids[d.x];
+    const Unit u = unit_of<V, strip_cols<V>(), 1>(R, d, cta, g, g.h);
+    const T* P = Pl + g.poff;
+    const int nb = u.nv * (int)sizeof(T);
+    int64_t orow = (int64_t)u.y0 * g.pitch + u.at;               // next row to issue
+    Back<T, V> B;
+    auto planes_row = [&](int r, int64_t o) {
+        T* dst = ring_at<T, V, NA>(r, 0);
+#pragma unroll
+        for (int p = 0; p < kNH; ++p) copy_async<T, V>(dst + p * 32 * V, P + o + p * g.pstride, nb);
+    };
+    auto prefetch = [&]() {
+        if (!u.active) return;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (u.y0 + k < u.y1) planes_row(k, orow + k * g.pitch);
+        back_init<T, V>(B, P, g, u.y0, u);
+    };
+    const bool early = !CG || looks_running(st + g.inst);
+    if (early) prefetch();
+    grid_wait();
     bool first = true;
     int par = 0;
     T beta = T(0);
     if (CG) {
-        const InstState& s = st[g.inst];
-        if (s.status != kRunning) return;
-        first = (s.flags & kFirst) != 0;
-        par = s.iters & 1;
-        beta = (T)s.beta;
+        const volatile InstState* s = st + g.inst;
+        if (s->status != kRunning) {
+            copy_wait_all();
+            return;
+        }
+        first = (s->flags & kFirst) != 0;
+        par = s->iters & 1;
+        beta = (T)s->beta;
     }
-    const Unit u = unit_of<V, strip_cols<V>(), 1>(R, d, cta, g, 1, g.h);
+    if (!early) prefetch();
     double sum[1] = {0.0};
     if (u.active) {
-        const T* P = Pl + g.poff;
         const T* Z = z + g.voff;
         const T* Q = (par ? p1 : p0) + g.voff;
         T* pn = (par ? p0 : p1) + g.voff;
         T* ap = Ap + g.voff;
-        const int nb = u.nv * (int)sizeof(T);
-        const T* prow = P + (int64_t)u.y0 * g.pitch + u.at;      // next row to issue
-        int64_t orow = (int64_t)u.y0 * g.pitch + u.at;
         int ri = 0;
-        auto issue = [&](int y) {
+        auto issue = [&](int y, bool pl) {
             if (y < u.y1) {
+                if (pl) planes_row(ri, orow);
                 T* dst = ring_at<T, V, NA>(ri, 0);
-#pragma unroll
-                for (int p = 0; p < kNH; ++p) copy_async<T, V>(dst + p * 32 * V, prow + p * g.pstride, nb);
                 const bool ok = y + 2 < g.h;
                 const int64_t o2 = ok ? orow + 2 * g.pitch : orow;
                 copy_async<T, V>(dst + kNH * 32 * V, Z + o2, ok ? nb : 0);
                 if (CG && !first) copy_async<T, V>(dst + (kNH + 1) * 32 * V, Q + o2, ok ? nb : 0);
-                prow += g.pitch;
                 orow += g.pitch;
                 ri = ri + 1 == kRing ? 0 : ri + 1;
             }
             copy_commit();
         };
 #pragma unroll
-        for (int k = 0; k < kAhead; ++k) issue(u.y0 + k);
+        for (int k = 0; k < kAhead; ++k) issue(u.y0 + k, false);
         T W[5][V + 4];
-        Back<T, V> B;
         auto operand = [&](T (&zv)[V], const T (&qv)[V]) {
             if (CG && !first) {
 #pragma unroll
@@ -287,18 +306,17 @@ k_rows_apply(RowList R, int rev, const T* __restrict__ Pl, const T* __restrict__
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             T zv[V], qv[V];
-            load_row<T, V>(Z, g.pitch, u.y0 - 2 + k, g.h, u, zv);
-            if (CG && !first) load_row<T, V>(Q, g.pitch, u.y0 - 2 + k, g.h, u, qv);
+            load_row<T, V, true>(Z, g.pitch, u.y0 - 2 + k, g.h, u, zv);
+            if (CG && !first) load_row<T, V, true>(Q, g.pitch, u.y0 - 2 + k, g.h, u, qv);
             operand(zv, qv);
             widen<T, V>(zv, W[k + 1]);
         }
-        back_init<T, V>(B, P, g, u.y0, u);
         const int lane = threadIdx.x & 31;
         const bool out = lane >= 1 && lane < 31 && u.nv > 0;
         int r = 0;
 #pragma unroll 1
         for (int y = u.y0; y < u.y1; ++y) {
-            issue(y + kAhead);
+            issue(y + kAhead, true);
             copy_wait<kAhead>();
             roll(W);
             const T* row = ring_at<T, V, NA>(r, 0);
@@ -327,11 +345,11 @@ k_rows_apply(RowList R, int rev, const T* __restrict__ Pl, const T* __restrict__
         copy_wait<0>();
     }
     if (CG) {
-        InstState* s = st + g.inst;
-        tile_reduce<1>(sum, partials, gridDim.x, u.cta, u.c0, u.c1, s, s_red, [&](double* t) {
+        volatile InstState* s = st + g.inst;
+        tile_reduce<1>(sum, partials, gridDim.x, u.cta, u.c0, u.c1, st + g.inst, s_red, [&](double* t) {
             s->pap = t[0];
             s->alpha = s->rz / t[0];
-            s->flags &= ~kFirst;
+            s->flags = s->flags & ~kFirst;
         });
     }
 }
@@ -343,67 +361,89 @@ k_rows_apply(RowList R, int rev, const T* __restrict__ Pl, const T* __restrict__
 // columns; the residual rows of a unit are 2 Y0 - 1 .. 2 Y1 - 1.
 // --------------------------------------------------------------------------
 
-template <typename T, int V>
-__global__ void __launch_bounds__(kUnitWarps * 32, kRowCtas<T, V>)
+template <typename T>
+__global__ void __launch_bounds__(kUnitWarps * 32, kRowCtas)
 k_rows_down(RowList R, int rev, const GridDesc* fine, const T* __restrict__ Pl,
-            const T* __restrict__ b, T* bc, double omega, const InstState* st) {
-    constexpr int NA = kNH + 1;         // planes 1..12 of row y; plane 0 and b of row y + 2
+            const T* b, T* bc, double omega, const InstState* st) {
+    constexpr int V = kVec<T>, NA = kNH + 1;   // planes 1..12 of row y; plane 0 and b of row y + 2
+    grid_trigger();
     const int cta = rev ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
     const int4 d = R.cta[cta];
     const GridDesc gc = R.grids[d.x];
     const GridDesc g = fine[d.x];
-    if (st && st[g.inst].status != kRunning) return;
-    const Unit u = unit_of<V, 2 * strip_coarse<V>(), 2>(R, d, cta, g, 2, gc.h);
-    if (!u.active) return;
+    const Unit u = unit_of<V, 2 * strip_coarse<V>(), 2>(R, d, cta, g, gc.h);
     const T* P = Pl + g.poff;
-    const T* bf = b + g.voff;
-    const int ys = 2 * u.y0 - 1, ye = 2 * u.y1;      // residual rows ys .. ye - 1
+    const int ys = 2 * u.y0 - 1, ye = 2 * u.y1;      // residual rows ys .. ye - 1 (ye <= h)
     const int nb = u.nv * (int)sizeof(T);
-    int64_t orow = (int64_t)ys * g.pitch + u.at;         // next row to issue
-    int ri = 0;
-    auto issue = [&](int y) {
-        if (y < ye) {
-            T* dst = ring_at<T, V, NA>(ri, 0);
-            const bool ok = y >= 0;                      // ye <= h
-            const T* prow = P + (ok ? orow : (int64_t)u.at);
+    int64_t orow = (int64_t)ys * g.pitch + u.at;     // next row to issue
+    T W[5][V + 4], bb[3][V], dd[4][V];
+    Back<T, V> B;
+    auto planes_row = [&](int r, int y, int64_t o) {
+        T* dst = ring_at<T, V, NA>(r, 0);
+        const bool ok = y >= 0;
+        const T* prow = P + (ok ? o : (int64_t)u.at);
 #pragma unroll
-            for (int p = 1; p < kNH; ++p)
-                copy_async<T, V>(dst + p * 32 * V, prow + p * g.pstride, ok ? nb : 0);
+        for (int p = 1; p < kNH; ++p)
+            copy_async<T, V>(dst + p * 32 * V, prow + p * g.pstride, ok ? nb : 0);
+        const bool ok2 = y + 2 < g.h;
+        copy_async<T, V>(dst, P + (ok2 ? o + 2 * g.pitch : (int64_t)u.at), ok2 ? nb : 0);
+    };
+    // Planes of the first rows: before the wait for the kernel that writes b.
+    auto prefetch = [&]() {
+        if (!u.active) return;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (ys + k < ye) planes_row(k, ys + k, orow + k * g.pitch);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) load_row<T, V, false>(P, g.pitch, ys - 2 + k, g.h, u, dd[k]);
+        back_init<T, V>(B, P, g, ys, u);
+    };
+    const bool early = !st || looks_running(st + g.inst);
+    if (early) prefetch();
+    grid_wait();
+    if (st && __ldcg(&st[g.inst].status) != kRunning) {
+        copy_wait_all();
+        return;
+    }
+    if (!u.active) return;
+    if (!early) prefetch();
+    const T* bf = b + g.voff;
+    int ri = 0;
+    auto issue = [&](int y, bool pl) {
+        if (y < ye) {
+            if (pl) planes_row(ri, y, orow);
             const bool ok2 = y + 2 < g.h;
-            const int64_t o2 = ok2 ? orow + 2 * g.pitch : (int64_t)u.at;
-            copy_async<T, V>(dst, P + o2, ok2 ? nb : 0);
-            copy_async<T, V>(dst + kNH * 32 * V, bf + o2, ok2 ? nb : 0);
+            copy_async<T, V>(ring_at<T, V, NA>(ri, kNH), bf + (ok2 ? orow + 2 * g.pitch : (int64_t)u.at),
+                             ok2 ? nb : 0);
             orow += g.pitch;
             ri = ri + 1 == kRing ? 0 : ri + 1;
         }
         copy_commit();
     };
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) issue(ys + k);
+    for (int k = 0; k < kAhead; ++k) issue(ys + k, false);
     auto sweep = [&](const T (&bv)[V], const T (&dv)[V], int y, T (&x1)[V]) {
 #pragma unroll
         for (int v = 0; v < V; ++v)
             x1[v] = (y >= 0 && y < g.h && v < u.nv)
                         ? smooth_div<T>((T)omega * bv[v], dv[v]) : T(0);
     };
-    T W[5][V + 4], bb[3][V], dd[3][V];
-    Back<T, V> B;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        T bv[V], dv[V], x1[V];
-        load_row<T, V>(bf, g.pitch, ys - 2 + k, g.h, u, bv);
-        load_row<T, V>(P, g.pitch, ys - 2 + k, g.h, u, dv);
-        sweep(bv, dv, ys - 2 + k, x1);
+        T bv[V], x1[V];
+        load_row<T, V, true>(bf, g.pitch, ys - 2 + k, g.h, u, bv);
+        sweep(bv, dd[k], ys - 2 + k, x1);
         widen<T, V>(x1, W[k + 1]);
         if (k >= 2) {
 #pragma unroll
-            for (int v = 0; v < V; ++v) {
-                bb[k - 1][v] = bv[v];
-                dd[k - 1][v] = dv[v];
-            }
+            for (int v = 0; v < V; ++v) bb[k - 1][v] = bv[v];
         }
     }
-    back_init<T, V>(B, P, g, ys, u);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        dd[1][v] = dd[2][v];                         // dd[k] is the row bb[k] is
+        dd[2][v] = dd[3][v];
+    }
     const int lane = threadIdx.x & 31;
     const int X = u.col >> 1;
     const bool out = lane >= 2 && lane < 31 && X < gc.w;
@@ -413,7 +453,7 @@ k_rows_down(RowList R, int rev, const GridDesc* fine, const T* __restrict__ Pl,
     int r = 0;
 #pragma unroll 1
     for (int y = ys; y < ye; ++y) {
-        issue(y + kAhead);
+        issue(y + kAhead, true);
         copy_wait<kAhead>();
         roll(W);
 #pragma unroll
@@ -472,64 +512,80 @@ k_rows_down(RowList R, int rev, const GridDesc* fine, const T* __restrict__ Pl,
 // r . z with r = b (and (r - r_old) . z) and beta.
 // --------------------------------------------------------------------------
 
-template <typename T, int V>
-__global__ void __launch_bounds__(kUnitWarps * 32, kRowCtas<T, V>)
+template <typename T>
+__global__ void __launch_bounds__(kUnitWarps * 32, kRowCtas)
 k_rows_up(RowList R, int rev, const GridDesc* coarse, const T* __restrict__ Pl,
-          const T* __restrict__ b, const T* __restrict__ xc, T* xout, double omega, InstState* st,
-          int level0, const T* __restrict__ dr, int reorth, double* partials) {
-    // Ring row y: planes 1..12 of row y; plane 0, b and the second coarse
-    // parent row of row y + 2. A lane needs coarse columns X .. X + V / 2.
-    constexpr int NA = kNH + 1, NC = V / 2 + 1;
+          const T* b, const T* xc, T* xout, double omega, InstState* st,
+          int level0, const T* dr, int reorth, double* partials) {
+    // Ring row y: planes 1..12 of row y; plane 0 and b of row y + 2. The
+    // second parent row of row y + 2 comes through registers, one row ahead.
+    // A lane needs coarse columns X .. X + V / 2.
+    constexpr int V = kVec<T>, NA = kNH + 1, NC = V / 2 + 1;
     __shared__ double s_red[2 * 32];
+    grid_trigger();
     const int cta = rev ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
     const int4 d = R.cta[cta];
     const GridDesc g = R.grids[d.x];
     const GridDesc gc = coarse[d.x];
-    if (st && st[g.inst].status != kRunning) return;
-    const Unit u = unit_of<V, strip_cols<V>(), 1>(R, d, cta, g, 1, g.h);
+    const Unit u = unit_of<V, strip_cols<V>(), 1>(R, d, cta, g, g.h);
+    const T* P = Pl + g.poff;
+    const int nb = u.nv * (int)sizeof(T);
+    int64_t orow = (int64_t)u.y0 * g.pitch + u.at;               // next row to issue
+    T W[5][V + 4], bb[3][V], dd[4][V];
+    Back<T, V> B;
+    auto planes_row = [&](int r, int y, int64_t o) {
+        T* dst = ring_at<T, V, NA>(r, 0);
+#pragma unroll
+        for (int p = 1; p < kNH; ++p) copy_async<T, V>(dst + p * 32 * V, P + o + p * g.pstride, nb);
+        const bool ok2 = y + 2 < g.h;
+        copy_async<T, V>(dst, P + (ok2 ? o + 2 * g.pitch : o), ok2 ? nb : 0);
+    };
+    // Planes of the first rows: before the wait for the kernel that writes xc.
+    auto prefetch = [&]() {
+        if (!u.active) return;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (u.y0 + k < u.y1) planes_row(k, u.y0 + k, orow + k * g.pitch);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) load_row<T, V, false>(P, g.pitch, u.y0 - 2 + k, g.h, u, dd[k]);
+        back_init<T, V>(B, P, g, u.y0, u);
+    };
+    const bool early = !st || looks_running(st + g.inst);
+    if (early) prefetch();
+    grid_wait();
+    if (st && __ldcg(&st[g.inst].status) != kRunning) {
+        copy_wait_all();
+        return;
+    }
+    if (!early) prefetch();
     double sum[2] = {0.0, 0.0};
     if (u.active) {
-        const T* P = Pl + g.poff;
         const T* bf = b + g.voff;
         const T* cf = xc + gc.voff;
         T* xo = xout + g.voff;
         const int X = u.col >> 1;
-        T* cring = reinterpret_cast<T*>(r_smem) + kUnitWarps * kRing * NA * 32 * V +
-                   (threadIdx.x >> 5) * kRing * NC * 32 + (threadIdx.x & 31);
         bool cok[NC];
 #pragma unroll
         for (int j = 0; j < NC; ++j) cok[j] = X + j >= 0 && X + j < gc.w;
-        const int nb = u.nv * (int)sizeof(T);
-        int64_t orow = (int64_t)u.y0 * g.pitch + u.at;           // next row to issue
         int ri = 0;
-        auto issue = [&](int y) {
+        auto issue = [&](int y, bool pl) {
             if (y < u.y1) {
-                T* dst = ring_at<T, V, NA>(ri, 0);
-                const T* prow = P + orow;
-#pragma unroll
-                for (int p = 1; p < kNH; ++p) copy_async<T, V>(dst + p * 32 * V, prow + p * g.pstride, nb);
+                if (pl) planes_row(ri, y, orow);
                 const bool ok2 = y + 2 < g.h;
-                const int64_t o2 = ok2 ? orow + 2 * g.pitch : orow;
-                copy_async<T, V>(dst, P + o2, ok2 ? nb : 0);
-                copy_async<T, V>(dst + kNH * 32 * V, bf + o2, ok2 ? nb : 0);
-                const int Yc = (y + 3) >> 1;         // second parent row of row y + 2
-                const T* crow = cf + (Yc < gc.h ? (int64_t)Yc * gc.pitch : 0);
-#pragma unroll
-                for (int j = 0; j < NC; ++j)
-                    copy_async<T, 1>(cring + (ri * NC + j) * 32, crow + (cok[j] ? X + j : 0),
-                                     cok[j] && Yc < gc.h ? (int)sizeof(T) : 0);
+                copy_async<T, V>(ring_at<T, V, NA>(ri, kNH), bf + (ok2 ? orow + 2 * g.pitch : orow),
+                                 ok2 ? nb : 0);
                 orow += g.pitch;
                 ri = ri + 1 == kRing ? 0 : ri + 1;
             }
             copy_commit();
         };
 #pragma unroll
-        for (int k = 0; k < kAhead; ++k) issue(u.y0 + k);
-        T ca[NC], cb[NC];                            // parent rows of the newest row
+        for (int k = 0; k < kAhead; ++k) issue(u.y0 + k, false);
+        T ca[NC], cb[NC], cnext[NC];                 // parent rows of the newest row, and next
         auto coarse_row = [&](int Y, T (&c)[NC]) {
 #pragma unroll
             for (int j = 0; j < NC; ++j)
-                c[j] = cok[j] && Y >= 0 && Y < gc.h ? cf[(int64_t)Y * gc.pitch + X + j] : T(0);
+                c[j] = cok[j] && Y >= 0 && Y < gc.h ? __ldcg(cf + (int64_t)Y * gc.pitch + X + j) : T(0);
         };
         // x2 of row y from b, plane 0 and its parent rows: an even coordinate
         // has one parent (weight 2), an odd one two (weight 1); the second
@@ -554,15 +610,12 @@ k_rows_up(RowList R, int rev, const GridDesc* coarse, const T* __restrict__ Pl,
                 x2[v] = val;
             }
         };
-        T W[5][V + 4], bb[3][V], dd[3][V];
-        Back<T, V> B;
         coarse_row((u.y0 - 2) >> 1, cb);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int y = u.y0 - 2 + k;
-            T bv[V], dv[V], x2[V];
-            load_row<T, V>(bf, g.pitch, y, g.h, u, bv);
-            load_row<T, V>(P, g.pitch, y, g.h, u, dv);
+            T bv[V], x2[V];
+            load_row<T, V, true>(bf, g.pitch, y, g.h, u, bv);
             // Parent rows: y >> 1, and for odd rows the next one.
             T cn[NC];
             coarse_row((y + 1) >> 1, cn);
@@ -572,23 +625,25 @@ k_rows_up(RowList R, int rev, const GridDesc* coarse, const T* __restrict__ Pl,
                 else ca[j] = cn[j];
                 cb[j] = cn[j];
             }
-            prolong(bv, dv, y, x2);
+            prolong(bv, dd[k], y, x2);
             widen<T, V>(x2, W[k + 1]);
             if (k >= 2) {
 #pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    bb[k - 1][v] = bv[v];
-                    dd[k - 1][v] = dv[v];
-                }
+                for (int v = 0; v < V; ++v) bb[k - 1][v] = bv[v];
             }
         }
-        back_init<T, V>(B, P, g, u.y0, u);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            dd[1][v] = dd[2][v];                     // dd[k] is the row bb[k] is
+            dd[2][v] = dd[3][v];
+        }
+        coarse_row((u.y0 + 3) >> 1, cnext);
         const int lane = threadIdx.x & 31;
         const bool out = lane >= 1 && lane < 31 && u.nv > 0;
         int r = 0;
 #pragma unroll 1
         for (int y = u.y0; y < u.y1; ++y) {
-            issue(y + kAhead);
+            issue(y + kAhead, true);
             copy_wait<kAhead>();
             roll(W);
 #pragma unroll
@@ -603,11 +658,11 @@ k_rows_up(RowList R, int rev, const GridDesc* coarse, const T* __restrict__ Pl,
             ldv<T, V>(row, dd[2]);
 #pragma unroll
             for (int j = 0; j < NC; ++j) {
-                const T cn = cring[(r * NC + j) * 32];
                 if (y & 1) ca[j] = cb[j];
-                else ca[j] = cn;
-                cb[j] = cn;
+                else ca[j] = cnext[j];
+                cb[j] = cnext[j];
             }
+            if (y + 1 < u.y1) coarse_row((y + 4) >> 1, cnext);
             T x2[V];
             prolong(bb[2], dd[2], y + 2, x2);
             widen<T, V>(x2, W[4]);
@@ -622,7 +677,7 @@ k_rows_up(RowList R, int rev, const GridDesc* coarse, const T* __restrict__ Pl,
                         x3[v] = W[2][2 + v] + smooth_div<T>((T)omega * (bb[0][v] - ax[v]), dd[0][v]);
                         if (level0) {
                             sum[0] += (double)bb[0][v] * (double)x3[v];
-                            if (reorth) sum[1] += (double)dr[g.voff + i + v] * (double)x3[v];
+                            if (reorth) sum[1] += (double)__ldcg(dr + g.voff + i + v) * (double)x3[v];
                         }
                     } else {
                         x3[v] = T(0);
@@ -649,16 +704,11 @@ k_rows_up(RowList R, int rev, const GridDesc* coarse, const T* __restrict__ Pl,
 
 namespace {
 
-template <typename T, int V> constexpr size_t ring_bytes(int na) {
-    return (size_t)kUnitWarps * kRing * na * 32 * V * sizeof(T);
+template <typename T> constexpr size_t ring_bytes(int na) {
+    return (size_t)kUnitWarps * kRing * na * 32 * 16;
 }
-template <typename T, int V> constexpr size_t smem_rows_apply(bool cg) {
-    return ring_bytes<T, V>(kNH + (cg ? 2 : 1));
-}
-template <typename T, int V> constexpr size_t smem_rows_down() { return ring_bytes<T, V>(kNH + 1); }
-template <typename T, int V> constexpr size_t smem_rows_up() {
-    return ring_bytes<T, V>(kNH + 1) + (size_t)kUnitWarps * kRing * (V / 2 + 1) * 32 * sizeof(T);
-}
+template <typename T> constexpr size_t smem_apply(bool cg) { return ring_bytes<T>(kNH + (cg ? 2 : 1)); }
+template <typename T> constexpr size_t smem_cycle() { return ring_bytes<T>(kNH + 1); }
 
 template <typename K> int rows_resident(K kernel, size_t smem) {
     int n = 0;
@@ -669,84 +719,68 @@ template <typename K> int rows_resident(K kernel, size_t smem) {
     return n < 1 ? 1 : n;
 }
 
-template <typename T, int V> void prepare_rows_v() {
+template <typename T> void prepare_rows_t() {
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaFuncSetAttribute(k_rows_apply<T, V, true>, attr, (int)smem_rows_apply<T, V>(true));
-    cudaFuncSetAttribute(k_rows_apply<T, V, false>, attr, (int)smem_rows_apply<T, V>(false));
-    cudaFuncSetAttribute(k_rows_down<T, V>, attr, (int)smem_rows_down<T, V>());
-    cudaFuncSetAttribute(k_rows_up<T, V>, attr, (int)smem_rows_up<T, V>());
+    cudaFuncSetAttribute(k_rows_apply<T, true>, attr, (int)smem_apply<T>(true));
+    cudaFuncSetAttribute(k_rows_apply<T, false>, attr, (int)smem_apply<T>(false));
+    cudaFuncSetAttribute(k_rows_down<T>, attr, (int)smem_cycle<T>());
+    cudaFuncSetAttribute(k_rows_up<T>, attr, (int)smem_cycle<T>());
 }
 
 }  // namespace
 
 void prepare_rows() {
-    prepare_rows_v<double, 2>();
-    prepare_rows_v<float, 2>();
-    prepare_rows_v<float, 4>();
+    prepare_rows_t<double>();
+    prepare_rows_t<float>();
 }
 
-int rows_strip(int kind, int vec) {
-    return kind == kRowsDown ? 29 * vec / 2 : 30 * vec;
+template <typename T> int rows_strip(int kind) {
+    return kind == kRowsDown ? strip_coarse<kVec<T>>() : strip_cols<kVec<T>>();
 }
 
-template <typename T> int rows_resident_of(int kind, int vec) {
-    constexpr int VW = sizeof(T) == 4 ? 4 : 2;
-#define PMB_RES(V)                                                                             \
-    (kind == kRowsApply ? rows_resident(k_rows_apply<T, V, true>, smem_rows_apply<T, V>(true)) \
-     : kind == kRowsDown ? rows_resident(k_rows_down<T, V>, smem_rows_down<T, V>())            \
-                         : rows_resident(k_rows_up<T, V>, smem_rows_up<T, V>()))
-    return vec == 4 && VW == 4 ? PMB_RES(VW) : PMB_RES(2);
-#undef PMB_RES
+template <typename T> int rows_resident_of(int kind) {
+    return kind == kRowsApply  ? rows_resident(k_rows_apply<T, true>, smem_apply<T>(true))
+           : kind == kRowsDown ? rows_resident(k_rows_down<T>, smem_cycle<T>())
+                               : rows_resident(k_rows_up<T>, smem_cycle<T>());
 }
 
 template <typename T>
-void launch_rows_apply(int vec, const RowList& R, int rev, const T* P, const T* z, T* p0, T* p1,
-                       T* Ap, InstState* st, double* part, cudaStream_t s) {
-    constexpr int VW = sizeof(T) == 4 ? 4 : 2;
+void launch_rows_apply(const RowList& R, int rev, const T* P, const T* z, T* p0, T* p1, T* Ap,
+                       InstState* st, double* part, cudaStream_t s) {
     if (R.total <= 0) return;
-#define PMB_RA(V, CG)                                                                         \
-    k_rows_apply<T, V, CG><<<R.total, kUnitWarps * 32, smem_rows_apply<T, V>(CG), s>>>(       \
-        R, rev, P, z, p0, p1, Ap, st, part)
-    if (!st) {
-        if (vec == 4 && VW == 4) PMB_RA(VW, false);
-        else PMB_RA(2, false);
-    } else if (vec == 4 && VW == 4) PMB_RA(VW, true);
-    else PMB_RA(2, true);
-#undef PMB_RA
-}
-
-template <typename T>
-void launch_rows_down(int vec, const RowList& R, int rev, const GridDesc* fine, const T* P, const T* b,
-                      T* bc, double omega, const InstState* st, cudaStream_t s) {
-    constexpr int VW = sizeof(T) == 4 ? 4 : 2;
-    if (R.total <= 0) return;
-    if (vec == 4 && VW == 4)
-        k_rows_down<T, VW><<<R.total, kUnitWarps * 32, smem_rows_down<T, VW>(), s>>>(R, rev, fine, P, b, bc, omega, st);
+    if (st)
+        launch_chain(k_rows_apply<T, true>, R.total, kUnitWarps * 32, smem_apply<T>(true), s, R, rev, P,
+                     z, p0, p1, Ap, st, part);
     else
-        k_rows_down<T, 2><<<R.total, kUnitWarps * 32, smem_rows_down<T, 2>(), s>>>(R, rev, fine, P, b, bc, omega, st);
+        launch_chain(k_rows_apply<T, false>, R.total, kUnitWarps * 32, smem_apply<T>(false), s, R, rev,
+                     P, z, p0, p1, Ap, st, part);
 }
 
 template <typename T>
-void launch_rows_up(int vec, const RowList& R, int rev, const GridDesc* coarse, const T* P, const T* b,
+void launch_rows_down(const RowList& R, int rev, const GridDesc* fine, const T* P, const T* b, T* bc,
+                      double omega, const InstState* st, cudaStream_t s) {
+    if (R.total <= 0) return;
+    launch_chain(k_rows_down<T>, R.total, kUnitWarps * 32, smem_cycle<T>(), s, R, rev, fine, P, b, bc,
+                 omega, st);
+}
+
+template <typename T>
+void launch_rows_up(const RowList& R, int rev, const GridDesc* coarse, const T* P, const T* b,
                     const T* xc, T* xout, double omega, InstState* st, int level0, const T* dr,
                     int reorth, double* part, cudaStream_t s) {
-    constexpr int VW = sizeof(T) == 4 ? 4 : 2;
     if (R.total <= 0) return;
-    if (vec == 4 && VW == 4)
-        k_rows_up<T, VW><<<R.total, kUnitWarps * 32, smem_rows_up<T, VW>(), s>>>(
-            R, rev, coarse, P, b, xc, xout, omega, st, level0, dr, reorth, part);
-    else
-        k_rows_up<T, 2><<<R.total, kUnitWarps * 32, smem_rows_up<T, 2>(), s>>>(
-            R, rev, coarse, P, b, xc, xout, omega, st, level0, dr, reorth, part);
+    launch_chain(k_rows_up<T>, R.total, kUnitWarps * 32, smem_cycle<T>(), s, R, rev, coarse, P, b, xc,
+                 xout, omega, st, level0, dr, reorth, part);
 }
 
 #define PMB_ROWS_INST(T)                                                                          \
-    template int rows_resident_of<T>(int, int);                                                   \
-    template void launch_rows_apply<T>(int, const RowList&, int, const T*, const T*, T*, T*, T*,  \
+    template int rows_strip<T>(int);                                                              \
+    template int rows_resident_of<T>(int);                                                        \
+    template void launch_rows_apply<T>(const RowList&, int, const T*, const T*, T*, T*, T*,       \
                                        InstState*, double*, cudaStream_t);                        \
-    template void launch_rows_down<T>(int, const RowList&, int, const GridDesc*, const T*,        \
-                                      const T*, T*, double, const InstState*, cudaStream_t);      \
-    template void launch_rows_up<T>(int, const RowList&, int, const GridDesc*, const T*, const T*,\
+    template void launch_rows_down<T>(const RowList&, int, const GridDesc*, const T*, const T*,   \
+                                      T*, double, const InstState*, cudaStream_t);                \
+    template void launch_rows_up<T>(const RowList&, int, const GridDesc*, const T*, const T*,     \
                                     const T*, T*, double, InstState*, int, const T*, int,         \
                                     double*, cudaStream_t);
 PMB_ROWS_INST(float)
