@@ -126,7 +126,7 @@ cf_assemble_kernel(AssembleArgs a) {
     if (x >= w || y >= h) return;
     const int64_t i = (int64_t)y * w + x;
 
-    // Row accumulators. In the half mode only forward slots are needed.
+    // Row accumulators.
     double acc[NS];
 #pragma unroll
     for (int q = 0; q < NS; ++q) acc[q] = 0.0;
@@ -152,7 +152,6 @@ cf_assemble_kernel(AssembleArgs a) {
                 for (int jx = 0; jx < SZ; ++jx) {
                     const int ddy = wy - 2 * R + jy;   // (yj - yi)
                     const int ddx = wx - 2 * R + jx;   // (xj - xi)
-                    if (MODE == kModeHalf && half_index(ddy, ddx) < 0) continue;
                     const double* Ij = s_img + ((ty + 2 * R + ddy) * IW + (tx + 2 * R + ddx)) * 3;
                     double cj0 = Ij[0] - mu[0], cj1 = Ij[1] - mu[1], cj2 = Ij[2] - mu[2];
                     double temp = c0 * cj0 + c1 * cj1 + c2 * cj2;
@@ -191,17 +190,13 @@ cf_assemble_kernel(AssembleArgs a) {
             const int yj = y + dy, xj = x + dx;
             const bool in = (yj >= 0 && yj < h && xj >= 0 && xj < w);
             double v = in ? acc[slot] : 0.0;
-            if (MODE == kModeHalf) {
-                if (p == 0 && a.diag_mask && a.diag_mask[i]) v = v + a.diag_value;
+            // Hard constraints: keep only unknown-unknown couplings; a known
+            // pixel's row becomes the identity.
+            if (p == 0) {
+                v = ki ? 1.0 : v;
             } else {
-                // Hard constraints: keep only unknown-unknown couplings; a
-                // known pixel's row becomes the identity.
-                if (p == 0) {
-                    v = ki ? 1.0 : v;
-                } else {
-                    const bool kj = in ? a.known[(int64_t)yj * w + xj] != 0 : true;
-                    v = (ki || kj) ? 0.0 : v;
-                }
+                const bool kj = in ? a.known[(int64_t)yj * w + xj] != 0 : true;
+                v = (ki || kj) ? 0.0 : v;
             }
             a.planes[p * pstride + pi] = v;
         }
@@ -228,6 +223,234 @@ cf_assemble_kernel(AssembleArgs a) {
     }
 }
 
+// --------------------------------------------------------------------------
+// Radius 1: the reference's CSR rows and the half-stencil planes
+// --------------------------------------------------------------------------
+//
+// The same terms in the same order as cf_assemble_kernel<1, MODE>, arranged
+// for what bounds it, the FP64 pipe: 81 pair terms a pixel (45 for the
+// planes), of which the division by 9 was half. A warp owns 32 pixels of a
+// row; per window row it holds the three windows' means and M c_i in
+// registers and walks the pixels j that they cover, so an I_j is read once
+// for all three. Shared arrays are one plane per component (8-byte lanes next
+// to each other). CSR rows are staged in shared memory and leave as
+// contiguous runs: written slot by slot, every 32-byte sector went out in
+// four pieces. 1280x720 CSR: 377 -> 166 us; 1920x1080 planes: 335 -> 227 us
+// (FP64 pipe half busy; 16 warps per SM is what the registers allow).
+
+// x / 9, correctly rounded. RN(1/9) is 2^-54 (relative) below 1/9, so
+// q = RN(x RN(1/9)) is within one ulp of x / 9, its remainder is exact in one
+// fused multiply-add, and the corrected quotient is the rounded one
+// (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990). Outside the exponents where the remainder
+// cannot underflow: zero keeps its sign, anything else takes the division.
+__device__ __forceinline__ double div9(double x) {
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;
+    if (e >= 120 && e < 2040) {
+        const double y = 1.0 / 9.0;
+        const double q = x * y;
+        return __fma_rn(__fma_rn(-9.0, q, x), y, q);
+    }
+    return x == 0.0 ? x : x / 9.0;
+}
+
+// The same for x = 1 + temp, which is zero or at least 2^-53 (or not finite).
+__device__ __forceinline__ double div9_near1(double x) {
+    const double y = 1.0 / 9.0;
+    const double q = x * y;
+    const double r = __fma_rn(__fma_rn(-9.0, q, x), y, q);
+    return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000 ? q : r;
+}
+
+// Pixels of a CTA, and its warps: each takes two rows, so that the windows
+// (1.2 per pixel, 1.33 for one row a warp) fill the threads better.
+constexpr int kR1X = 32, kR1Y = 16, kR1Warps = 8, kR1Threads = 32 * kR1Warps;
+constexpr int kR1IW = kR1X + 4, kR1IH = kR1Y + 4;      // image tile
+constexpr int kR1WW = kR1X + 2, kR1WH = kR1Y + 2;      // window tile
+constexpr int kR1I = kR1IW * kR1IH, kR1W = kR1WW * kR1WH;
+
+// Shared memory (doubles): image 3, mean 3, M 6 components; CSR staging.
+constexpr size_t r1_smem(bool ell) {
+    return sizeof(double) * (3 * kR1I + 9 * kR1W + (ell ? kR1X * kR1Warps * 25 : 0));
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kR1Threads, 2)
+cf_assemble_r1(AssembleArgs a) {
+    extern __shared__ __align__(16) double r1_sm[];
+    __shared__ uint8_t s_known[kR1I], s_act[kR1W];
+    double* s_img = r1_sm;
+    double* s_mean = s_img + 3 * kR1I;
+    double* s_m = s_mean + 3 * kR1W;
+    const int h = a.h, w = a.w;
+    const int x0 = blockIdx.x * kR1X, y0 = blockIdx.y * kR1Y;
+    const int tid = threadIdx.x;
+    for (int q = tid; q < kR1I; q += kR1Threads) {
+        const int ly = q / kR1IW, lx = q - ly * kR1IW;
+        const int y = y0 - 2 + ly, x = x0 - 2 + lx;
+        const bool in = y >= 0 && y < h && x >= 0 && x < w;
+        const int64_t gi = (int64_t)y * w + x;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) s_img[c * kR1I + q] = in ? a.image[gi * 3 + c] : 0.0;
+        s_known[q] = in ? (a.known ? a.known[gi] : 0) : 1;
+    }
+    __syncthreads();
+    for (int q = tid; q < kR1W; q += kR1Threads) {
+        const int ly = q / kR1WW, lx = q - ly * kR1WW;
+        const int ky = y0 - 1 + ly, kx = x0 - 1 + lx;
+        bool act = ky >= 1 && ky < h - 1 && kx >= 1 && kx < w - 1;
+        const int at = ly * kR1IW + lx;
+        if (act) {
+            bool all_known = true;
+#pragma unroll
+            for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx) all_known = all_known && s_known[at + dy * kR1IW + dx];
+            act = !all_known;
+        }
+        s_act[q] = act;
+        if (!act) continue;
+        double mean[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            double s = 0.0;
+#pragma unroll
+            for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx) s += s_img[c * kR1I + at + dy * kR1IW + dx];
+            mean[c] = div9(s);
+            s_mean[c * kR1W + q] = mean[c];
+        }
+        double a00 = a.epsilon, a01 = 0.0, a02 = 0.0;
+        double a11 = a.epsilon, a12 = 0.0, a22 = a.epsilon;
+#pragma unroll
+        for (int dy = 0; dy < 3; ++dy) {
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+                const double* p = s_img + at + dy * kR1IW + dx;
+                const double c0 = p[0] - mean[0], c1 = p[kR1I] - mean[1], c2 = p[2 * kR1I] - mean[2];
+                a00 += c0 * c0;
+                a01 += c0 * c1;
+                a02 += c0 * c2;
+                a11 += c1 * c1;
+                a12 += c1 * c2;
+                a22 += c2 * c2;
+            }
+        }
+        a00 = div9(a00); a01 = div9(a01); a02 = div9(a02);
+        a11 = div9(a11); a12 = div9(a12); a22 = div9(a22);
+        const double det = a00 * a12 * a12 + a01 * a01 * a22 + a02 * a02 * a11
+                           - a00 * a11 * a22 - 2 * a01 * a02 * a12;
+        const double inv_det = 1.0 / det;
+        s_m[0 * kR1W + q] = (a12 * a12 - a11 * a22) * inv_det;
+        s_m[1 * kR1W + q] = (a01 * a22 - a02 * a12) * inv_det;
+        s_m[2 * kR1W + q] = (a02 * a11 - a01 * a12) * inv_det;
+        s_m[3 * kR1W + q] = (a02 * a02 - a00 * a22) * inv_det;
+        s_m[4 * kR1W + q] = (a00 * a12 - a01 * a02) * inv_det;
+        s_m[5 * kR1W + q] = (a01 * a01 - a00 * a11) * inv_det;
+    }
+    __syncthreads();
+
+    const int tx = tid & 31, warp = tid >> 5;
+    const int x = x0 + tx;
+    const bool in_img = x < w;
+    const int64_t pstride = (int64_t)h * a.pitch;
+    double* const src = s_m + 6 * kR1W + warp * (kR1X * 25);       // kModeEll
+    double* const stage = src + tx * 25;
+#pragma unroll 1
+    for (int ty = warp; ty < kR1Y && y0 + ty < h; ty += kR1Warps) {
+        const int y = y0 + ty;
+        const int64_t row = (int64_t)y * w;
+        const int ii = (ty + 2) * kR1IW + tx + 2;
+        const double i0 = s_img[ii], i1 = s_img[kR1I + ii], i2 = s_img[2 * kR1I + ii];
+        const bool diag = in_img && a.diag_mask && a.diag_mask[row + x];
+        double acc[25];
+#pragma unroll
+        for (int q = 0; q < 25; ++q) acc[q] = 0.0;
+        // Rows dy of slots are complete once window row wy = min(dy + 2, 2) is.
+        auto emit = [&](int dy) {
+#pragma unroll
+            for (int dx = -2; dx <= 2; ++dx) {
+                const int slot = (dy + 2) * 5 + dx + 2;
+                double v = acc[slot];
+                if (MODE == kModeEll) {
+                    if (dy == 0 && dx == 0 && diag) v = v + a.diag_value;
+                    stage[slot] = v;
+                } else if (half_index(dy, dx) >= 0) {
+                    if (!(y + dy < h && x + dx >= 0 && x + dx < w)) v = 0.0;
+                    if (dy == 0 && dx == 0 && diag) v = v + a.diag_value;
+                    if (in_img) a.planes[half_index(dy, dx) * pstride + (int64_t)y * a.pitch + x] = v;
+                }
+            }
+        };
+#pragma unroll
+        for (int wy = 0; wy < 3; ++wy) {
+            double mu[3][3], cc[3][3];
+            bool act[3];
+#pragma unroll
+            for (int wx = 0; wx < 3; ++wx) {
+                const int q = (ty + wy) * kR1WW + tx + wx;
+                act[wx] = s_act[q];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) mu[wx][c] = s_mean[c * kR1W + q];
+                const double* m = s_m + q;
+                const double s = i0 - mu[wx][0], t = i1 - mu[wx][1], u = i2 - mu[wx][2];
+                cc[wx][0] = m[0] * s + m[kR1W] * t + m[2 * kR1W] * u;
+                cc[wx][1] = m[kR1W] * s + m[3 * kR1W] * t + m[4 * kR1W] * u;
+                cc[wx][2] = m[2 * kR1W] * s + m[4 * kR1W] * t + m[5 * kR1W] * u;
+            }
+#pragma unroll
+            for (int dy = wy - 2; dy <= wy; ++dy) {
+#pragma unroll
+                for (int dx = -2; dx <= 2; ++dx) {
+                    if (MODE == kModeHalf && half_index(dy, dx) < 0) continue;
+                    const int j = ii + dy * kR1IW + dx;
+                    const double j0 = s_img[j], j1 = s_img[kR1I + j], j2 = s_img[2 * kR1I + j];
+#pragma unroll
+                    for (int wx = (dx > 0 ? dx : 0); wx <= (dx < 0 ? dx + 2 : 2); ++wx) {
+                        const double c0 = j0 - mu[wx][0], c1 = j1 - mu[wx][1], c2 = j2 - mu[wx][2];
+                        const double temp = cc[wx][0] * c0 + cc[wx][1] * c1 + cc[wx][2] * c2;
+                        const double value = ((dy == 0 && dx == 0) ? 1.0 : 0.0) - div9_near1(1 + temp);
+                        if (act[wx]) acc[(dy + 2) * 5 + dx + 2] += value;
+                    }
+                }
+            }
+            if (MODE == kModeEll && wy < 2) emit(wy - 2);
+        }
+        emit(0);
+        emit(1);
+        emit(2);
+        if (MODE == kModeEll) {
+            __syncwarp();
+            const int nx = min(kR1X, w - x0);
+            const int64_t base = (row + x0) * 25;
+            for (int e = tx; e < nx * 25; e += 32) {
+                const int px = e / 25, slot = e - px * 25;
+                const int dy = slot / 5 - 2, dx = slot - (slot / 5) * 5 - 2;
+                const int yj = y + dy, xj = x0 + px + dx;
+                const bool in = yj >= 0 && yj < h && xj >= 0 && xj < w;
+                a.values[base + e] = src[e];
+                a.indices[base + e] = in ? (int64_t)yj * w + xj : 0;
+            }
+            if (in_img) {
+                a.indptr[row + x + 1] = (row + x + 1) * 25;
+                if (row + x == 0) a.indptr[0] = 0;
+            }
+            __syncwarp();
+        }
+    }
+}
+
+template <int MODE>
+static int launch_r1(const AssembleArgs& a, cudaStream_t s) {
+    const size_t smem = r1_smem(MODE == kModeEll);
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(cf_assemble_r1<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    dim3 grid((a.w + kR1X - 1) / kR1X, (a.h + kR1Y - 1) / kR1Y);
+    cf_assemble_r1<MODE><<<grid, kR1Threads, smem, s>>>(a);
+    return launch_status();
+}
+
 }  // namespace pmb
 
 using namespace pmb;
@@ -241,8 +464,8 @@ int pmb_launch_cf_ell(const double* image, const uint8_t* known, int h, int w, i
     a.values = values; a.indices = indices; a.indptr = indptr;
     a.diag_mask = diag_mask; a.diag_value = diag_value;
     dim3 grid((w + kAT - 1) / kAT, (h + kAT - 1) / kAT);
-    if (r == 1) cf_assemble_kernel<1, kModeEll><<<grid, kAT * kAT, 0, s>>>(a);
-    else if (r == 2) cf_assemble_kernel<2, kModeEll><<<grid, kAT * kAT, 0, s>>>(a);
+    if (r == 1) return launch_r1<kModeEll>(a, s);
+    if (r == 2) cf_assemble_kernel<2, kModeEll><<<grid, kAT * kAT, 0, s>>>(a);
     else return -1;
     return launch_status();
 }
@@ -253,9 +476,7 @@ int pmb_launch_cf_half(const double* image, const uint8_t* known, int h, int w, 
     AssembleArgs a = {};
     a.image = image; a.known = known; a.h = h; a.w = w; a.epsilon = eps;
     a.planes = planes; a.pitch = pitch; a.diag_mask = diag_mask; a.diag_value = diag_value;
-    dim3 grid((w + kAT - 1) / kAT, (h + kAT - 1) / kAT);
-    cf_assemble_kernel<1, kModeHalf><<<grid, kAT * kAT, 0, s>>>(a);
-    return launch_status();
+    return launch_r1<kModeHalf>(a, s);
 }
 
 int pmb_launch_cf_hard(const double* image, const uint8_t* known, const uint8_t* fg, int h,
