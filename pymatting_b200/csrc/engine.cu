@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -126,6 +127,73 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
+// What a solver object needs from the runtime: a stream, two events and
+// pinned host memory (per-image state, staging of descriptors). Making and
+// freeing these took 2 to 5 ms of a solve (cudaHostAlloc and cudaFreeHost
+// synchronise with the driver), so objects return them to a pool: at most
+// kPooled idle sets of kPinBytes each, a set held by one object at a time.
+struct SolverRes {
+    int device = -1;
+    cudaStream_t stream = nullptr;
+    cudaEvent_t ev_in = nullptr, ev_out = nullptr;
+    char* pin = nullptr;
+    size_t cap = 0;
+};
+constexpr size_t kPinBytes = 256 * 1024;
+constexpr size_t kPooled = 8;
+static std::mutex g_res_mutex;
+static std::vector<SolverRes> g_res_idle;
+
+static void free_res(SolverRes& r) {
+    if (r.stream) cudaStreamDestroy(r.stream);
+    if (r.ev_in) cudaEventDestroy(r.ev_in);
+    if (r.ev_out) cudaEventDestroy(r.ev_out);
+    if (r.pin) cudaFreeHost(r.pin);
+    r = SolverRes();
+}
+
+static int acquire_res(SolverRes& r, size_t bytes) {
+    int device = 0;
+    PMB_CUDA(cudaGetDevice(&device));
+    {
+        std::lock_guard<std::mutex> lock(g_res_mutex);
+        for (size_t i = 0; i < g_res_idle.size(); ++i)
+            if (g_res_idle[i].device == device && g_res_idle[i].cap >= bytes) {
+                r = g_res_idle[i];
+                g_res_idle.erase(g_res_idle.begin() + i);
+                return 0;
+            }
+    }
+    r = SolverRes();
+    r.device = device;
+    r.cap = std::max(bytes, kPinBytes);
+    auto make = [&]() -> int {
+        PMB_CUDA(cudaStreamCreateWithFlags(&r.stream, cudaStreamNonBlocking));
+        PMB_CUDA(cudaEventCreateWithFlags(&r.ev_in, cudaEventDisableTiming));
+        PMB_CUDA(cudaEventCreateWithFlags(&r.ev_out, cudaEventDisableTiming));
+        PMB_CUDA(cudaHostAlloc((void**)&r.pin, r.cap, cudaHostAllocDefault));
+        return 0;
+    };
+    const int rc = make();
+    if (rc) free_res(r);
+    return rc;
+}
+
+// Waits for the stream, then keeps or frees the set.
+static void release_res(SolverRes& r) {
+    if (!r.stream) return;
+    const bool ok = cudaStreamSynchronize(r.stream) == cudaSuccess;
+    if (ok && r.cap <= kPinBytes) {
+        std::lock_guard<std::mutex> lock(g_res_mutex);
+        if (g_res_idle.size() < kPooled) {
+            g_res_idle.push_back(r);
+            r = SolverRes();
+            return;
+        }
+    }
+    free_res(r);
+}
+
 struct HostList {
     std::vector<GridDesc> grids;     // descriptors of this list
     std::vector<GridDesc> partner;   // matching grid on the other level (or empty)
@@ -191,6 +259,7 @@ struct Stencil {
     size_t ws_bytes = 0;
     size_t o_state = 0, o_outer = 0, o_part = 0, o_uoff = 0, o_direct64 = 0, o_direct32 = 0;
     size_t o_inv = 0, o_invwork = 0, o_status = 0, o_err = 0, o_maps = 0;
+    size_t meta_lo = 0, meta_hi = 0;    // what bind uploads
     size_t o_b64 = 0, o_x64 = 0, o_r64 = 0, o_z64 = 0, o_p064 = 0, o_p164 = 0, o_ap64 = 0, o_dr64 = 0;
     size_t o_P032 = 0;
     size_t o_r32 = 0, o_z32 = 0, o_p032 = 0, o_p132 = 0, o_ap32 = 0, o_dr32 = 0, o_xin32 = 0;
@@ -198,10 +267,16 @@ struct Stencil {
     // bound state
     char* ws = nullptr;
     const double* P0 = nullptr;     // caller-owned level-0 FP64 planes
-    cudaStream_t stream = nullptr;
-    cudaEvent_t ev_in = nullptr, ev_out = nullptr;
-    InstState* h_state = nullptr;   // pinned copy of the per-image state
+    SolverRes res;
+    cudaStream_t stream = nullptr;  // res.stream
+    // Pinned copy of the per-image states and the error words, as they lie in
+    // the workspace.
+    InstState* h_state = nullptr;
     InstState* h_outer = nullptr;
+    int* h_err = nullptr;
+    bool stats_fresh = false;       // the copy is of the last solve's end
+    char* stage = nullptr;          // bind: host image of the workspace from meta_lo on
+    int64_t solves = 0;             // iterated solves so far
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
     int graph_reorth = -1;
@@ -464,8 +539,6 @@ static int plan_stencil(Stencil& S) {
     // Workspace layout.
     Carve c;
     const int64_t v0 = S.levels[0].vec_elems;
-    S.o_state = c.take<InstState>(n);
-    S.o_outer = c.take<InstState>(n);
     int64_t maxt = std::max<int64_t>(std::max(S.fine0.starts.back(), S.flat0.starts.back()),
                                      S.fine0.cta_cap);
     for (auto& lv : S.levels) {
@@ -479,9 +552,12 @@ static int plan_stencil(Stencil& S) {
     const int64_t gmax = std::min<int64_t>(maxt, 148 * kMaxCtasPerSm);
     S.partials_count = std::max<int64_t>(maxt, (int64_t)n * gmax);
     S.o_part = c.take<double>(3 * S.partials_count);
+    S.o_state = c.take<InstState>(2 * n + 1);          // inner, outer, error and status words
+    S.o_outer = S.o_state + sizeof(InstState) * n;
+    S.o_err = S.o_outer + sizeof(InstState) * n;
+    S.o_status = S.o_err + 4 * sizeof(int);
+    S.meta_lo = S.o_state;
     S.o_uoff = c.take<int64_t>(n + 1);
-    S.o_status = c.take<int>(4);
-    S.o_err = c.take<int>(4);
     S.o_maps = c.take<CUtensorMap>((int64_t)S.nmaps * kMapsPerGrid);
     carve_list(c, S.fine0);
     carve_list(c, S.flat0);
@@ -494,6 +570,7 @@ static int plan_stencil(Stencil& S) {
     S.o_tail = c.take<TailDesc<double>>((int64_t)S.tail_images.size());
     S.o_direct64 = c.take<DirectDesc>((int64_t)S.direct64.size());
     S.o_direct32 = c.take<DirectDesc>((int64_t)S.direct64.size());
+    S.meta_hi = c.off;
     S.o_inv = c.take<double>(S.direct_doubles);
     S.o_invwork = c.take<double>(S.direct_doubles);
     // Level-0 vectors. FP64 always holds b and x (the refinement iterate in
@@ -555,11 +632,17 @@ static void list_view(Stencil& S, HostList& L) {
     L.R.grids = L.wl.grids;
 }
 
-static int upload_rows(Stencil& S, HostList& L) {
-    if (!L.cta.empty())
-        PMB_CUDA(cudaMemcpyAsync(S.ws + L.d_cta, L.cta.data(), sizeof(int4) * L.cta.size(),
-                                 cudaMemcpyHostToDevice, S.stream));
+// `bytes` bytes to workspace offset `off`: into the staging image while bind
+// collects one, else copied on the solver's stream.
+static int upload(Stencil& S, size_t off, const void* src, size_t bytes) {
+    if (!bytes) return 0;
+    if (S.stage) std::memcpy(S.stage + (off - S.meta_lo), src, bytes);
+    else PMB_CUDA(cudaMemcpyAsync(S.ws + off, src, bytes, cudaMemcpyHostToDevice, S.stream));
     return 0;
+}
+
+static int upload_rows(Stencil& S, HostList& L) {
+    return L.rows < 0 ? 0 : upload(S, L.d_cta, L.cta.data(), sizeof(int4) * L.cta.size());
 }
 
 // After a knob of list L changed: its table again.
@@ -573,14 +656,9 @@ static int retune_rows(Stencil& S, HostList& L) {
 }
 
 static int upload_list(Stencil& S, HostList& L) {
-    if (!L.grids.empty())
-        PMB_CUDA(cudaMemcpyAsync(S.ws + L.d_grids, L.grids.data(), sizeof(GridDesc) * L.grids.size(),
-                                 cudaMemcpyHostToDevice, S.stream));
-    if (!L.partner.empty())
-        PMB_CUDA(cudaMemcpyAsync(S.ws + L.d_partner, L.partner.data(),
-                                 sizeof(GridDesc) * L.partner.size(), cudaMemcpyHostToDevice, S.stream));
-    PMB_CUDA(cudaMemcpyAsync(S.ws + L.d_starts, L.starts.data(), sizeof(int) * L.starts.size(),
-                             cudaMemcpyHostToDevice, S.stream));
+    if (int rc = upload(S, L.d_grids, L.grids.data(), sizeof(GridDesc) * L.grids.size())) return rc;
+    if (int rc = upload(S, L.d_partner, L.partner.data(), sizeof(GridDesc) * L.partner.size())) return rc;
+    if (int rc = upload(S, L.d_starts, L.starts.data(), sizeof(int) * L.starts.size())) return rc;
     list_view(S, L);
     return upload_rows(S, L);
 }
@@ -589,11 +667,11 @@ static int upload_list(Stencil& S, HostList& L) {
 // queued on the caller's stream and before anything queued there later.
 template <typename Fn>
 static int on_stream(Stencil& S, cudaStream_t caller, Fn fn) {
-    PMB_CUDA(cudaEventRecord(S.ev_in, caller));
-    PMB_CUDA(cudaStreamWaitEvent(S.stream, S.ev_in, 0));
+    PMB_CUDA(cudaEventRecord(S.res.ev_in, caller));
+    PMB_CUDA(cudaStreamWaitEvent(S.stream, S.res.ev_in, 0));
     int rc = fn();
-    PMB_CUDA(cudaEventRecord(S.ev_out, S.stream));
-    PMB_CUDA(cudaStreamWaitEvent(caller, S.ev_out, 0));
+    PMB_CUDA(cudaEventRecord(S.res.ev_out, S.stream));
+    PMB_CUDA(cudaStreamWaitEvent(caller, S.res.ev_out, 0));
     return rc;
 }
 
@@ -646,13 +724,18 @@ static int encode_grid_maps(Stencil& S, int l, const GridDesc& g, CUtensorMap* m
         XB = mixed ? (const void*)S.at<float>(lv.xb32) : (const void*)S.at<double>(lv.xb64);
     }
     int rc = 0;
-    rc |= encode_map(m + kMapPlF, P, g, true, mixed, kBW, kBH);
-    rc |= encode_map(m + kMapPlD, P, g, true, mixed, kBW, DH);
-    rc |= encode_map(m + kMapBF, B, g, false, mixed, kBW, kBH);
-    rc |= encode_map(m + kMapBD, B, g, false, mixed, kBW, DH);
-    rc |= encode_map(m + kMapXC, X, g, false, mixed, kCBW, kCBH);
-    rc |= encode_map(m + kMapXF, X, g, false, mixed, kBW, kBH);
     rc |= encode_map(m + kMapPlG, planes64(S, l), g, true, false, kGCols, kGRows);
+    // The default cycle's kernels address memory themselves; the tile kernels
+    // of other cycles, and level 0's initial residual, use the others.
+    const bool tiles = S.precond == kPrecVcycle && !(S.pre == 1 && S.post == 1);
+    if (l == 0 || tiles) rc |= encode_map(m + kMapPlF, P, g, true, mixed, kBW, kBH);
+    if (tiles) {
+        rc |= encode_map(m + kMapPlD, P, g, true, mixed, kBW, DH);
+        rc |= encode_map(m + kMapBF, B, g, false, mixed, kBW, kBH);
+        rc |= encode_map(m + kMapBD, B, g, false, mixed, kBW, DH);
+        rc |= encode_map(m + kMapXC, X, g, false, mixed, kCBW, kCBH);
+        rc |= encode_map(m + kMapXF, X, g, false, mixed, kBW, kBH);
+    }
     if (XA) {
         rc |= encode_map(m + kMapXAF, XA, g, false, mixed, kBW, kBH);
         rc |= encode_map(m + kMapXAD, XA, g, false, mixed, kBW, DH);
@@ -660,12 +743,8 @@ static int encode_grid_maps(Stencil& S, int l, const GridDesc& g, CUtensorMap* m
         rc |= encode_map(m + kMapXBD, XB, g, false, mixed, kBW, DH);
     }
     if (l == 0) {
-        const void* Z = X;
         const void* Q0 = mixed ? (const void*)S.at<float>(S.o_p032) : (const void*)S.at<double>(S.o_p064);
-        const void* Q1 = mixed ? (const void*)S.at<float>(S.o_p132) : (const void*)S.at<double>(S.o_p164);
-        rc |= encode_map(m + kMapZF, Z, g, false, mixed, kBW, kBH);
         rc |= encode_map(m + kMapP0F, Q0, g, false, mixed, kBW, kBH);
-        rc |= encode_map(m + kMapP1F, Q1, g, false, mixed, kBW, kBH);
         if (mixed) {
             rc |= encode_map(m + kMapX64F, S.at<double>(S.o_x64), g, false, false, kBW, kBH);
             rc |= encode_map(m + kMapP64F, S.P0, g, true, false, kBW, kBH);
@@ -713,10 +792,7 @@ static int encode_maps(Stencil& S, std::vector<CUtensorMap>& maps) {
 
 static int upload_tail(Stencil& S);
 
-static int bind_stencil(Stencil& S, void* ws, const double* P0) {
-    S.ws = reinterpret_cast<char*>(ws);
-    S.P0 = P0;
-    stencil_prepare();
+static int collect_meta(Stencil& S) {
     if (int rc = upload_list(S, S.fine0)) return rc;
     if (int rc = upload_list(S, S.flat0)) return rc;
     for (auto& lv : S.levels) {
@@ -725,13 +801,10 @@ static int bind_stencil(Stencil& S, void* ws, const double* P0) {
         if (int rc = upload_list(S, lv.flat)) return rc;
         if (int rc = upload_list(S, lv.gal)) return rc;
     }
-    PMB_CUDA(cudaMemcpyAsync(S.ws + S.o_uoff, S.user_off.data(), sizeof(int64_t) * S.user_off.size(),
-                             cudaMemcpyHostToDevice, S.stream));
+    if (int rc = upload(S, S.o_uoff, S.user_off.data(), sizeof(int64_t) * S.user_off.size())) return rc;
     std::vector<CUtensorMap> maps;
     if (int rc = encode_maps(S, maps)) return rc;
-    if (!maps.empty())
-        PMB_CUDA(cudaMemcpyAsync(S.ws + S.o_maps, maps.data(), sizeof(CUtensorMap) * maps.size(),
-                                 cudaMemcpyHostToDevice, S.stream));
+    if (int rc = upload(S, S.o_maps, maps.data(), sizeof(CUtensorMap) * maps.size())) return rc;
     // Direct descriptors: the inverse pointers are absolute.
     S.direct32 = S.direct64;
     for (size_t i = 0; i < S.direct64.size(); ++i) {
@@ -740,32 +813,59 @@ static int bind_stencil(Stencil& S, void* ws, const double* P0) {
         S.direct32[i].inv = S.direct64[i].inv;
         S.direct32[i].P = S.direct64[i].P;
     }
-    if (!S.direct64.empty()) {
-        PMB_CUDA(cudaMemcpyAsync(S.ws + S.o_direct64, S.direct64.data(),
-                                 sizeof(DirectDesc) * S.direct64.size(), cudaMemcpyHostToDevice, S.stream));
-        PMB_CUDA(cudaMemcpyAsync(S.ws + S.o_direct32, S.direct32.data(),
-                                 sizeof(DirectDesc) * S.direct32.size(), cudaMemcpyHostToDevice, S.stream));
+    if (int rc = upload(S, S.o_direct64, S.direct64.data(), sizeof(DirectDesc) * S.direct64.size())) return rc;
+    if (int rc = upload(S, S.o_direct32, S.direct32.data(), sizeof(DirectDesc) * S.direct32.size())) return rc;
+    return upload_tail(S);
+}
+
+// Everything the kernels read besides the planes goes up in one copy, from
+// pinned memory where it fits (states and error words start at zero).
+static int bind_stencil(Stencil& S, void* ws, const double* P0) {
+    S.ws = reinterpret_cast<char*>(ws);
+    S.P0 = P0;
+    stencil_prepare();
+    const size_t bytes = S.meta_hi - S.meta_lo, states = sizeof(InstState) * (2 * (size_t)S.nimg + 1);
+    std::vector<char> heap;
+    if (S.res.cap >= states + bytes) {
+        // A rebind must not overwrite the staging of a copy in flight.
+        if (S.bound) PMB_CUDA(cudaStreamSynchronize(S.stream));
+        S.stage = S.res.pin + states;
+        std::memset(S.stage, 0, bytes);
+    } else {
+        heap.assign(bytes, 0);
+        S.stage = heap.data();
     }
-    if (int rc = upload_tail(S)) return rc;
-    PMB_CUDA(cudaMemsetAsync(S.ws + S.o_state, 0, sizeof(InstState) * S.nimg, S.stream));
-    PMB_CUDA(cudaMemsetAsync(S.ws + S.o_outer, 0, sizeof(InstState) * S.nimg, S.stream));
-    PMB_CUDA(cudaMemsetAsync(S.ws + S.o_err, 0, sizeof(int) * 4, S.stream));
-    PMB_CUDA(cudaStreamSynchronize(S.stream));
+    const char* from = S.stage;
+    const int rc = collect_meta(S);
+    S.stage = nullptr;
+    if (rc) return rc;
+    PMB_CUDA(cudaMemcpyAsync(S.ws + S.meta_lo, from, bytes, cudaMemcpyHostToDevice, S.stream));
+    if (!heap.empty()) PMB_CUDA(cudaStreamSynchronize(S.stream));
     if (S.graph) {
         cudaGraphExecDestroy(S.graph);
         S.graph = nullptr;
     }
     S.bound = true;
     S.setup_done = false;
+    S.stats_fresh = false;
     return 0;
 }
 
-static int check_err(Stencil& S) {
-    int e = 0;
-    PMB_CUDA(cudaMemcpyAsync(&e, S.err(), sizeof(int), cudaMemcpyDeviceToHost, S.stream));
+static int read_states(Stencil& S) {
+    PMB_CUDA(cudaMemcpyAsync(S.h_state, S.state(), sizeof(InstState) * (2 * (size_t)S.nimg + 1),
+                             cudaMemcpyDeviceToHost, S.stream));
     PMB_CUDA(cudaStreamSynchronize(S.stream));
-    if (e) return fail(kErrState, "a TMA transfer did not complete in time");
     return 0;
+}
+
+// The error word of the last read_states.
+static int seen_err(Stencil& S) {
+    return S.h_err[0] ? fail(kErrState, "a TMA transfer did not complete in time") : 0;
+}
+
+static int check_err(Stencil& S) {
+    if (int rc = read_states(S)) return rc;
+    return seen_err(S);
 }
 
 static int setup_stencil(Stencil& S) {
@@ -792,9 +892,8 @@ static int setup_stencil(Stencil& S) {
                                S.levels[l].plane_elems, s);
     }
     PMB_CUDA(cudaGetLastError());
-    int status = 0;
-    PMB_CUDA(cudaMemcpyAsync(&status, S.ws + S.o_status, sizeof(int), cudaMemcpyDeviceToHost, s));
-    PMB_CUDA(cudaStreamSynchronize(s));
+    if (int rc = read_states(S)) return rc;
+    const int status = S.h_err[4];
     // A non-finite operator (non-finite image data) is not fatal here: the
     // solve stops that image alone with status kNonFinite.
     if (status == 2) return fail(kErrState, "coarsest multigrid operator is singular");
@@ -858,12 +957,8 @@ static int upload_tail_t(Stencil& S) {
         }
         t.inv = S.direct64[k].inv;
     }
-    if (!d.empty())
-        PMB_CUDA(cudaMemcpyAsync(S.ws + S.o_tail, d.data(), sizeof(TailDesc<T>) * d.size(),
-                                 cudaMemcpyHostToDevice, S.stream));
-    return 0;
+    return upload(S, S.o_tail, d.data(), sizeof(TailDesc<T>) * d.size());
 }
-
 static int upload_tail(Stencil& S) {
     if (S.tail_images.empty()) return 0;
     return S.precision == 1 ? upload_tail_t<float>(S) : upload_tail_t<double>(S);
@@ -1032,30 +1127,27 @@ static void cg_iteration(Stencil& S, int reorth) {
     if (S.precond == kPrecVcycle) run_vcycle<T>(S, v.r, v.z, st, v.dr, reorth);
 }
 
-static int read_states(Stencil& S, bool outer) {
-    PMB_CUDA(cudaMemcpyAsync(S.h_state, S.state(), sizeof(InstState) * S.nimg,
-                             cudaMemcpyDeviceToHost, S.stream));
-    if (outer)
-        PMB_CUDA(cudaMemcpyAsync(S.h_outer, S.outer(), sizeof(InstState) * S.nimg,
-                                 cudaMemcpyDeviceToHost, S.stream));
-    PMB_CUDA(cudaStreamSynchronize(S.stream));
-    return 0;
-}
-
 static bool any_running(const InstState* st, int n) {
     for (int k = 0; k < n; ++k)
         if (st[k].status == kRunning) return true;
     return false;
 }
 
-// Iterate until every image has left the running state. Iterations are
-// replayed from a CUDA graph of `chunk` iterations; images that finish early
-// turn the remaining kernels of the chunk into no-ops.
+// Iterate until every image has left the running state, `chunk` iterations
+// between looks at the states; images that finish early turn the remaining
+// kernels of the chunk into no-ops. A system's first solve launches its kernels
+// (the GPU takes longer than the host does, 13 launches of 2.5 us against 70 us
+// and more an iteration); one that is solved again replays a CUDA graph of the
+// chunk, whose capture and instantiation (0.3 ms, and 0.13 ms to drop it) only
+// then pay.
 template <typename T>
 static int iterate(Stencil& S, int reorth, int maxiter) {
     const int chunk = S.chunk;
-    if (!S.graph || S.graph_reorth != reorth || S.graph_iters != chunk ||
-        S.graph_delta != S.delta || S.graph_max_outer != S.max_outer) {
+    const bool replay = S.solves++ > 0;
+    S.stats_fresh = false;
+    if (!replay) S.pass = 0;
+    if (replay && (!S.graph || S.graph_reorth != reorth || S.graph_iters != chunk ||
+        S.graph_delta != S.delta || S.graph_max_outer != S.max_outer)) {
         if (S.graph) {
             cudaGraphExecDestroy(S.graph);
             S.graph = nullptr;
@@ -1079,14 +1171,19 @@ static int iterate(Stencil& S, int reorth, int maxiter) {
     }
     int done_iters = 0;
     for (;;) {
-        if (int rc = read_states(S, false)) return rc;
+        if (int rc = read_states(S)) return rc;
         if (!any_running(S.h_state, S.nimg)) break;
         if (done_iters > maxiter + chunk) return fail(kErrState, "iteration control lost");
-        PMB_CUDA(cudaGraphLaunch(S.graph, S.stream));
-        S.launches += S.graph_kernels;
+        if (replay) {
+            PMB_CUDA(cudaGraphLaunch(S.graph, S.stream));
+            S.launches += S.graph_kernels;
+        } else {
+            for (int i = 0; i < chunk; ++i) cg_iteration<T>(S, reorth);
+        }
         done_iters += chunk;
     }
-    return check_err(S);
+    S.stats_fresh = true;
+    return seen_err(S);
 }
 
 // Initial residual and first preconditioner apply of an FP64 solve.
@@ -1128,13 +1225,9 @@ static int start_mixed(Stencil& S, const double* x0, double atol, double rtol, i
     PMB_CUDA(cudaMemsetAsync(S.err() + kPendingSlot, 0, sizeof(int), s));
     // Outer state: every image starts running; its first FP64 residual sets
     // |b|, the tolerance and the first FP32 phase.
-    std::vector<InstState> init(S.nimg);
-    for (auto& o : init) {
-        std::memset(&o, 0, sizeof(o));
-        o.status = kRunning;
-    }
-    PMB_CUDA(cudaMemcpyAsync(S.outer(), init.data(), sizeof(InstState) * S.nimg,
-                             cudaMemcpyHostToDevice, s));
+    std::memset(S.h_outer, 0, sizeof(InstState) * S.nimg);
+    for (int k = 0; k < S.nimg; ++k) S.h_outer[k].status = kRunning;
+    PMB_CUDA(cudaMemcpyAsync(S.outer(), S.h_outer, sizeof(InstState) * S.nimg, cudaMemcpyHostToDevice, s));
     launch_refine_residual(S.precond, 1, LaunchCfg{grid_for(a, smem_init<double>())}, a.wl, S.maps(), v.P,
                            S.at<double>(S.o_b64), v.r, v.x, v.z, S.outer(), S.state(),
                            S.partials(), atol, rtol, inner_rtol, maxiter, max_outer, S.err(), s);
@@ -1153,8 +1246,8 @@ static int solve_mixed(Stencil& S, const double* x0, double atol, double rtol, i
     launch_refine_correct(LaunchCfg{persistent_grid(S.flat0)}, S.flat0.wl, x64, v.x, nullptr,
                           S.err() + kPendingSlot, S.stream);
     S.launches += 1;
-    if (int rc = read_states(S, true)) return rc;
-    return check_err(S);
+    if (int rc = read_states(S)) return rc;
+    return seen_err(S);
 }
 
 }  // namespace pmb
@@ -1557,11 +1650,11 @@ PMB_API int pmb_stencil_bind(pmb_stencil* p, void* workspace, const double* plan
     if (!p || !workspace || !planes64) return fail(kErrArg, "pmb_stencil_bind: bad arguments");
     Stencil& S = p->S;
     if (!S.stream) {
-        PMB_CUDA(cudaStreamCreateWithFlags(&S.stream, cudaStreamNonBlocking));
-        PMB_CUDA(cudaEventCreateWithFlags(&S.ev_in, cudaEventDisableTiming));
-        PMB_CUDA(cudaEventCreateWithFlags(&S.ev_out, cudaEventDisableTiming));
-        PMB_CUDA(cudaHostAlloc((void**)&S.h_state, sizeof(InstState) * 2 * S.nimg, cudaHostAllocDefault));
+        if (int rc = acquire_res(S.res, sizeof(InstState) * (2 * (size_t)S.nimg + 1))) return rc;
+        S.stream = S.res.stream;
+        S.h_state = reinterpret_cast<InstState*>(S.res.pin);
         S.h_outer = S.h_state + S.nimg;
+        S.h_err = reinterpret_cast<int*>(S.h_outer + S.nimg);
     }
     return on_stream(S, (cudaStream_t)stream, [&]() { return bind_stencil(S, workspace, planes64); });
 }
@@ -1655,7 +1748,8 @@ PMB_API int pmb_stencil_stats(pmb_stencil* p, int image, int* iters, int* status
                               double* norm_b, int* outer_iters) {
     if (!p || image < 0 || image >= p->S.nimg) return fail(kErrArg, "pmb_stencil_stats: bad image");
     Stencil& S = p->S;
-    if (int rc = read_states(S, true)) return rc;
+    if (!S.stats_fresh)
+        if (int rc = read_states(S)) return rc;
     // Mixed precision: the FP32 state carries the final status (convergence
     // is only declared on an FP64 residual); the norms are the FP64 ones.
     const InstState& st = S.precision == 1 ? S.h_outer[image] : S.h_state[image];
@@ -1749,14 +1843,8 @@ PMB_API int pmb_stencil_tuning(const pmb_stencil* p, int knob) {
 PMB_API int pmb_stencil_destroy(pmb_stencil* p) {
     if (!p) return 0;
     Stencil& S = p->S;
+    release_res(S.res);
     if (S.graph) cudaGraphExecDestroy(S.graph);
-    if (S.stream) {
-        cudaStreamSynchronize(S.stream);
-        cudaStreamDestroy(S.stream);
-    }
-    if (S.ev_in) cudaEventDestroy(S.ev_in);
-    if (S.ev_out) cudaEventDestroy(S.ev_out);
-    if (S.h_state) cudaFreeHost(S.h_state);
     delete p;
     return 0;
 }
@@ -2098,9 +2186,10 @@ struct Csr {
     char* ws = nullptr;
     size_t ws_bytes = 0, o_state = 0, o_part = 0;
     int nparts = 0;
-    cudaStream_t stream = nullptr;
-    cudaEvent_t ev_in = nullptr, ev_out = nullptr;
+    SolverRes res;
+    cudaStream_t stream = nullptr;   // res.stream
     InstState* h_state = nullptr;
+    int64_t solves = 0;
     cudaGraphExec_t graph = nullptr;
     int graph_reorth = -1;
     int reorth = 0;
@@ -2139,11 +2228,11 @@ static void csr_iteration(Csr& C, cudaStream_t s) {
 
 template <typename Fn>
 static int csr_on_stream(Csr& C, cudaStream_t caller, Fn fn) {
-    PMB_CUDA(cudaEventRecord(C.ev_in, caller));
-    PMB_CUDA(cudaStreamWaitEvent(C.stream, C.ev_in, 0));
+    PMB_CUDA(cudaEventRecord(C.res.ev_in, caller));
+    PMB_CUDA(cudaStreamWaitEvent(C.stream, C.res.ev_in, 0));
     int rc = fn();
-    PMB_CUDA(cudaEventRecord(C.ev_out, C.stream));
-    PMB_CUDA(cudaStreamWaitEvent(caller, C.ev_out, 0));
+    PMB_CUDA(cudaEventRecord(C.res.ev_out, C.stream));
+    PMB_CUDA(cudaStreamWaitEvent(caller, C.res.ev_out, 0));
     return rc;
 }
 
@@ -2199,10 +2288,9 @@ PMB_API int pmb_csr_bind(pmb_csr* p, void* workspace, double* vectors, const int
     C.invd = C.v(kVinvd);
     C.A = CsrMat{indptr, indices, data};
     if (!C.stream) {
-        PMB_CUDA(cudaStreamCreateWithFlags(&C.stream, cudaStreamNonBlocking));
-        PMB_CUDA(cudaEventCreateWithFlags(&C.ev_in, cudaEventDisableTiming));
-        PMB_CUDA(cudaEventCreateWithFlags(&C.ev_out, cudaEventDisableTiming));
-        PMB_CUDA(cudaHostAlloc((void**)&C.h_state, sizeof(InstState), cudaHostAllocDefault));
+        if (int rc = acquire_res(C.res, sizeof(InstState))) return rc;
+        C.stream = C.res.stream;
+        C.h_state = reinterpret_cast<InstState*>(C.res.pin);
     }
     if (C.graph) {
         cudaGraphExecDestroy(C.graph);
@@ -2242,7 +2330,8 @@ PMB_API int pmb_csr_solve(pmb_csr* p, const double* b, const double* x0, double*
     return csr_on_stream(C, (cudaStream_t)stream, [&]() -> int {
         if (int rc = csr_begin(C, b, x0, atol, rtol, maxiter, reorthogonalize)) return rc;
         const int chunk = 4;
-        if (!C.graph || C.graph_reorth != reorthogonalize) {
+        const bool replay = C.solves++ > 0;       // as in iterate()
+        if (replay && (!C.graph || C.graph_reorth != reorthogonalize)) {
             if (C.graph) cudaGraphExecDestroy(C.graph);
             C.graph = nullptr;
             cudaGraph_t g;
@@ -2258,7 +2347,9 @@ PMB_API int pmb_csr_solve(pmb_csr* p, const double* b, const double* x0, double*
             if (int rc = csr_read_state(C)) return rc;
             if (C.h_state->status != kRunning) break;
             if (done > maxiter + chunk) return fail(kErrState, "iteration control lost");
-            PMB_CUDA(cudaGraphLaunch(C.graph, C.stream));
+            if (replay) PMB_CUDA(cudaGraphLaunch(C.graph, C.stream));
+            else
+                for (int i = 0; i < chunk; ++i) csr_iteration(C, C.stream);
             done += chunk;
         }
         PMB_CUDA(cudaMemcpyAsync(x_out, C.v(kVx), sizeof(double) * C.n, cudaMemcpyDeviceToDevice, C.stream));
@@ -2345,14 +2436,8 @@ PMB_API int pmb_csr_stats(pmb_csr* p, int* iters, int* status, double* norm_r, d
 PMB_API int pmb_csr_destroy(pmb_csr* p) {
     if (!p) return 0;
     Csr& C = p->C;
+    release_res(C.res);
     if (C.graph) cudaGraphExecDestroy(C.graph);
-    if (C.stream) {
-        cudaStreamSynchronize(C.stream);
-        cudaStreamDestroy(C.stream);
-    }
-    if (C.ev_in) cudaEventDestroy(C.ev_in);
-    if (C.ev_out) cudaEventDestroy(C.ev_out);
-    if (C.h_state) cudaFreeHost(C.h_state);
     delete p;
     return 0;
 }
