@@ -710,10 +710,10 @@ def run_hard(args, rank, world, local):
                        "parallelism": "weak: one image per GPU, no collective"},
             "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s",
                          "frac": gbs / peak, "peak_source": peak_kind, "traffic": None,
-                         "kernel": "k_ichol_factor_cluster", "kernel_ms": f_ms,
+                         "kernel": "k_ichol_factor_pipe", "kernel_ms": f_ms,
                          "bytes_per_launch": alg_bytes,
                          "note": "latency-bound: the factor is a chain of one dependent "
-                                 "column per unknown (front on chip in a CTA cluster); bytes "
+                                 "column per unknown; bytes "
                                  "are A's lower part in and L out"},
             "e2e": {"value": world * npx / (e2e_ms * 1e-3) / 1e6, "unit": "Mpix/s",
                     "h2d_bytes_per_step": int(img.nbytes + tri.nbytes),

@@ -407,9 +407,9 @@ int pmb_ichol_factor(pmb_ichol* f, const int64_t* Ap, const int64_t* Ar, const d
                      int64_t* result, void* stream);
 /* Dependency levels of the factor (length of the triangular-solve schedule). */
 int pmb_ichol_levels(const pmb_ichol* f);
-/* CTAs of the cluster that held the factorisation's band front in
- * distributed shared memory in the last pmb_ichol_factor (1..8), 0 when the
- * front was in global memory (bandwidth too wide), -1 before any factor. */
+/* Size class of the last factor: the CTAs whose shared memory its band front
+ * would fill (1..8), 0 for more than 8 (bandwidth above 448), -1 before any
+ * factor. */
 int pmb_ichol_cluster(const pmb_ichol* f);
 /* Device time (CUDA events on the factor's stream) of the factorisation
  * kernel in the last pmb_ichol_factor, in milliseconds; -1 before any. */

@@ -1865,7 +1865,7 @@ struct Ichol {
     char* ws = nullptr;
     int64_t nnz = -1;
     int nlevels = 0;
-    int cluster = -1;     // CTAs holding the front in the last factorisation (0: global memory)
+    int cluster = -1;     // size class of the last factorisation (ichol_cluster_size)
     cudaEvent_t ev_f0 = nullptr, ev_f1 = nullptr;   // around the factor kernel
     float factor_ms = -1.0f;
     // Streamed solves (n <= kStreamMaxRows): chunk blocks of both sweeps.
@@ -1882,7 +1882,7 @@ static void plan_ichol(Ichol& I) {
     I.o_rsum = c.take<double>(n);
     I.o_level = c.take<int>(n);
     I.o_band = c.take<unsigned long long>(1);
-    I.o_F = c.take<double>(W * W);
+    I.o_F = c.take<double>(std::max(W, kPipeMinW) * std::max(W, kPipeMinW));
     I.o_pat = c.take<uint8_t>(W * W);
     I.o_cand = c.take<int>(W);
     I.o_keptv = c.take<double>(W);
@@ -2070,8 +2070,6 @@ PMB_API int pmb_ichol_factor(pmb_ichol* p, const int64_t* Ap, const int64_t* Ar,
     cudaStream_t s = (cudaStream_t)stream;
     const int64_t n = I.n, W = I.W;
     ichol_prepare();
-    PMB_CUDA(cudaMemsetAsync(I.ws + I.o_F, 0, sizeof(double) * W * W, s));
-    PMB_CUDA(cudaMemsetAsync(I.ws + I.o_pat, 0, (size_t)(W * W), s));
     ichol_launch_init(n, Ap, Ar, Av, shift, I.at<double>(I.o_d), I.at<double>(I.o_rsum),
                       I.at<int>(I.o_level), I.at<unsigned long long>(I.o_band), s);
     if (!I.ev_f0) {
@@ -2079,17 +2077,32 @@ PMB_API int pmb_ichol_factor(pmb_ichol* p, const int64_t* Ap, const int64_t* Ar,
         PMB_CUDA(cudaEventCreate(&I.ev_f1));
     }
     PMB_CUDA(cudaEventRecord(I.ev_f0, s));
-    I.cluster = ichol_launch_factor(n, W, Ap, Ar, Av, I.at<double>(I.o_d), I.at<double>(I.o_rsum),
-                        I.at<int>(I.o_level), I.at<double>(I.o_F), I.at<uint8_t>(I.o_pat),
-                        I.at<int>(I.o_cand), I.at<double>(I.o_keptv), I.at<int64_t>(I.o_kepti),
-                        I.at<int64_t>(I.o_Lp), I.at<int64_t>(I.o_Lr), I.at<double>(I.o_Lv), I.cap,
-                        discard_threshold, max_nnz, relative_discard_threshold, diag_keep_discarded,
-                        I.at<int64_t>(I.o_result), s);
-    PMB_CUDA(cudaGetLastError());
-    PMB_CUDA(cudaEventRecord(I.ev_f1, s));
-    int64_t res = 0;
-    PMB_CUDA(cudaMemcpyAsync(&res, I.ws + I.o_result, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    PMB_CUDA(cudaStreamSynchronize(s));
+    int64_t res = kIcholRetry;
+    I.cluster = ichol_cluster_size(W);
+    if (ichol_launch_factor_pipe(n, W, Ap, Ar, Av, I.at<double>(I.o_d), I.at<double>(I.o_rsum),
+                                 I.at<int>(I.o_level), I.at<int64_t>(I.o_Lp), I.at<int64_t>(I.o_Lr),
+                                 I.at<double>(I.o_Lv), I.at<double>(I.o_F), I.at<uint16_t>(I.o_Rc), I.cap,
+                                 discard_threshold, max_nnz, relative_discard_threshold, diag_keep_discarded,
+                                 I.at<int64_t>(I.o_result), s)) {
+        PMB_CUDA(cudaGetLastError());
+        PMB_CUDA(cudaEventRecord(I.ev_f1, s));
+        PMB_CUDA(cudaMemcpyAsync(&res, I.ws + I.o_result, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+        PMB_CUDA(cudaStreamSynchronize(s));
+    }
+    if (res == kIcholRetry) {
+        PMB_CUDA(cudaMemsetAsync(I.ws + I.o_F, 0, sizeof(double) * W * W, s));
+        PMB_CUDA(cudaMemsetAsync(I.ws + I.o_pat, 0, (size_t)(W * W), s));
+        ichol_launch_factor(n, W, Ap, Ar, Av, I.at<double>(I.o_d), I.at<double>(I.o_rsum),
+                            I.at<int>(I.o_level), I.at<double>(I.o_F), I.at<uint8_t>(I.o_pat),
+                            I.at<int>(I.o_cand), I.at<double>(I.o_keptv), I.at<int64_t>(I.o_kepti),
+                            I.at<int64_t>(I.o_Lp), I.at<int64_t>(I.o_Lr), I.at<double>(I.o_Lv), I.cap,
+                            discard_threshold, max_nnz, relative_discard_threshold, diag_keep_discarded,
+                            I.at<int64_t>(I.o_result), s);
+        PMB_CUDA(cudaGetLastError());
+        PMB_CUDA(cudaEventRecord(I.ev_f1, s));
+        PMB_CUDA(cudaMemcpyAsync(&res, I.ws + I.o_result, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+        PMB_CUDA(cudaStreamSynchronize(s));
+    }
     PMB_CUDA(cudaEventElapsedTime(&I.factor_ms, I.ev_f0, I.ev_f1));
     *result = res;
     I.nnz = res;

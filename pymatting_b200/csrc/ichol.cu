@@ -25,8 +25,6 @@
 // rows subtract their terms in the reference's order, levels separated by
 // block barriers (single CTA: the systems this preconditioner is used on
 // are the compressed unknown regions, tens of thousands of rows).
-#include <cooperative_groups.h>
-
 #include "pm_common.cuh"
 #include "ichol.cuh"
 #include "tma.cuh"
@@ -35,6 +33,7 @@ namespace pmb {
 
 constexpr int kIcholThreads = 1024;
 constexpr int kIcholChunks = 8;      // front columns of up to 256 rows load in one burst
+constexpr size_t kFactorSmem = 227 * 1024 - 256;
 constexpr int64_t kIcholSmemRows = 27 * 1024;   // x of the shared-memory solve: 216 KB
 
 // Per-column statistics of A (lower part, CSC): diagonal (+ shift), sum of
@@ -234,374 +233,460 @@ k_ichol_factor(int64_t n, int64_t W, const int64_t* __restrict__ Ap,
     if (threadIdx.x == 0) *result = s_fail ? (int64_t)s_fail : s_nnz;
 }
 
+// CTAs of shared memory that the W x W band front of FP64 values, pattern and
+// lists would fill; 0 above 8, or wider than 449. A size class of the system
+// that callers can ask for; the pipeline below holds no front.
+int ichol_cluster_size(int64_t W) {
+    if (W < 1 || W - 1 > 32 * 14) return 0;
+    const int64_t Wp = (W + 7) & ~(int64_t)7;
+    for (int64_t C = 1; C <= 8; ++C) {
+        const int64_t S = (W + C - 1) / C;
+        const int64_t bytes = S * Wp * 9 + S * 12 + W * 32;
+        if (((bytes + 15) & ~(int64_t)15) <= (int64_t)kFactorSmem) return (int)C;
+    }
+    return 0;
+}
+
 // ---------------------------------------------------------------------------
-// The same factorisation with the front on chip: a cluster of C CTAs keeps the
-// W x W front in distributed shared memory, CTA r owning the slots s with
-// s mod C = r (at most S = ceil(W / C) of them) with their FP64 values,
-// pattern bytes, ring entries of the diagonal d and of the dependency level.
-// Per column j:
+// The same factorisation, left-looking, as a pipeline of the warps of one CTA.
 //
-//   phase F  warp 0 of EVERY CTA reads slot j from its owner (one DSMEM round
-//            trip) and runs the serial part of the column (pivot, threshold,
-//            compaction) on identical data with identical instructions, so all
-//            CTAs hold the same kept list and take the same control path; the
-//            owner writes the column of L. Meanwhile the last warp recycles the
-//            slot of column j - 1 for column j - 1 + W from registers it loaded
-//            one column earlier (A's entries) and two columns earlier (A's
-//            column pointers), so no global load latency is on the chain.
-//   phase P  each CTA applies the pair updates F[ib][ia - ib] -= L_ia L_ib whose
-//            target column ib it owns, and the diagonal and level updates of
-//            the rows it owns: every write is CTA-local.
+//   walkers   the other warps, column j on walker j mod their number: A's entries
+//             of column j into an accumulator of W values in shared memory,
+//             then minus L_jk L_ik for every column k < j - kLag with a kept
+//             entry in row j, in ascending k, as those columns are done.
+//   finishers kFin warps, every column in turn, one offset below the pivot per
+//             lane (and chunk): the last kLag columns' terms from dense copies
+//             in shared memory, one quotient, thresholds, diagonal update, the
+//             entry's place in L and in its row's list.
+//   pivot     one warp: the next pivot's root and reciprocal while the
+//             finishers write the column, and the wait for the walker of the
+//             column after that.
 //
-// One cluster barrier per column orders phase P of column j before phase F of
-// column j + 1 in every CTA. Updates land in the same order as in
-// k_ichol_factor (column order, one pair per front entry per column), so the
-// two kernels produce identical factors.
+// What stays on the chain from one column to the next is the last term, the
+// root, the quotient and two barriers of the finishers and the pivot warp;
+// about 1,800 cycles, where the front spread over a cluster's shared memory
+// (every CTA reading, dividing and compacting the pivot column, then a cluster
+// barrier) took 4,300: 11,407 columns, 45 kept in each, 25.9 -> 10.9 ms.
+//
+// L itself, in global memory, is what the walkers read (one CTA: its columns
+// come from L1 or L2), so nothing limits the number of entries. Row i's list,
+// in ascending columns, has the place in L of each kept entry of row i, how
+// many entries of its column follow, and its offset; entries nearer than
+// kLag to the diagonal are not listed. Every subtraction of an entry runs in
+// ascending k with one rounding for the product and one for the difference, as
+// in the kernels above: the factors are identical.
+//
+// An accumulator or a dense copy that holds -0.0 has no entry (an entry is
+// never -0.0: A's are non-zero and every update ends with + 0.0).
 // ---------------------------------------------------------------------------
 
-constexpr int kClThreads = 512;
-constexpr int kClMaxChunks = 14;      // offsets 1 .. W - 1 in chunks of 32: W <= 449
-constexpr int kClMaxCluster = 8;      // portable cluster size
-constexpr size_t kClSmemLimit = 227 * 1024 - 256;
+constexpr int kPipeWarps = 24;        // finishers, pivot and walkers
+constexpr int kPipeThreads = 32 * kPipeWarps;
+constexpr int kLag = 4;
+constexpr int kDense = 8;             // dense columns kept (a power of two above kLag)
+constexpr int kPipeMaxChunks = 32;    // 32-offset chunks of a column: W <= 1025
+constexpr int kBatch = 2;             // nodes whose entries a walker has in flight
+constexpr uint32_t kPipeSpinLimit = 1u << 22;
+constexpr int kPipeStop = 0x7fffffff;
+constexpr int64_t kPipeMax = (int64_t)1 << 30;
 
-struct ClLayout {
-    int64_t Wp, S;
-    size_t o_F, o_d, o_kv, o_cL, o_lev, o_ki, o_ci, o_own, o_pre, o_pat, bytes;
+struct PipeLayout {
+    int Wp;
+    size_t o_dense, o_d, o_lev, o_pos, o_cnt, bytes;
 };
 
-__host__ __device__ inline ClLayout cl_layout(int64_t W, int C) {
-    ClLayout L;
-    L.Wp = (W + 7) & ~(int64_t)7;
-    L.S = (W + C - 1) / C;
-    size_t o = 0;
-    L.o_F = o;   o += (size_t)(L.S * L.Wp) * sizeof(double);
-    L.o_d = o;   o += (size_t)L.S * sizeof(double);
-    L.o_kv = o;  o += (size_t)W * sizeof(double);
-    L.o_cL = o;  o += (size_t)W * sizeof(double);
-    L.o_lev = o; o += (size_t)L.S * sizeof(int);
-    L.o_ki = o;  o += (size_t)W * sizeof(int);
-    L.o_ci = o;  o += (size_t)W * sizeof(int);
-    L.o_own = o; o += (size_t)W * sizeof(int);
-    L.o_pre = o; o += (size_t)W * sizeof(int);
-    L.o_pat = o; o += (size_t)(L.S * L.Wp);
+__host__ __device__ inline PipeLayout pipe_layout(int64_t W, int walkers) {
+    PipeLayout L;
+    L.Wp = (int)((W + kLag + 7) & ~(int64_t)7);
+    size_t o = (size_t)walkers * L.Wp * 8;
+    L.o_dense = o; o += (size_t)kDense * L.Wp * 8;
+    L.o_d = o;     o += (size_t)L.Wp * 8;
+    L.o_lev = o;   o += (size_t)L.Wp * 4;
+    L.o_pos = o;   o += (size_t)L.Wp * 4;
+    L.o_cnt = o;   o += (size_t)L.Wp * 4;
     L.bytes = (o + 15) & ~(size_t)15;
     return L;
 }
 
-// Smallest cluster size whose per-CTA share of the front fits in shared
-// memory; 0 when none up to the portable limit does (or W is too wide for
-// the register chunks of phase F).
-int ichol_cluster_size(int64_t W) {
-    if (W < 1 || W - 1 > 32 * kClMaxChunks) return 0;
-    for (int C = 1; C <= kClMaxCluster; ++C)
-        if (cl_layout(W, C).bytes <= kClSmemLimit) return C;
-    return 0;
+__device__ __forceinline__ void st_release(int* p, int v) {
+    asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
 }
 
-// NCH: 32-offset chunks of a front column held in registers by phase F
-// (ceil((W - 1) / 32) rounded up to 2, 4, 8 or 14). Slots are tracked
-// incrementally in 32-bit arithmetic. Phase F compacts the column's
-// candidates first and divides only those, lane-strided: an FP64 division
-// costs about 130 cycles of latency (about 300 with a zero numerator), and
-// a column has a quarter of its offsets as candidates or fewer.
-template <int NCH>
-__global__ void __launch_bounds__(kClThreads, 1)
-k_ichol_factor_cluster(int64_t n, int W, int C, const int64_t* __restrict__ Ap,
-                       const int64_t* __restrict__ Ar, const double* __restrict__ Av,
-                       const double* __restrict__ d0, const double* __restrict__ rsum,
-                       int* level, int64_t* Lp, int64_t* Lr, double* Lv, int64_t cap,
-                       double discard, int64_t max_nnz, double rel_discard, int diag_keep,
-                       int64_t* result) {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    extern __shared__ __align__(16) unsigned char cl_smem[];
-    __shared__ int64_t s_nnz;
-    __shared__ int s_cn, s_nown, s_np, s_levj, s_kept, s_owner, s_fail;
-    __shared__ double s_sj;
-    const ClLayout Ly = cl_layout(W, C);
-    const int S = (int)Ly.S, Wp = (int)Ly.Wp;
-    double* F = reinterpret_cast<double*>(cl_smem + Ly.o_F);
-    double* dl = reinterpret_cast<double*>(cl_smem + Ly.o_d);
-    double* kv = reinterpret_cast<double*>(cl_smem + Ly.o_kv);
-    double* cL = reinterpret_cast<double*>(cl_smem + Ly.o_cL);
-    int* lev = reinterpret_cast<int*>(cl_smem + Ly.o_lev);
-    int* ki = reinterpret_cast<int*>(cl_smem + Ly.o_ki);
-    int* ci = reinterpret_cast<int*>(cl_smem + Ly.o_ci);
-    int* own = reinterpret_cast<int*>(cl_smem + Ly.o_own);
-    int* pre = reinterpret_cast<int*>(cl_smem + Ly.o_pre);
-    uint8_t* pat = cl_smem + Ly.o_pat;
-    const int r = (int)cluster.block_rank();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const unsigned lt = (1u << lane) - 1u;
-    // Slot s belongs to CTA s mod C at local index s / C (interleaved, so the
-    // heavy targets just below the pivot spread over the cluster). s < 449
-    // and C <= 8: (s * mC) >> 16 with mC = ceil(65536 / C) is s / C exactly.
-    const int mC = (65536 + C - 1) / C;
-    auto divC = [mC](int v) { return (v * mC) >> 16; };
+template <int FIN>
+__device__ __forceinline__ void pipe_barrier(int id) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(32 * (FIN + 1)) : "memory");
+}
 
-    // Initial front: columns 0 .. min(W, n) - 1 sit in slots 0 .. W - 1.
-    for (int q = threadIdx.x; q < S * Wp; q += blockDim.x) {
-        F[q] = 0.0;
-        pat[q] = 0;
+// Exponents for which a quotient by `pipe_quotient` cannot leave the normal
+// range, nor its remainders.
+__device__ __forceinline__ bool mid_range(double x) {
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;
+    return e > 523 && e < 1523;
+}
+
+// a / b, correctly rounded, from y = RN(1 / b): a y is within two ulp, one
+// correction by its exact remainder makes it faithful and a second one the
+// rounded quotient (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990). For a zero or in the range above.
+__device__ __forceinline__ double pipe_quotient(double a, double b, double y) {
+    double q = a * y;
+    q = __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+__device__ __forceinline__ bool has_entry(double a) {
+    return __double_as_longlong(a) != (long long)0x8000000000000000ull;
+}
+
+// list: W x W nodes, row i's at slot i mod W; a node is the entry's place in
+// L and (entries of its column after it) << 16 | offset.
+template <int kFin, int M>
+__global__ void __launch_bounds__(kPipeThreads, 1)
+k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t* __restrict__ Ar,
+                    const double* __restrict__ Av, const double* __restrict__ d0,
+                    const double* __restrict__ rsum, int* level, int64_t* Lp, int64_t* Lr, double* Lv,
+                    int2* list, uint16_t* offs, int64_t cap, double discard, int64_t max_nnz, double rel_discard,
+                    int diag_keep, int64_t* result) {
+    extern __shared__ __align__(16) unsigned char pipe_smem[];
+    constexpr int kWalkers = kPipeWarps - 1 - kFin;
+    __shared__ __align__(16) int s_count[2][kFin * M];  // candidates << 16 | kept, per chunk
+    __shared__ double s_dj, s_sj, s_y;
+    __shared__ int s_ready[kWalkers];          // column whose accumulator is ready
+    __shared__ int s_done, s_stop;
+    __shared__ int64_t s_result;
+    const PipeLayout Ly = pipe_layout(W, kWalkers);
+    const int Wp = Ly.Wp;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned all = 0xffffffffu, lt = (1u << lane) - 1u;
+    double* accs = reinterpret_cast<double*>(pipe_smem);
+    double* dense = reinterpret_cast<double*>(pipe_smem + Ly.o_dense);
+    double* dl = reinterpret_cast<double*>(pipe_smem + Ly.o_d);
+    int* lev = reinterpret_cast<int*>(pipe_smem + Ly.o_lev);
+    int* rowpos = reinterpret_cast<int*>(pipe_smem + Ly.o_pos);   // finishers' list lengths
+    int* rowcnt = reinterpret_cast<int*>(pipe_smem + Ly.o_cnt);   // published list lengths
+
+    for (int q = threadIdx.x; q < kDense * Wp; q += blockDim.x) dense[q] = -0.0;
+    for (int q = threadIdx.x; q < Wp; q += blockDim.x) {
+        dl[q] = q < W && q < n ? d0[q] : 0.0;
+        lev[q] = 0;
+        rowpos[q] = rowcnt[q] = 0;
+    }
+    if (threadIdx.x < kWalkers) s_ready[threadIdx.x] = -1;
+    if (threadIdx.x == 0) {
+        s_done = -1;
+        s_stop = 0;
+        s_result = 0;
+        Lp[0] = 0;
     }
     __syncthreads();
-    for (int ls = warp; r + ls * C < W; ls += nw) {
-        const int64_t c = r + ls * C;
-        if (c >= n) continue;
-        for (int64_t k = Ap[c] + lane; k < Ap[c + 1]; k += 32) {
-            const int64_t i = Ar[k];
-            const double v = Av[k];
-            if (i > c && v != 0.0) {
-                F[ls * Wp + (int)(i - c)] = v;
-                pat[ls * Wp + (int)(i - c)] = 1;
-            }
-        }
-        if (lane == 0) {
-            dl[ls] = d0[c];
-            lev[ls] = 0;
-        }
-    }
-    if (threadIdx.x == 0) {
-        s_nnz = 0;
-        s_fail = 0;
-        if (r == 0) Lp[0] = 0;
-    }
-    cluster.sync();
 
-    // Last warp: A's column pointers of column j + W (loaded a column ahead)
-    // and entries of column j - 1 + W (loaded at the previous column).
-    int64_t pk0 = 0, pk1 = 0, ebeg = 0, eend = 0;
-    int64_t ei[2] = {-1, -1};
-    double ev[2] = {0.0, 0.0}, ed0 = 0.0;
-    if (warp == nw - 1 && W < n) {
-        pk0 = Ap[W];
-        pk1 = Ap[W + 1];
-    }
-    double rs_next = (warp == 0) ? rsum[0] : 0.0;
-    int slot = 0, pslot = W - 1;      // j % W and (j - 1) % W
-
-    for (int64_t j = 0; j < n; ++j) {
-        if (warp == 0) {
-            const int lsj = divC(slot), f = slot - lsj * C;
-            const double rs = rs_next;
-            if (j + 1 < n) rs_next = rsum[j + 1];
-            const double* Fj = cluster.map_shared_rank(F, f) + lsj * Wp;
-            const uint8_t* Pj = cluster.map_shared_rank(pat, f) + lsj * Wp;
-            const double dj = cluster.map_shared_rank(dl, f)[lsj];
-            const int levj = cluster.map_shared_rank(lev, f)[lsj];
-            // Offsets o = 1 + lane + 32 k: lane order is ascending rows, the
-            // order in which the reference sorts its candidates (ichol.py:87-89).
-            double a[NCH];
-            bool flag[NCH];
-#pragma unroll
-            for (int k = 0; k < NCH; ++k) {
-                const int o = 1 + lane + 32 * k;
-                const bool in = o < W && j + o < n;
-                a[k] = in ? Fj[o] : 0.0;
-                flag[k] = in && Pj[o] != 0;
+    if (warp > kFin) {
+        // ---- walker ----
+        const int me = warp - kFin - 1;
+        double* acc = accs + me * Wp;
+        int slot = me % W;
+        const int step = kWalkers % W;
+        bool stop = false;
+        for (int j = me; j < n && !stop; j += kWalkers) {
+            int64_t p0 = Ap[j];
+            const int64_t p1 = Ap[j + 1];
+            // First entries of the column while the accumulator is in use.
+            int64_t i0 = -1;
+            double v0 = 0.0;
+            if (p0 + lane < p1) {
+                i0 = Ar[p0 + lane];
+                v0 = Av[p0 + lane];
             }
-            unsigned fm[NCH];
-            int cn = 0;
-#pragma unroll
-            for (int k = 0; k < NCH; ++k) {
-                fm[k] = __ballot_sync(0xffffffffu, flag[k]);
-                cn += __popc(fm[k]);
-            }
-            const int64_t nnz = s_nnz;
-            int fail = 0;
-            if (!(dj > 0.0)) fail = -1;                                         // ichol.py:80-81
-            else if (nnz + 1 + cn > max_nnz || nnz + 1 + cn > cap) fail = -2;   // ichol.py:82-83
-            const bool owner = f == r;
-            const int64_t nnz0 = nnz + 1;
-            // Candidates in ascending rows: value and offset, compacted.
-            int cpos = 0;
-#pragma unroll
-            for (int k = 0; k < NCH; ++k) {
-                if (flag[k]) {
-                    const int q = cpos + __popc(fm[k] & lt);
-                    cL[q] = a[k];
-                    ci[q] = 1 + lane + 32 * k;
+            int at = 0;                  // nodes taken
+            bool fresh = false;          // the accumulator holds A's column
+            for (uint32_t spins = 0;; ++spins) {
+                const int done_ = *(volatile int*)&s_done;
+                const int cnt_ = *(volatile int*)&rowcnt[slot];
+                const int done = __shfl_sync(all, done_, 0);
+                int cnt = __shfl_sync(all, cnt_, 0);
+                if (done == kPipeStop || spins >= kPipeSpinLimit) {
+                    stop = true;
+                    break;
                 }
-                cpos += __popc(fm[k]);
+                // The accumulator is free once this walker's last column is
+                // done, the slot is row j's once column j - W is.
+                // Columns still to come before the list is complete: sleep for
+                // most of them (polls take the finishers' issue slots).
+                const int away = j - 1 - kLag - done;
+                if (done < j - kWalkers || done < j - W) {
+                    __nanosleep(200);
+                    continue;
+                }
+                __threadfence_block();
+                if (!fresh) {
+                    for (int o = lane; o < W; o += 32) acc[o] = -0.0;
+                    __syncwarp();
+                    if (i0 > j && v0 != 0.0) acc[i0 - j] = v0;
+                    for (int64_t k = p0 + 32 + lane; k < p1; k += 32) {
+                        const int64_t i = Ar[k];
+                        const double v = Av[k];
+                        if (i > j && v != 0.0) acc[i - j] = v;
+                    }
+                    __syncwarp();
+                    fresh = true;
+                }
+                if (at < cnt) {
+                    const int2* row = list + slot * W;
+                    for (int base = at; base < cnt; base += kBatch) {
+                        // Entries of kBatch nodes in flight (an L2 round trip
+                        // is ten times the work on one node).
+                        int2 node[kBatch];
+                        double f[kBatch], v[kBatch], v2[kBatch];
+                        int i[kBatch], i2[kBatch];
+#pragma unroll
+                        for (int q = 0; q < kBatch; ++q)
+                            node[q] = base + q < cnt ? row[base + q] : make_int2(0, 0);
+#pragma unroll
+                        for (int q = 0; q < kBatch; ++q) {
+                            const int rest = node[q].y >> 16;
+                            const double* Lg = Lv + node[q].x;
+                            const uint16_t* Ig = offs + node[q].x;
+                            f[q] = Lg[0];
+                            v[q] = v2[q] = 0.0;
+                            i[q] = i2[q] = 0;
+                            if (lane < rest) {
+                                v[q] = Lg[1 + lane];
+                                i[q] = Ig[1 + lane];
+                            }
+                            if (rest > 32 && lane + 32 < rest) {
+                                v2[q] = Lg[33 + lane];
+                                i2[q] = Ig[33 + lane];
+                            }
+                        }
+#pragma unroll
+                        for (int q = 0; q < kBatch; ++q) {
+                            const int rest = node[q].y >> 16;
+                            double* from = acc - (node[q].y & 0xffff);   // offsets are from column k
+                            if (lane < rest) {
+                                double* x = from + i[q];
+                                *x = (*x - v[q] * f[q]) + 0.0;
+                            }
+                            if (rest > 32 && lane + 32 < rest) {
+                                double* x = from + i2[q];
+                                *x = (*x - v2[q] * f[q]) + 0.0;
+                            }
+                            for (int c = 64 + lane; c < rest; c += 32) {
+                                double* x = from + offs[node[q].x + 1 + c];
+                                *x = (*x - Lv[node[q].x + 1 + c] * f[q]) + 0.0;
+                            }
+                            __syncwarp();
+                        }
+                    }
+                    at = cnt;
+                    spins = 0;
+                }
+                if (away <= 0) break;                 // the list was complete when read
+                __nanosleep(away > 4 ? 1000 : away > 1 ? 200 : 40);
             }
+            if (stop) break;
             __syncwarp();
-            int kept = 0, nown = 0;
-            if (!fail) {
-                const double sj = sqrt(dj);
-                const double rel = rel_discard * rs;
-                if (lane == 0) s_sj = sj;
-                // One quotient per candidate, lane-strided (the candidates
-                // of a column are a quarter of its offsets or fewer).
-                for (int t0 = 0; t0 < cn; t0 += 32) {
-                    const int t = t0 + lane;
-                    double L = 0.0;
-                    bool keep = false, mine = false;
-                    int o = 0;
-                    if (t < cn) {
-                        const double av = cL[t];
-                        o = ci[t];
-                        L = av / sj;
-                        keep = fabs(L) > discard && fabs(av) > rel;
-                        int sl = slot + o;
-                        if (sl >= W) sl -= W;
-                        mine = keep && sl - divC(sl) * C == r;
-                        cL[t] = L;
-                        ci[t] = keep ? o : -o;
-                    }
-                    const unsigned km = __ballot_sync(0xffffffffu, keep);
-                    const unsigned om = __ballot_sync(0xffffffffu, mine);
-                    if (keep) {
-                        const int pos = kept + __popc(km & lt);
-                        kv[pos] = L;
-                        ki[pos] = o;
-                        if (mine) own[nown + __popc(om & lt)] = pos;
-                    }
-                    kept += __popc(km);
-                    nown += __popc(om);
+            if (lane == 0) st_release(&s_ready[me], j);
+            slot += step;
+            if (slot >= W) slot -= W;
+        }
+    } else if (warp == kFin) {
+        // ---- pivot: s_dj, s_sj, s_y of column j + 1 between the barriers of
+        // column j, and the walker of column j + 2 ----
+        int ready = 0;                        // columns below are known to be ready
+        int wk = 0;
+        auto await = [&](int c) {             // accumulator of column c, c = ready
+            bool ok = false;
+            for (uint32_t spins = 0; spins < kPipeSpinLimit; ++spins) {
+                if (__shfl_sync(all, *(volatile int*)&s_ready[wk], 0) >= c) {
+                    ok = true;
+                    break;
                 }
+                __nanosleep(20);
             }
-            // Exclusive prefix of the owned targets' pair counts (kept - 1 -
-            // pb pairs for the target at kept index pb).
-            int np = 0;
-            for (int t0 = 0; t0 < nown; t0 += 32) {
-                const int t = t0 + lane;
-                const int cnt = t < nown ? kept - 1 - own[t] : 0;
-                int incl = cnt;
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, incl, d);
-                    if (lane >= d) incl += v;
-                }
-                if (t < nown) pre[t] = np + incl - cnt;
-                np += __shfl_sync(0xffffffffu, incl, 31);
+            __threadfence_block();
+            if (!ok && lane == 0) {
+                s_result = kIcholRetry;
+                s_stop = 1;
             }
+            ++ready;
+            wk = wk + 1 == kWalkers ? 0 : wk + 1;
+        };
+        auto root = [&](double d) {
+            const double s = sqrt(d);
+            const double y = 1.0 / s;
             if (lane == 0) {
-                s_fail = fail;
-                if (!fail) {
-                    s_cn = cn;
-                    s_nown = nown;
-                    s_np = np;
-                    s_levj = levj;
-                    s_kept = kept;
-                    s_owner = owner;
-                    s_nnz = nnz0 + kept;
-                }
+                s_dj = d;
+                s_sj = s;
+                s_y = y;
             }
-        } else if (warp == nw - 1) {
-            // Recycle slot (j - 1) % W for column c = j - 1 + W (its readers
-            // all passed the barrier of column j - 1).
-            const int64_t c = j - 1 + W;
-            const int pls = divC(pslot);
-            if (j >= 1 && c < n && pslot - pls * C == r) {
-                double* Fc = F + pls * Wp;
-                uint8_t* Pc = pat + pls * Wp;
-                for (int o = lane; o < W; o += 32) {
-                    Fc[o] = 0.0;
-                    Pc[o] = 0;
-                }
-                __syncwarp();
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int64_t k = ebeg + lane + 32 * e;
-                    if (k < eend && ei[e] > c && ev[e] != 0.0) {
-                        Fc[ei[e] - c] = ev[e];
-                        Pc[ei[e] - c] = 1;
-                    }
-                }
-                for (int64_t k = ebeg + 64 + lane; k < eend; k += 32) {   // rows longer than 64
-                    const int64_t i = Ar[k];
-                    const double v = Av[k];
-                    if (i > c && v != 0.0) {
-                        Fc[i - c] = v;
-                        Pc[i - c] = 1;
-                    }
-                }
-                if (lane == 0) {
-                    dl[pls] = ed0;
-                    lev[pls] = 0;
-                }
-            }
-            // Entries of column j + W for the next column's recycle.
-            if (j + W < n) {
-                ebeg = pk0;
-                eend = pk1;
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int64_t k = pk0 + lane + 32 * e;
-                    ei[e] = k < pk1 ? Ar[k] : -1;
-                    ev[e] = k < pk1 ? Av[k] : 0.0;
-                }
-                ed0 = d0[j + W];
-            }
-            // Column pointers of column j + 1 + W.
-            if (j + 1 + W < n) {
-                pk0 = Ap[j + 1 + W];
-                pk1 = Ap[j + 2 + W];
-            }
+        };
+        await(0);
+        if (n > 1) await(1);
+        root(dl[0]);
+        pipe_barrier<kFin>(2);
+        int slot = 1;
+        for (int j = 0; j < n && !*(volatile int*)&s_stop; ++j) {
+            pipe_barrier<kFin>(1);
+            if (j + 1 < n) root(dl[slot]);
+            if (j + 2 < n) await(j + 2);
+            pipe_barrier<kFin>(2);
+            // Column j - 1 is in its rows' lists.
+            if (lane == 0) st_release(&s_done, j - 1);
+            slot = slot + 1 == W ? 0 : slot + 1;
         }
-        __syncthreads();
-        if (s_fail) break;
-        // Phase P: CTA-local updates of the rows and front columns owned here.
-        // Pairs are spread evenly over the threads (target found by binary
-        // search of the prefix); the diagonal and level updates go to the
-        // threads with the fewest pairs.
-        const int nown = s_nown, cn = s_cn, np = s_np, lj = s_levj + 1;
-        // The owner of slot j writes column j of L from the kept list
-        // (threads 128.., which have the fewest pairs besides the diagonal
-        // and level updates).
-        if (s_owner) {
-            const int kept = s_kept;
-            const int64_t end = s_nnz, nnz = end - kept - 1;
-            for (int q = (int)((threadIdx.x + blockDim.x - 128) % blockDim.x); q <= kept;
-                 q += blockDim.x) {
-                if (q == 0) {
-                    Lv[nnz] = s_sj;
-                    Lr[nnz] = j;
-                    level[j] = s_levj;
-                    Lp[j + 1] = end;
+        if (lane == 0) st_release(&s_done, kPipeStop);
+    } else {
+        // ---- finishers: lane's offsets 1 + lane + 32 (warp + kFin m) ----
+        int slot = 0, wk = 0;
+        int64_t nnz = 0;
+        double dnext = W < n ? d0[W] : 0.0, rnow = rsum[0], rnext = n > 1 ? rsum[1] : 0.0;
+        int psl[M], pcnt[M];                 // list lengths to publish for the column before
+        double a[M];
+#pragma unroll
+        for (int m = 0; m < M; ++m) pcnt[m] = 0;
+        // The accumulator of column c and the terms of the dense columns.
+        auto gather = [&](int c) {
+            const double* acc = accs + wk * Wp;
+            wk = wk + 1 == kWalkers ? 0 : wk + 1;
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int o = 1 + lane + 32 * (warp + kFin * m);
+                a[m] = o < W ? acc[o] : -0.0;
+            }
+            double f[kLag], x[kLag][M];
+#pragma unroll
+            for (int b = kLag; b >= 1; --b) {
+                const double* dc = dense + ((c - b) & (kDense - 1)) * Wp;
+                f[b - 1] = dc[b];
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const int o = 1 + lane + 32 * (warp + kFin * m);
+                    x[b - 1][m] = o < W ? dc[o + b] : -0.0;
+                }
+            }
+#pragma unroll
+            for (int b = kLag; b >= 1; --b) {
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const double t = (a[m] - x[b - 1][m] * f[b - 1]) + 0.0;
+                    if (has_entry(f[b - 1]) && has_entry(x[b - 1][m])) a[m] = t;
+                }
+            }
+        };
+        pipe_barrier<kFin>(2);
+        if (!*(volatile int*)&s_stop) {
+            gather(0);
+            for (int j = 0; j < n; ++j) {
+                // Quotients, thresholds, diagonal updates, dense copy.
+                const double dj = s_dj, sj = s_sj, y = s_y;
+                const int levj = lev[slot];
+                int sl[M], lv[M], pos[M];
+                double du[M];
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const int o = 1 + lane + 32 * (warp + kFin * m);
+                    sl[m] = o >= W ? slot : slot + o >= W ? slot + o - W : slot + o;
+                    du[m] = dl[sl[m]];
+                    lv[m] = lev[sl[m]];
+                    pos[m] = rowpos[sl[m]];
+                }
+                const double rel = rel_discard * rnow;
+                double L[M];
+                bool keep[M];
+                bool odd = !mid_range(sj);
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    odd |= has_entry(a[m]) && !(a[m] == 0.0 || mid_range(a[m]));
+                    L[m] = pipe_quotient(a[m], sj, y);
+                }
+                if (__any_sync(all, odd)) {
+#pragma unroll
+                    for (int m = 0; m < M; ++m) L[m] = a[m] / sj;
+                }
+                unsigned km[M];
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const int o = 1 + lane + 32 * (warp + kFin * m);
+                    const bool in = has_entry(a[m]);
+                    keep[m] = in && fabs(L[m]) > discard && fabs(a[m]) > rel;
+                    if (in && (diag_keep || keep[m])) dl[sl[m]] = du[m] - L[m] * L[m];
+                    if (o < W) dense[(j & (kDense - 1)) * Wp + o] = keep[m] ? L[m] : -0.0;
+                    const unsigned fm = __ballot_sync(all, in);
+                    km[m] = __ballot_sync(all, keep[m]);
+                    if (lane == 0) s_count[j & 1][warp + kFin * m] = __popc(fm) << 16 | __popc(km[m]);
+                }
+                pipe_barrier<kFin>(1);
+                // Lengths of the lists that column j - 1 extended: its entries
+                // were written before the barrier.
+                __threadfence_block();
+#pragma unroll
+                for (int m = 0; m < M; ++m)
+                    if (pcnt[m]) *(volatile int*)&rowcnt[psl[m]] = pcnt[m];
+                // Places in L: chunks in ascending offsets.
+                int before[M], total = 0;
+#pragma unroll
+                for (int c = 0; c < kFin * M; ++c) {
+                    if (c % kFin == warp) before[c / kFin] = total & 0xffff;
+                    total += s_count[j & 1][c];
+                }
+                const int cn = total >> 16, kept = total & 0xffff;
+                int64_t fail = 0;
+                if (!(dj > 0.0)) fail = -1;                                              // ichol.py:80-81
+                else if (nnz + 1 + cn > max_nnz || nnz + 1 + cn > cap) fail = -2;        // ichol.py:82-83
+                if (fail) {
+                    if (threadIdx.x == 0) {
+                        s_result = fail;
+                        s_stop = 1;
+                    }
                 } else {
-                    Lv[nnz + q] = kv[q - 1];
-                    Lr[nnz + q] = j + ki[q - 1];
+#pragma unroll
+                    for (int m = 0; m < M; ++m) {
+                        pcnt[m] = 0;
+                        if (keep[m]) {
+                            const int o = 1 + lane + 32 * (warp + kFin * m);
+                            const int r = before[m] + __popc(km[m] & lt);
+                            const int64_t g = nnz + 1 + r;
+                            Lv[g] = L[m];
+                            Lr[g] = j + o;
+                            offs[g] = (uint16_t)o;
+                            if (lv[m] <= levj) lev[sl[m]] = levj + 1;
+                            if (o > kLag) {
+                                const int p = pos[m];
+                                rowpos[sl[m]] = p + 1;
+                                list[sl[m] * W + p] = make_int2((int)g, (kept - 1 - r) << 16 | o);
+                                psl[m] = sl[m];
+                                pcnt[m] = p + 1;
+                            }
+                        }
+                    }
+                    if (threadIdx.x == 0) {
+                        Lv[nnz] = sj;
+                        Lr[nnz] = j;
+                        Lp[j + 1] = nnz + 1 + kept;
+                        level[j] = levj;
+                        // The slot's next row.
+                        dl[slot] = dnext;
+                        lev[slot] = 0;
+                        rowpos[slot] = 0;
+                        *(volatile int*)&rowcnt[slot] = 0;
+                    }
+                    nnz += 1 + kept;
+                    slot = slot + 1 == W ? 0 : slot + 1;
+                    if (j + 1 < n) {
+                        rnow = rnext;
+                        if (j + 2 < n) rnext = rsum[j + 2];
+                        if (j + 1 + W < n) dnext = d0[j + 1 + W];
+                        gather(j + 1);
+                    }
                 }
+                pipe_barrier<kFin>(2);
+                if (*(volatile int*)&s_stop) break;
             }
         }
-        for (int p = threadIdx.x; p < np; p += blockDim.x) {
-            int tl = 0, th = nown - 1;
-            while (tl < th) {
-                const int mid = (tl + th + 1) >> 1;
-                if (pre[mid] <= p) tl = mid;
-                else th = mid - 1;
-            }
-            const int pb = own[tl];
-            const int q = pb + 1 + (p - pre[tl]);
-            const int ob = ki[pb];
-            int sl = slot + ob;
-            if (sl >= W) sl -= W;
-            const int o = ki[q] - ob;
-            F[divC(sl) * Wp + o] -= kv[q] * kv[pb];
-            pat[divC(sl) * Wp + o] = 1;
-        }
-        for (int q = (int)blockDim.x - 1 - (int)threadIdx.x; q < cn; q += blockDim.x) {
-            const int code = ci[q];
-            int sl = slot + (code < 0 ? -code : code);
-            if (sl >= W) sl -= W;
-            const int ls = divC(sl);
-            if (sl - ls * C != r || (!diag_keep && code < 0)) continue;
-            dl[ls] -= cL[q] * cL[q];
-        }
-        for (int t = (int)(threadIdx.x ^ (blockDim.x >> 1)); t < nown; t += blockDim.x) {
-            int sl = slot + ki[own[t]];
-            if (sl >= W) sl -= W;
-            const int ls = divC(sl);
-            if (lev[ls] < lj) lev[ls] = lj;
-        }
-        pslot = slot;
-        slot = slot + 1 == W ? 0 : slot + 1;
-        cluster.sync();
+        if (threadIdx.x == 0 && !s_result) s_result = nnz;
     }
-    // No CTA leaves while another may still read its shared memory.
-    cluster.sync();
-    if (r == 0 && threadIdx.x == 0) *result = s_fail ? (int64_t)s_fail : s_nnz;
+    __syncthreads();
+    if (threadIdx.x == 0) *result = s_result;
 }
 
 // Level histogram / order of rows, and the row (CSR) view of L used by the
@@ -1039,46 +1124,41 @@ void ichol_launch_init(int64_t n, const int64_t* Ap, const int64_t* Ar, const do
     if (n > 0) k_ichol_init<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, Ap, Ar, Av, shift, d, rsum, level, band);
 }
 
-int ichol_launch_factor(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
-                        const double* Av, double* d, const double* rsum, int* level, double* F,
-                        uint8_t* pat, int* cand, double* keptv, int64_t* kepti, int64_t* Lp,
-                        int64_t* Lr, double* Lv, int64_t cap, double discard, int64_t max_nnz,
-                        double rel, int diag_keep, int64_t* result, cudaStream_t s) {
-    // Front on chip when a cluster of at most 8 CTAs holds it and such a
-    // cluster can be resident; otherwise the front lives in global memory.
-    const int C = ichol_cluster_size(W);
-    if (C > 0) {
-        const ClLayout L = cl_layout(W, C);
-        const int chunks = (int)((W - 1 + 31) / 32);
-        auto kern = chunks <= 2 ? k_ichol_factor_cluster<2>
-                  : chunks <= 4 ? k_ichol_factor_cluster<4>
-                  : chunks <= 8 ? k_ichol_factor_cluster<8> : k_ichol_factor_cluster<kClMaxChunks>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)C);
-        cfg.blockDim = dim3(kClThreads);
-        cfg.dynamicSmemBytes = L.bytes;
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)C;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters >= 1) {
-            if (cudaLaunchKernelEx(&cfg, kern, n, (int)W, C, Ap, Ar, Av, (const double*)d, rsum,
-                                   level, Lp, Lr, Lv, cap, discard, max_nnz, rel, diag_keep,
-                                   result) == cudaSuccess)
-                return C;
-        }
+// The pipelined kernel, for the bandwidths that its shared memory takes.
+// False: not launched. `list` holds max(W, kPipeMinW)^2 doubles.
+bool ichol_launch_factor_pipe(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
+                              const double* Av, const double* d, const double* rsum, int* level,
+                              int64_t* Lp, int64_t* Lr, double* Lv, double* list, uint16_t* offs, int64_t cap,
+                              double discard, int64_t max_nnz, double rel, int diag_keep,
+                              int64_t* result, cudaStream_t s) {
+    W = W < kPipeMinW ? kPipeMinW : W;
+    if (W > 32 * kPipeMaxChunks + 1 || n > kPipeMax || cap > kPipeMax) return false;
+    const int chunks = (int)((W - 1 + 31) / 32);
+    const int fin = chunks <= 8 ? 4 : 8;
+    const PipeLayout L = pipe_layout(W, kPipeWarps - 1 - fin);
+    if (L.bytes > kFactorSmem - 512) return false;
+    auto kern = chunks <= 4 ? k_ichol_factor_pipe<4, 1>
+              : chunks <= 8 ? k_ichol_factor_pipe<4, 2>
+              : chunks <= 16 ? k_ichol_factor_pipe<8, 2> : k_ichol_factor_pipe<8, 4>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes) !=
+        cudaSuccess) {
         cudaGetLastError();
+        return false;
     }
+    kern<<<1, kPipeThreads, L.bytes, s>>>((int)n, (int)W, Ap, Ar, Av, d, rsum, level, Lp, Lr, Lv,
+                                          reinterpret_cast<int2*>(list), offs, cap, discard, max_nnz, rel,
+                                          diag_keep, result);
+    return true;
+}
+
+void ichol_launch_factor(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
+                         const double* Av, double* d, const double* rsum, int* level, double* F,
+                         uint8_t* pat, int* cand, double* keptv, int64_t* kepti, int64_t* Lp,
+                         int64_t* Lr, double* Lv, int64_t cap, double discard, int64_t max_nnz,
+                         double rel_discard, int diag_keep, int64_t* result, cudaStream_t s) {
     k_ichol_factor<<<1, kIcholThreads, 0, s>>>(n, W, Ap, Ar, Av, d, rsum, level, F, pat, cand, keptv,
-                                               kepti, Lp, Lr, Lv, cap, discard, max_nnz, rel,
+                                               kepti, Lp, Lr, Lv, cap, discard, max_nnz, rel_discard,
                                                diag_keep, result);
-    return 0;
 }
 
 void ichol_launch_levels(int64_t n, const int* level, int64_t* cnt, int* maxlevel, cudaStream_t s) {

@@ -57,8 +57,17 @@ void ichol_launch_solve_stream(int64_t n, int total, const StreamFirst& first,
 void ichol_launch_init(int64_t n, const int64_t* Ap, const int64_t* Ar, const double* Av,
                        double shift, double* d, double* rsum, int* level, unsigned long long* band,
                        cudaStream_t s);
-// Returns the cluster size of the kernel launched (0: the global-front kernel).
-int ichol_launch_factor(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
+// Result of the pipelined kernel when a wait ran out: the factor is made by
+// ichol_launch_factor.
+constexpr int64_t kIcholRetry = -100;
+constexpr int64_t kPipeMinW = 8;      // rows of its ring (narrower bands are padded)
+bool ichol_launch_factor_pipe(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
+                              const double* Av, const double* d, const double* rsum, int* level,
+                              int64_t* Lp, int64_t* Lr, double* Lv, double* list, uint16_t* offs, int64_t cap,
+                              double discard, int64_t max_nnz, double rel, int diag_keep,
+                              int64_t* result, cudaStream_t s);
+// The global-front kernel: bands that the pipelined kernel does not take.
+void ichol_launch_factor(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
                         const double* Av, double* d, const double* rsum, int* level, double* F,
                         uint8_t* pat, int* cand, double* keptv, int64_t* kepti, int64_t* Lp,
                         int64_t* Lr, double* Lv, int64_t cap, double discard, int64_t max_nnz,
@@ -71,7 +80,7 @@ void ichol_launch_rows(int64_t n, const int64_t* Lp, const int64_t* Lr, const do
 void ichol_launch_row_fill(int64_t n, const int64_t* Lp, const int64_t* Lr, const double* Lv,
                            int64_t* rfill, int64_t* Rc, double* Rv, const int64_t* Rp,
                            cudaStream_t s);
-// Cluster size of the on-chip factorisation for bandwidth W - 1; 0 = global front.
+// Size class of a band of W rows (see ichol.cu).
 int ichol_cluster_size(int64_t W);
 void ichol_prepare();
 void ichol_launch_solve(int64_t n, int nlevels, const int64_t* lptr, const int* order,

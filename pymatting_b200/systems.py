@@ -271,8 +271,8 @@ class IcholFactor:
         return float(_ffi.lib().pmb_ichol_factor_ms(self._h))
 
     def cluster(self):
-        """CTAs that held the band front on chip in the last factorisation
-        (0: the front was in global memory)."""
+        """Size class of the last factorisation: the CTAs whose shared memory
+        its band front would fill (0: more than 8)."""
         return int(_ffi.lib().pmb_ichol_cluster(self._h))
 
     def apply(self, b):
