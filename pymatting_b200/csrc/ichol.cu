@@ -256,17 +256,18 @@ int ichol_cluster_size(int64_t W) {
 //             entry in row j, in ascending k, as those columns are done.
 //   finishers kFin warps, every column in turn, one offset below the pivot per
 //             lane (and chunk): the last kLag columns' terms from dense copies
-//             in shared memory, one quotient, thresholds, diagonal update, the
-//             entry's place in L and in its row's list.
-//   pivot     one warp: the next pivot's root and reciprocal while the
-//             finishers write the column, and the wait for the walker of the
-//             column after that.
+//             in shared memory, one quotient, thresholds, diagonal update.
+//   pivot     one warp: the next pivot's root and its reciprocal, and the wait
+//             for the walker of the column after that.
+//   publishers kFin warps: the entries' places in L and in their rows' lists.
 //
-// What stays on the chain from one column to the next is the last term, the
-// root, the quotient and two barriers of the finishers and the pivot warp;
-// about 1,800 cycles, where the front spread over a cluster's shared memory
+// What stays on the chain from one column to the next is the quotient, the
+// root and two barriers of the finishers, the publishers and the pivot warp;
+// about 1,700 cycles, where the front spread over a cluster's shared memory
 // (every CTA reading, dividing and compacting the pivot column, then a cluster
-// barrier) took 4,300: 11,407 columns, 45 kept in each, 25.9 -> 10.9 ms.
+// barrier) took 4,300. 11,407 columns (W = 232), 45 entries kept in each: 25.9
+// -> 10.2 ms; without publishers of their own (the finishers writing L) 10.9.
+// The walkers' reads of L bound it now: with 11 of them 13.9 ms, 15: 12.1.
 //
 // L itself, in global memory, is what the walkers read (one CTA: its columns
 // come from L1 or L2), so nothing limits the number of entries. Row i's list,
@@ -280,8 +281,9 @@ int ichol_cluster_size(int64_t W) {
 // never -0.0: A's are non-zero and every update ends with + 0.0).
 // ---------------------------------------------------------------------------
 
-constexpr int kPipeWarps = 24;        // finishers, pivot and walkers
-constexpr int kPipeThreads = 32 * kPipeWarps;
+// Warps for `fin` finishers: as many publishers, the pivot, and walkers.
+__host__ __device__ constexpr int pipe_warps(int fin) { return fin <= 6 ? 28 : 32; }
+__host__ __device__ constexpr int pipe_walkers(int fin) { return pipe_warps(fin) - 1 - 2 * fin; }
 constexpr int kLag = 4;
 constexpr int kDense = 8;             // dense columns kept (a power of two above kLag)
 constexpr int kPipeMaxChunks = 32;    // 32-offset chunks of a column: W <= 1025
@@ -314,7 +316,7 @@ __device__ __forceinline__ void st_release(int* p, int v) {
 
 template <int FIN>
 __device__ __forceinline__ void pipe_barrier(int id) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(32 * (FIN + 1)) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(32 * (2 * FIN + 1)) : "memory");
 }
 
 // Exponents for which a quotient by `pipe_quotient` cannot leave the normal
@@ -324,10 +326,19 @@ __device__ __forceinline__ bool mid_range(double x) {
     return e > 523 && e < 1523;
 }
 
-// a / b, correctly rounded, from y = RN(1 / b): a y is within two ulp, one
-// correction by its exact remainder makes it faithful and a second one the
-// rounded quotient (Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", 1990). For a zero or in the range above.
+// Roots whose reciprocal `y` in the pivot warp serves `pipe_quotient`.
+__device__ __forceinline__ bool root_range(double s) {
+    return mid_range(s) && (__double2hiint(s) & 0xfffff) != 0xfffff;
+}
+
+// a / b, correctly rounded, from y within (1/2 + 2^-48) ulp of 1 / b: a y is
+// within two ulp, one correction by its remainder makes it faithful and a
+// second one, whose remainder is exact, the rounded quotient (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990). With the significand of b at beta 2^53, beta < 1, the corrected value
+// is within 2^-54 beta (1 + 2^-47) ulp of a / b before its rounding, and a / b
+// is at least 2^-54 / beta ulp from a midpoint of two doubles; the range of b
+// leaves out the beta next to 1. For a zero or in the range above.
 __device__ __forceinline__ double pipe_quotient(double a, double b, double y) {
     double q = a * y;
     q = __fma_rn(__fma_rn(-q, b, a), y, q);
@@ -341,14 +352,14 @@ __device__ __forceinline__ bool has_entry(double a) {
 // list: W x W nodes, row i's at slot i mod W; a node is the entry's place in
 // L and (entries of its column after it) << 16 | offset.
 template <int kFin, int M>
-__global__ void __launch_bounds__(kPipeThreads, 1)
+__global__ void __launch_bounds__(32 * pipe_warps(kFin), 1)
 k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t* __restrict__ Ar,
                     const double* __restrict__ Av, const double* __restrict__ d0,
                     const double* __restrict__ rsum, int* level, int64_t* Lp, int64_t* Lr, double* Lv,
                     int2* list, uint16_t* offs, int64_t cap, double discard, int64_t max_nnz, double rel_discard,
                     int diag_keep, int64_t* result) {
     extern __shared__ __align__(16) unsigned char pipe_smem[];
-    constexpr int kWalkers = kPipeWarps - 1 - kFin;
+    constexpr int kWalkers = pipe_walkers(kFin);
     __shared__ __align__(16) int s_count[2][kFin * M];  // candidates << 16 | kept, per chunk
     __shared__ double s_dj, s_sj, s_y;
     __shared__ int s_ready[kWalkers];          // column whose accumulator is ready
@@ -380,9 +391,9 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
     }
     __syncthreads();
 
-    if (warp > kFin) {
+    if (warp > 2 * kFin) {
         // ---- walker ----
-        const int me = warp - kFin - 1;
+        const int me = warp - 2 * kFin - 1;
         double* acc = accs + me * Wp;
         int slot = me % W;
         const int step = kWalkers % W;
@@ -511,9 +522,12 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
             ++ready;
             wk = wk + 1 == kWalkers ? 0 : wk + 1;
         };
+        // y is one Newton step from rsqrt, which does not wait for the root:
+        // rsqrt's 2^-51 squares to 2^-102.
         auto root = [&](double d) {
             const double s = sqrt(d);
-            const double y = 1.0 / s;
+            const double y0 = rsqrt(d);
+            const double y = __fma_rn(__fma_rn(-s, y0, 1.0), y0, y0);
             if (lane == 0) {
                 s_dj = d;
                 s_sj = s;
@@ -528,32 +542,119 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
         for (int j = 0; j < n && !*(volatile int*)&s_stop; ++j) {
             pipe_barrier<kFin>(1);
             if (j + 1 < n) root(dl[slot]);
+            if (lane == 0) st_release(&s_done, j - 1);     // it is in its rows' lists
             if (j + 2 < n) await(j + 2);
             pipe_barrier<kFin>(2);
-            // Column j - 1 is in its rows' lists.
-            if (lane == 0) st_release(&s_done, j - 1);
             slot = slot + 1 == W ? 0 : slot + 1;
         }
         if (lane == 0) st_release(&s_done, kPipeStop);
+    } else if (warp > kFin) {
+        // ---- publishers: lane's offsets 1 + lane + 32 (me + kFin m) ----
+        const int me = warp - kFin - 1;
+        const bool first = me == 0 && lane == 0;
+        int slot = 0;
+        int64_t nnz = 0;
+        double dnext = W < n ? d0[W] : 0.0;
+        int psl[M], pcnt[M];                 // list lengths to publish for the column before
+#pragma unroll
+        for (int m = 0; m < M; ++m) pcnt[m] = 0;
+        pipe_barrier<kFin>(2);
+        for (int j = 0; j < n && !*(volatile int*)&s_stop; ++j) {
+            // While the finishers make column j: lengths of the lists that
+            // column j - 1 extended (written before the last barrier), and
+            // what this column's rows hold.
+            __threadfence_block();
+            const double dj = s_dj, sj = s_sj;
+            const int levj = lev[slot];
+            int sl[M], lv[M], pos[M];
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int o = 1 + lane + 32 * (me + kFin * m);
+                if (pcnt[m]) *(volatile int*)&rowcnt[psl[m]] = pcnt[m];
+                sl[m] = o >= W ? slot : slot + o >= W ? slot + o - W : slot + o;
+                lv[m] = lev[sl[m]];
+                pos[m] = rowpos[sl[m]];
+            }
+            pipe_barrier<kFin>(1);
+            // Places in L: chunks in ascending offsets.
+            const double* dc = dense + (j & (kDense - 1)) * Wp;
+            double L[M];
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int o = 1 + lane + 32 * (me + kFin * m);
+                L[m] = o < W ? dc[o] : -0.0;
+            }
+            int before[M], total = 0;
+#pragma unroll
+            for (int c = 0; c < kFin * M; ++c) {
+                if (c % kFin == me) before[c / kFin] = total & 0xffff;
+                total += s_count[j & 1][c];
+            }
+            const int cn = total >> 16, kept = total & 0xffff;
+            int64_t fail = 0;
+            if (!(dj > 0.0)) fail = -1;                                              // ichol.py:80-81
+            else if (nnz + 1 + cn > max_nnz || nnz + 1 + cn > cap) fail = -2;        // ichol.py:82-83
+            if (fail) {
+                if (first) {
+                    s_result = fail;
+                    s_stop = 1;
+                }
+            } else {
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    pcnt[m] = 0;
+                    const bool keep = has_entry(L[m]);
+                    const unsigned km = __ballot_sync(all, keep);
+                    if (keep) {
+                        const int o = 1 + lane + 32 * (me + kFin * m);
+                        const int r = before[m] + __popc(km & lt);
+                        const int64_t g = nnz + 1 + r;
+                        Lv[g] = L[m];
+                        Lr[g] = j + o;
+                        offs[g] = (uint16_t)o;
+                        if (lv[m] <= levj) lev[sl[m]] = levj + 1;
+                        if (o > kLag) {
+                            const int p = pos[m];
+                            rowpos[sl[m]] = p + 1;
+                            list[sl[m] * W + p] = make_int2((int)g, (kept - 1 - r) << 16 | o);
+                            psl[m] = sl[m];
+                            pcnt[m] = p + 1;
+                        }
+                    }
+                }
+                if (first) {
+                    Lv[nnz] = sj;
+                    Lr[nnz] = j;
+                    Lp[j + 1] = nnz + 1 + kept;
+                    level[j] = levj;
+                    // The slot's next row.
+                    dl[slot] = dnext;
+                    lev[slot] = 0;
+                    rowpos[slot] = 0;
+                    *(volatile int*)&rowcnt[slot] = 0;
+                    if (j + 1 + W < n) dnext = d0[j + 1 + W];
+                }
+                nnz += 1 + kept;
+                slot = slot + 1 == W ? 0 : slot + 1;
+            }
+            pipe_barrier<kFin>(2);
+        }
+        if (first && !s_result) s_result = nnz;
     } else {
         // ---- finishers: lane's offsets 1 + lane + 32 (warp + kFin m) ----
         int slot = 0, wk = 0;
-        int64_t nnz = 0;
-        double dnext = W < n ? d0[W] : 0.0, rnow = rsum[0], rnext = n > 1 ? rsum[1] : 0.0;
-        int psl[M], pcnt[M];                 // list lengths to publish for the column before
+        double rnow = rsum[0], rnext = n > 1 ? rsum[1] : 0.0;
         double a[M];
-#pragma unroll
-        for (int m = 0; m < M; ++m) pcnt[m] = 0;
         // The accumulator of column c and the terms of the dense columns.
         auto gather = [&](int c) {
             const double* acc = accs + wk * Wp;
             wk = wk + 1 == kWalkers ? 0 : wk + 1;
+            double f[kLag], x[kLag][M];
 #pragma unroll
             for (int m = 0; m < M; ++m) {
                 const int o = 1 + lane + 32 * (warp + kFin * m);
                 a[m] = o < W ? acc[o] : -0.0;
             }
-            double f[kLag], x[kLag][M];
 #pragma unroll
             for (int b = kLag; b >= 1; --b) {
                 const double* dc = dense + ((c - b) & (kDense - 1)) * Wp;
@@ -574,116 +675,44 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
             }
         };
         pipe_barrier<kFin>(2);
-        if (!*(volatile int*)&s_stop) {
-            gather(0);
-            for (int j = 0; j < n; ++j) {
-                // Quotients, thresholds, diagonal updates, dense copy.
-                const double dj = s_dj, sj = s_sj, y = s_y;
-                const int levj = lev[slot];
-                int sl[M], lv[M], pos[M];
-                double du[M];
+        if (!*(volatile int*)&s_stop) gather(0);
+        for (int j = 0; j < n && !*(volatile int*)&s_stop; ++j) {
+            // Quotients, thresholds, diagonal updates, dense copy.
+            const double sj = s_sj, y = s_y;
+            const double rel = rel_discard * rnow;
+            rnow = rnext;
+            if (j + 2 < n) rnext = rsum[j + 2];
+            double L[M], du[M];
+            int sl[M];
+            bool odd = !root_range(sj);
 #pragma unroll
-                for (int m = 0; m < M; ++m) {
-                    const int o = 1 + lane + 32 * (warp + kFin * m);
-                    sl[m] = o >= W ? slot : slot + o >= W ? slot + o - W : slot + o;
-                    du[m] = dl[sl[m]];
-                    lv[m] = lev[sl[m]];
-                    pos[m] = rowpos[sl[m]];
-                }
-                const double rel = rel_discard * rnow;
-                double L[M];
-                bool keep[M];
-                bool odd = !mid_range(sj);
-#pragma unroll
-                for (int m = 0; m < M; ++m) {
-                    odd |= has_entry(a[m]) && !(a[m] == 0.0 || mid_range(a[m]));
-                    L[m] = pipe_quotient(a[m], sj, y);
-                }
-                if (__any_sync(all, odd)) {
-#pragma unroll
-                    for (int m = 0; m < M; ++m) L[m] = a[m] / sj;
-                }
-                unsigned km[M];
-#pragma unroll
-                for (int m = 0; m < M; ++m) {
-                    const int o = 1 + lane + 32 * (warp + kFin * m);
-                    const bool in = has_entry(a[m]);
-                    keep[m] = in && fabs(L[m]) > discard && fabs(a[m]) > rel;
-                    if (in && (diag_keep || keep[m])) dl[sl[m]] = du[m] - L[m] * L[m];
-                    if (o < W) dense[(j & (kDense - 1)) * Wp + o] = keep[m] ? L[m] : -0.0;
-                    const unsigned fm = __ballot_sync(all, in);
-                    km[m] = __ballot_sync(all, keep[m]);
-                    if (lane == 0) s_count[j & 1][warp + kFin * m] = __popc(fm) << 16 | __popc(km[m]);
-                }
-                pipe_barrier<kFin>(1);
-                // Lengths of the lists that column j - 1 extended: its entries
-                // were written before the barrier.
-                __threadfence_block();
-#pragma unroll
-                for (int m = 0; m < M; ++m)
-                    if (pcnt[m]) *(volatile int*)&rowcnt[psl[m]] = pcnt[m];
-                // Places in L: chunks in ascending offsets.
-                int before[M], total = 0;
-#pragma unroll
-                for (int c = 0; c < kFin * M; ++c) {
-                    if (c % kFin == warp) before[c / kFin] = total & 0xffff;
-                    total += s_count[j & 1][c];
-                }
-                const int cn = total >> 16, kept = total & 0xffff;
-                int64_t fail = 0;
-                if (!(dj > 0.0)) fail = -1;                                              // ichol.py:80-81
-                else if (nnz + 1 + cn > max_nnz || nnz + 1 + cn > cap) fail = -2;        // ichol.py:82-83
-                if (fail) {
-                    if (threadIdx.x == 0) {
-                        s_result = fail;
-                        s_stop = 1;
-                    }
-                } else {
-#pragma unroll
-                    for (int m = 0; m < M; ++m) {
-                        pcnt[m] = 0;
-                        if (keep[m]) {
-                            const int o = 1 + lane + 32 * (warp + kFin * m);
-                            const int r = before[m] + __popc(km[m] & lt);
-                            const int64_t g = nnz + 1 + r;
-                            Lv[g] = L[m];
-                            Lr[g] = j + o;
-                            offs[g] = (uint16_t)o;
-                            if (lv[m] <= levj) lev[sl[m]] = levj + 1;
-                            if (o > kLag) {
-                                const int p = pos[m];
-                                rowpos[sl[m]] = p + 1;
-                                list[sl[m] * W + p] = make_int2((int)g, (kept - 1 - r) << 16 | o);
-                                psl[m] = sl[m];
-                                pcnt[m] = p + 1;
-                            }
-                        }
-                    }
-                    if (threadIdx.x == 0) {
-                        Lv[nnz] = sj;
-                        Lr[nnz] = j;
-                        Lp[j + 1] = nnz + 1 + kept;
-                        level[j] = levj;
-                        // The slot's next row.
-                        dl[slot] = dnext;
-                        lev[slot] = 0;
-                        rowpos[slot] = 0;
-                        *(volatile int*)&rowcnt[slot] = 0;
-                    }
-                    nnz += 1 + kept;
-                    slot = slot + 1 == W ? 0 : slot + 1;
-                    if (j + 1 < n) {
-                        rnow = rnext;
-                        if (j + 2 < n) rnext = rsum[j + 2];
-                        if (j + 1 + W < n) dnext = d0[j + 1 + W];
-                        gather(j + 1);
-                    }
-                }
-                pipe_barrier<kFin>(2);
-                if (*(volatile int*)&s_stop) break;
+            for (int m = 0; m < M; ++m) {
+                const int o = 1 + lane + 32 * (warp + kFin * m);
+                sl[m] = o >= W ? slot : slot + o >= W ? slot + o - W : slot + o;
+                du[m] = dl[sl[m]];
+                odd |= has_entry(a[m]) && !(a[m] == 0.0 || mid_range(a[m]));
+                L[m] = pipe_quotient(a[m], sj, y);
             }
+            if (__any_sync(all, odd)) {
+#pragma unroll
+                for (int m = 0; m < M; ++m) L[m] = a[m] / sj;
+            }
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                const int o = 1 + lane + 32 * (warp + kFin * m);
+                const bool in = has_entry(a[m]);
+                const bool keep = in && fabs(L[m]) > discard && fabs(a[m]) > rel;
+                if (in && (diag_keep || keep)) dl[sl[m]] = du[m] - L[m] * L[m];
+                if (o < W) dense[(j & (kDense - 1)) * Wp + o] = keep ? L[m] : -0.0;
+                const unsigned fm = __ballot_sync(all, in);
+                const unsigned km = __ballot_sync(all, keep);
+                if (lane == 0) s_count[j & 1][warp + kFin * m] = __popc(fm) << 16 | __popc(km);
+            }
+            pipe_barrier<kFin>(1);
+            slot = slot + 1 == W ? 0 : slot + 1;
+            if (j + 1 < n) gather(j + 1);
+            pipe_barrier<kFin>(2);
         }
-        if (threadIdx.x == 0 && !s_result) s_result = nnz;
     }
     __syncthreads();
     if (threadIdx.x == 0) *result = s_result;
@@ -1134,18 +1163,19 @@ bool ichol_launch_factor_pipe(int64_t n, int64_t W, const int64_t* Ap, const int
     W = W < kPipeMinW ? kPipeMinW : W;
     if (W > 32 * kPipeMaxChunks + 1 || n > kPipeMax || cap > kPipeMax) return false;
     const int chunks = (int)((W - 1 + 31) / 32);
-    const int fin = chunks <= 8 ? 4 : 8;
-    const PipeLayout L = pipe_layout(W, kPipeWarps - 1 - fin);
+    const int fin = chunks <= 8 ? 4 : chunks <= 12 ? 6 : 8;
+    const PipeLayout L = pipe_layout(W, pipe_walkers(fin));
     if (L.bytes > kFactorSmem - 512) return false;
     auto kern = chunks <= 4 ? k_ichol_factor_pipe<4, 1>
               : chunks <= 8 ? k_ichol_factor_pipe<4, 2>
+              : chunks <= 12 ? k_ichol_factor_pipe<6, 2>
               : chunks <= 16 ? k_ichol_factor_pipe<8, 2> : k_ichol_factor_pipe<8, 4>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes) !=
         cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    kern<<<1, kPipeThreads, L.bytes, s>>>((int)n, (int)W, Ap, Ar, Av, d, rsum, level, Lp, Lr, Lv,
+    kern<<<1, 32 * pipe_warps(fin), L.bytes, s>>>((int)n, (int)W, Ap, Ar, Av, d, rsum, level, Lp, Lr, Lv,
                                           reinterpret_cast<int2*>(list), offs, cap, discard, max_nnz, rel,
                                           diag_keep, result);
     return true;
