@@ -72,9 +72,7 @@ enum : int {
     kMapXAD,       // buffer A, restriction box
     kMapXBF,       // smoothing ping-pong buffer B, fine box
     kMapXBD,       // buffer B, restriction box
-    kMapZF,        // CG z, fine box (level 0)
-    kMapP0F,       // CG p parity 0 (also x0 scratch), fine box
-    kMapP1F,       // CG p parity 1, fine box
+    kMapP0F,       // x0 scratch (CG p parity 0), fine box
     kMapX64F,      // FP64 refinement iterate, fine box
     kMapP64F,      // FP64 planes, fine box (refinement residual)
     kMapPlG,       // FP64 planes, Galerkin box (42 x 21 x 13)

@@ -2,14 +2,16 @@
 // the fused preconditioned conjugate-gradient steps, and the geometric
 // multigrid V-cycle used as its preconditioner.
 //
-// Every stencil kernel works on 64 x 8 pixel tiles. One thread of the CTA
-// issues TMA loads of the tile plus its halo: a single 3D box holds all 13
+// The operator apply, the restriction and the prolongation of the default
+// cycle are the row kernels of stencil_rows.cu. The stencil kernels here (other
+// numbers of sweeps, the residual replacement, setup) work on 64 x 8 pixel
+// tiles. One thread of the CTA issues TMA loads of the tile plus its halo: a single 3D box holds all 13
 // operator planes (72 x 12 x 13), 2D boxes hold the vector operands; the
 // hardware zero-fills everything outside the image, which supplies the
 // stencil's border terms. The kernels then read operators and operands from
 // shared memory only. Element-wise kernels stream chunks of elements.
 //
-// Every kernel walks a WorkList of tiles over a batch of grids (images of
+// Every tile kernel walks a WorkList of tiles over a batch of grids (images of
 // different sizes, or the same multigrid level of several images) with a
 // grid-stride loop, so one launch serves the whole batch. Per-image scalars
 // (alpha, beta, norms, convergence status) live in InstState on the device;
