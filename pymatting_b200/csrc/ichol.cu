@@ -971,17 +971,21 @@ k_ichol_solve_smem(int64_t n, int nlevels, const int64_t* __restrict__ lptr,
 //   double[ents]      L values of the row terms
 //   int[ents]         their x indices       (ents padded to a multiple of 4)
 //
-// One thread keeps kStreamStages chunks in flight with bulk copies into a
-// shared-memory ring (completion on one mbarrier per stage); every chunk
-// ends with the block barrier that separates levels and frees the stage.
-// The data of a chunk never depends on x, so the copies run ahead of the
-// dependency chain and no global-load latency sits on it. Within a row the
-// terms are summed lane-strided and reduced across the warp, as in
-// k_ichol_solve_smem, and x_i = (x_i - sum) / L_ii as the reference's
-// back substitutions (ichol.py:116-145).
+// A warp of its own keeps kStreamStages chunks in flight with bulk copies into
+// a shared-memory ring (completion on one mbarrier per stage) and waits for
+// each chunk two steps before it is used, so the other warps see its data
+// through the block barrier that ends a step. They take the record and the
+// entries of their row of the next chunk into registers while this one's sums
+// are made (neither depends on x); what is left on the chain from level to
+// level is the gather of x, the warp's reduction, the quotient (a corrected
+// product with the reciprocal that the packing made, rounded as the division)
+// and the barrier. Within a row the terms are summed lane-strided and reduced
+// across the warp, as in k_ichol_solve_smem, and x_i = (x_i - sum) / L_ii as
+// the reference's back substitutions (ichol.py:116-145).
 // ---------------------------------------------------------------------------
 
-constexpr int kStreamThreads = 256;
+constexpr int kStreamWarps = 8;       // that take rows; one more for the copies
+constexpr int kStreamThreads = 32 * (kStreamWarps + 1);
 constexpr size_t kStreamStageBytes =
     sizeof(StreamHead) + kStreamRowsMax * sizeof(StreamRow) + kStreamEntsMax * 12;
 static_assert(kStreamStageBytes % 16 == 0, "stages are 16-byte aligned");
@@ -990,17 +994,28 @@ size_t ichol_stream_smem(int64_t n) {
     return kStreamStages * kStreamStageBytes + (size_t)n * sizeof(double);
 }
 
+// x_i from its numerator: the division where the record does not vouch for the
+// reciprocal, or the numerator is outside the quotient's range.
+__device__ __forceinline__ double stream_quotient(double num, const StreamRow& rw) {
+    if (rw.fast && (num == 0.0 || mid_range(num))) return pipe_quotient(num, rw.diag, rw.inv);
+    return num / rw.diag;
+}
+
 __global__ void __launch_bounds__(kStreamThreads)
 k_ichol_solve_stream(int64_t n, int total, StreamFirst first, const unsigned char* __restrict__ blob,
                      const double* __restrict__ b, double* x, const InstState* st, uint32_t limit) {
     extern __shared__ __align__(16) unsigned char ss_smem[];
     __shared__ uint64_t full[kStreamStages];
-    __shared__ int s_bad;
+    __shared__ int s_bad[2];      // by step parity: written in a step, read in the next
     if (st && st->status != kRunning) return;
     double* sx = reinterpret_cast<double*>(ss_smem + kStreamStages * kStreamStageBytes);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (threadIdx.x == 0) {
-        s_bad = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool copier = warp == kStreamWarps && lane == 0;
+    auto landed = [&](int c) {
+        return c >= total ||
+               mbar_wait(&full[c % kStreamStages], (uint32_t)(c / kStreamStages) & 1u, limit);
+    };
+    if (copier) {
         for (int q = 0; q < kStreamStages; ++q) mbar_init(&full[q], 1);
         for (int q = 0; q < kStreamStages && q < total; ++q) {
             if (first.bytes[q] <= 0) continue;
@@ -1008,63 +1023,104 @@ k_ichol_solve_stream(int64_t n, int total, StreamFirst first, const unsigned cha
             bulk_load(ss_smem + q * kStreamStageBytes, blob + first.off[q], (uint32_t)first.bytes[q],
                       &full[q]);
         }
+        s_bad[1] = !(landed(0) && landed(1));
     }
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) sx[i] = b[i];
     __syncthreads();
+    // Row of this warp in the coming chunk.
+    StreamRow rw;
+    double v0 = 0.0, v1 = 0.0;
+    int c0 = 0, c1 = 0;
+    bool mine = false;
+    auto chunk = [&](int c, const StreamRow*& rec, const double*& val, const int*& col) {
+        const unsigned char* stage = ss_smem + (c % kStreamStages) * kStreamStageBytes;
+        const StreamHead* h = reinterpret_cast<const StreamHead*>(stage);
+        rec = reinterpret_cast<const StreamRow*>(stage + sizeof(StreamHead));
+        val = reinterpret_cast<const double*>(stage + sizeof(StreamHead) + h->rows * sizeof(StreamRow));
+        col = reinterpret_cast<const int*>(val + h->ents);
+        return h->rows;
+    };
+    auto fetch = [&](int c) {
+        const StreamRow* rec;
+        const double* val;
+        const int* col;
+        mine = c < total && warp < chunk(c, rec, val, col);
+        if (!mine) return;
+        rw = rec[warp];
+        v0 = v1 = 0.0;
+        c0 = c1 = rw.row;
+        if (lane < rw.count) {
+            v0 = val[rw.start + lane];
+            c0 = col[rw.start + lane];
+        }
+        if (lane + 32 < rw.count) {
+            v1 = val[rw.start + lane + 32];
+            c1 = col[rw.start + lane + 32];
+        }
+    };
     int c = 0;
-    for (; c < total; ++c) {
-        const int q = c % kStreamStages;
-        unsigned char* stage = ss_smem + q * kStreamStageBytes;
-        if (!mbar_wait(&full[q], (uint32_t)(c / kStreamStages) & 1u, limit)) {
-            s_bad = 1;
-        } else {
-            const StreamHead* h = reinterpret_cast<const StreamHead*>(stage);
-            const StreamRow* rec = reinterpret_cast<const StreamRow*>(stage + sizeof(StreamHead));
-            const int rows = h->rows, ents = h->ents;
-            const double* val = reinterpret_cast<const double*>(stage + sizeof(StreamHead) +
-                                                                rows * sizeof(StreamRow));
-            const int* col = reinterpret_cast<const int*>(val + ents);
-            for (int k = warp; k < rows; k += nw) {
-                const StreamRow rw = rec[k];
-                const double* rv = val + rw.start;
-                const int* rc = col + rw.start;
-                double acc = 0.0;
-                int e = lane;
-                for (; e + 32 < rw.count; e += 64) {     // two terms' loads in flight
-                    const double v0 = rv[e], v1 = rv[e + 32];
-                    const int c0 = rc[e], c1 = rc[e + 32];
-                    const double x0 = sx[c0], x1 = sx[c1];
-                    acc += v0 * x0;
-                    acc += v1 * x1;
-                }
-                if (e < rw.count) acc += rv[e] * sx[rc[e]];
+    int64_t next_off = 0;
+    int next_bytes = 0, issued = min(total, kStreamStages);
+    bool bad = s_bad[1] != 0;
+    if (warp < kStreamWarps && !bad) fetch(0);
+    for (; c < total && !bad; ++c) {
+        if (warp < kStreamWarps) {
+            const bool have = mine;
+            const StreamRow r = rw;
+            double acc = 0.0, x0 = 0.0, x1 = 0.0, xr = 0.0, w0 = v0, w1 = v1;
+            const bool two = have && lane + 32 < r.count;
+            if (have) {
+                x0 = sx[c0];
+                x1 = sx[c1];
+                xr = sx[r.row];
+            }
+            fetch(c + 1);
+            const StreamRow* rec;
+            const double* val;
+            const int* col;
+            const int rows = chunk(c, rec, val, col);
+            if (have) {
+                if (lane < r.count) acc += w0 * x0;
+                if (two) acc += w1 * x1;
+                for (int e = lane + 64; e < r.count; e += 32) acc += val[r.start + e] * sx[col[r.start + e]];
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                if (lane == 0) sx[rw.row] = (sx[rw.row] - acc) / rw.diag;
+                if (lane == 0) sx[r.row] = stream_quotient(xr - acc, r);
             }
+            for (int k = warp + kStreamWarps; k < rows; k += kStreamWarps) {
+                const StreamRow rk = rec[k];
+                acc = 0.0;
+                for (int e = lane; e < rk.count; e += 32) acc += val[rk.start + e] * sx[col[rk.start + e]];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                if (lane == 0) sx[rk.row] = stream_quotient(sx[rk.row] - acc, rk);
+            }
+        } else if (copier) {
+            // The stage that the last step left, then the chunk of the step
+            // after the next.
+            if (next_bytes > 0) {
+                uint64_t* bar = &full[(c - 1) % kStreamStages];
+                fence_proxy_async();
+                mbar_expect_tx(bar, (uint32_t)next_bytes);
+                bulk_load(ss_smem + ((c - 1) % kStreamStages) * kStreamStageBytes, blob + next_off,
+                          (uint32_t)next_bytes, bar);
+                ++issued;
+            }
+            const StreamHead* h =
+                reinterpret_cast<const StreamHead*>(ss_smem + (c % kStreamStages) * kStreamStageBytes);
+            next_off = h->next_off;
+            next_bytes = h->next_bytes;
+            s_bad[c & 1] = !landed(c + 2);
         }
         __syncthreads();          // level barrier; the stage is free again
-        if (s_bad) break;
-        // The last warp refills the stage: rows go to warps in order, so it
-        // only has rows of its own in chunks of more than nw - 1 rows.
-        if (threadIdx.x == blockDim.x - 32) {
-            const StreamHead* h = reinterpret_cast<const StreamHead*>(stage);
-            const int64_t off = h->next_off;
-            const int bytes = h->next_bytes;
-            if (bytes > 0) {
-                fence_proxy_async();
-                mbar_expect_tx(&full[q], (uint32_t)bytes);
-                bulk_load(stage, blob + off, (uint32_t)bytes, &full[q]);
-            }
-        }
+        bad = s_bad[c & 1] != 0;
     }
-    if (s_bad) {
+    if (bad) {
         // A copy did not complete: the result is NaN, and copies still in
         // flight are waited for (bounded) before the CTA leaves.
         for (int64_t i = threadIdx.x; i < n; i += blockDim.x) x[i] = __longlong_as_double(0x7ff8000000000000ll);
-        if (threadIdx.x == blockDim.x - 32) {
-            for (int k = c; k < c + kStreamStages && k < total; ++k)
-                mbar_wait(&full[k % kStreamStages], (uint32_t)(k / kStreamStages) & 1u, limit);
+        if (copier) {
+            for (int k = c; k < issued; ++k) landed(k);
         }
         __syncthreads();
         return;
@@ -1098,9 +1154,9 @@ __global__ void k_stream_pack_rows(int nrec, const StreamPackRow* __restrict__ r
         rw.row = R.row;
         rw.start = R.start;
         rw.count = R.count;
-        rw.pad = 0;
         rw.diag = Lv[Lp[R.row]];
-        rw.pad2 = 0.0;
+        rw.inv = 1.0 / rw.diag;
+        rw.fast = root_range(rw.diag);
         *rec = rw;
     }
 }

@@ -21,8 +21,9 @@ struct StreamHead {
     int pad[3];
 };
 struct StreamRow {
-    int row, start, count, pad;
-    double diag, pad2;
+    int row, start, count;
+    int fast;              // inv serves the quotient (root_range)
+    double diag, inv;      // L_ii and its reciprocal
 };
 static_assert(sizeof(StreamHead) == 32 && sizeof(StreamRow) == 32, "chunk records are 32 bytes");
 
