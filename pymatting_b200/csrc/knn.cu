@@ -423,12 +423,23 @@ __global__ void k_scatter(Passes P, long long n, int kt, const int64_t* off, int
         }
 }
 
+// Order-preserving map of doubles to unsigned. A total order: NaN, which the
+// soft kernel gives where a feature is not finite, has its place in it too.
+__device__ __forceinline__ unsigned long long ordered64(double v) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    return u >> 63 ? ~u : u | 1ull << 63;
+}
+__device__ __forceinline__ double unordered64(unsigned long long u) {
+    return __longlong_as_double((long long)(u >> 63 ? u & ~(1ull << 63) : ~u));
+}
+
 // Sort each row by (column, value), merge duplicates (sum in that order),
 // count the unique columns. A warp per row: entries find their ranks by
 // counting the smaller ones in shared memory (rows hold about 2 kt entries;
 // one thread per row shifting entries in global memory took 1.6 ms for 65536
-// rows). A row of more than kSortMax entries, one that many others list, takes
-// its whole CTA, of more than kSortWarps times that one thread.
+// rows); the ranks are a permutation because (column, ordered64, position) is
+// a total order. A row of more than kSortMax entries, one that many others
+// list, takes its whole CTA, of more than kSortWarps times that one thread.
 constexpr int kSortMax = 256, kSortWarps = 4;
 __host__ __device__ constexpr size_t sort_warp_smem() { return (size_t)kSortMax * 24; }
 
@@ -463,19 +474,19 @@ __device__ void sort_merge_one(long long a, long long m, int64_t* cols, double* 
 template <typename Sync>
 __device__ __forceinline__ void sort_merge_row(long long a, int m, int tid, int nthr, unsigned char* sm, int room,
                                                int64_t* cols, double* vals, int64_t* ucount, Sync sync) {
-    double* v0 = reinterpret_cast<double*>(sm);
-    double* v1 = v0 + room;
+    unsigned long long* v0 = reinterpret_cast<unsigned long long*>(sm);   // ordered64
+    double* v1 = reinterpret_cast<double*>(v0 + room);
     int* c0 = reinterpret_cast<int*>(v1 + room);
     int* c1 = c0 + room;
     const int m4 = (m + 3) & ~3;                       // <= room
     for (int e = tid; e < m4; e += nthr) {
         c0[e] = e < m ? (int)cols[a + e] : 0x7fffffff;
-        if (e < m) v0[e] = vals[a + e];
+        if (e < m) v0[e] = ordered64(vals[a + e]);
     }
     sync();
     for (int e = tid; e < m; e += nthr) {
         const int c = c0[e];
-        const double v = v0[e];
+        const unsigned long long v = v0[e];
         int rank = 0;
         for (int t = 0; t < m4; t += 4) {
             const int4 k = *reinterpret_cast<const int4*>(c0 + t);
@@ -485,7 +496,7 @@ __device__ __forceinline__ void sort_merge_row(long long a, int m, int tid, int 
                     rank += c0[q] == c && (v0[q] < v || (v0[q] == v && q < e));
         }
         c1[rank] = c;
-        v1[rank] = v;
+        v1[rank] = unordered64(v);
     }
     sync();
     // The first warp merges.

@@ -1,0 +1,36 @@
+"""knn_laplacian on images with pixels that are not finite. Their rows mean
+little, but the matrix must stay one: nothing here multiplies with it."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _bad_image(h, w, seed, bad, flat=False):
+    rng = np.random.default_rng(seed)
+    img = np.full((h, w, 3), 0.5) if flat else rng.random((h, w, 3))
+    for k, v in enumerate(bad):
+        img.reshape(-1, 3)[(h * w // 2 + 7 * k) % (h * w), k % 3] = v
+    return img
+
+
+# Equal points with distance weight 0 all list the same ones, whose rows then
+# hold up to 256 entries (sorted by a warp), up to 1024 (a CTA), more (a thread).
+@pytest.mark.parametrize("h,w,ks,flat", [(6, 9, [20, 10], False), (24, 25, [20, 10], False),
+                                         (10, 10, [6, 4], True), (15, 20, [6, 4], True), (25, 28, [6, 4], True)])
+@pytest.mark.parametrize("bad", [[np.nan], [np.inf], [np.nan, np.inf, -np.inf]])
+@pytest.mark.parametrize("kernel", ["binary", "soft"])
+def test_pattern(gpu, h, w, ks, flat, bad, kernel):
+    import pymatting_b200 as pm
+    n = h * w
+    img = _bad_image(h, w, n, bad, flat)
+    L = pm.knn_laplacian(img, n_neighbors=ks, distance_weights=[0.0, 0.0] if flat else [2.0, 0.1], kernel=kernel)
+    indptr, indices, data = L.indptr, L.indices, L.data
+    assert indptr[0] == 0 and indptr[-1] == len(indices) == len(data)
+    assert (np.diff(indptr) >= ks[0]).all()
+    assert indices.min() >= 0 and indices.max() < n
+    row = np.repeat(np.arange(n), np.diff(indptr))
+    assert (np.diff(row * n + indices) > 0).all()      # ascending and distinct in every row
+    if kernel == "binary":
+        assert np.isfinite(data).all()
