@@ -5,7 +5,8 @@
 // numpy.linspace(0, 1, .) grids, one pass per (k, dw). Neighbours come from
 // an exact search with the reference k-d tree's distance
 // (pymatting/util/kdtree.py:_find_knn: float32 squared differences summed in
-// float64), keeping the k smallest by (distance, index). The points are
+// float64), keeping the k smallest by (distance, index); a distance that is not
+// a number (a feature that is not finite) counts as infinite. The points are
 // brought into the order of a 5-D Morton curve first, so that 32 consecutive
 // ones (a tile) lie close together; tiles whose bounding box is farther than
 // every query's k-th distance are skipped. The reference keeps the first found
@@ -313,7 +314,9 @@ __global__ void __launch_bounds__(kKnnWarps * 32) k_knn(const float* __restrict_
                 dist = __dadd_rn(dist, (double)p2);
                 dist = __dadd_rn(dist, (double)p3);
                 dist = __dadd_rn(dist, (double)p4);
-                QD[qn * 32] = dist;
+                // The lists' order has no place for NaN: as infinite, it leaves
+                // finite queries' lists alone.
+                QD[qn * 32] = dist == dist ? dist : __longlong_as_double(0x7ff0000000000000ll);
                 QI[qn * 32] = __float_as_int(e.y);
                 ++qn;
             }

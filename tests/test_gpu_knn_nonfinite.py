@@ -4,6 +4,8 @@ little, but the matrix must stay one: nothing here multiplies with it."""
 import numpy as np
 import pytest
 
+import oracle
+
 pytestmark = pytest.mark.gpu
 
 
@@ -34,3 +36,52 @@ def test_pattern(gpu, h, w, ks, flat, bad, kernel):
     assert (np.diff(row * n + indices) > 0).all()      # ascending and distinct in every row
     if kernel == "binary":
         assert np.isfinite(data).all()
+
+
+def _knn_nan_last(f, k):
+    """The k smallest by (distance, index), a NaN distance as infinite."""
+    d = np.zeros((len(f), len(f)))
+    for c in range(f.shape[1]):
+        e = f[:, None, c] - f[None, :, c]
+        d += (e * e).astype(np.float64)
+    d[np.isnan(d)] = np.inf
+    idx = np.broadcast_to(np.arange(len(f)), d.shape)
+    return np.lexsort((idx, d), axis=1)[:, :k]
+
+
+@pytest.mark.parametrize("at", [100, 117, 333, 590])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("kernel", ["binary", "soft"])
+def test_one_bad_pixel_leaves_the_others_alone(gpu, monkeypatch, at, bad, kernel):
+    """Only the pixel's own list is arbitrary: the k first pixels. Values are
+    compared in the rows whose weights are finite, columns in all rows."""
+    import pymatting_b200 as pm
+    lists = []
+
+    def knn(f, k):
+        lists.append(_knn_nan_last(f, k))
+        return lists[-1]
+
+    monkeypatch.setattr(oracle, "knn", knn)
+    h, w = 20, 30
+    n = h * w
+    img = np.random.default_rng(1).random((h, w, 3))
+    img.reshape(-1, 3)[at, 1] = bad
+    kw = dict(n_neighbors=[7], distance_weights=[1.0], kernel=kernel)
+    with np.errstate(all="ignore"):
+        Lr = oracle.knn_laplacian(img, **kw).toarray()
+        L = pm.knn_laplacian(img, **kw)
+        dense = L.toarray()
+    pattern = np.zeros((n, n), bool)
+    pattern[np.repeat(np.arange(n), 7), lists[0].ravel()] = True
+    pattern |= pattern.T
+    stored = np.zeros((n, n), bool)
+    stored[np.repeat(np.arange(n), np.diff(L.indptr)), L.indices] = True
+    # The pixel does not list itself, so its own diagonal is left out here.
+    pattern[at, at] = stored[at, at] = False
+    dense[at, at] = Lr[at, at] = 0.0
+    assert np.array_equal(stored, pattern)
+    fine = ~pattern[:, at]
+    fine[at] = False
+    fine |= kernel == "binary"
+    assert np.array_equal(dense[fine], Lr[fine])
