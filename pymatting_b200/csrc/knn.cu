@@ -391,27 +391,40 @@ __device__ __forceinline__ double edge_value(const Passes& P, int pi, long long 
     return __dsub_rn(1.0, (double)__fdiv_rn(s, (float)kDims));
 }
 
-// in-degree of every row (edges q -> j give row j an entry)
-__global__ void k_indegree(Passes P, long long n, int64_t* cap) {
+// Whether pixel q is in one of its own lists. It is not where more than k
+// pixels are equal to it and have smaller indices; its row then gets an entry
+// (q, q) of weight zero, which L = I - D^-1 W needs for its diagonal.
+__device__ __forceinline__ bool lists_itself(const Passes& P, long long q) {
+    for (int pi = 0; pi < P.np; ++pi)
+        for (int e = 0; e < P.p[pi].k; ++e)
+            if (P.p[pi].nbr[q * P.p[pi].k + e] == q) return true;
+    return false;
+}
+
+// Entries of every row: its own, and one for each edge q -> j that gives row
+// j one.
+__global__ void k_degree(Passes P, long long n, int kt, int64_t* cap) {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (q >= n) return;
     for (int pi = 0; pi < P.np; ++pi)
         for (int e = 0; e < P.p[pi].k; ++e)
             atomicAdd((unsigned long long*)(cap + P.p[pi].nbr[q * P.p[pi].k + e]), 1ull);
+    atomicAdd((unsigned long long*)(cap + q), (unsigned long long)(kt + !lists_itself(P, q)));
 }
 
-__global__ void k_add_outdegree(long long n, int kt, int64_t* cap) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < n) cap[i] += kt;
-}
-
-// Scatter: own neighbours at the start of the row's slots, reverse edges
-// after them (slot claimed with an atomic counter).
+// Scatter: own neighbours at the start of the row's slots, the others (reverse
+// edges, the zero on the diagonal) after them (slot claimed with an atomic
+// counter).
 __global__ void k_scatter(Passes P, long long n, int kt, const int64_t* off, int64_t* fillc,
                           int64_t* cols, double* vals) {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (q >= n) return;
     long long o = off[q];
+    auto put = [&](long long row, long long col, double v) {
+        const long long slot = off[row] + kt + (long long)atomicAdd((unsigned long long*)(fillc + row), 1ull);
+        cols[slot] = col;
+        vals[slot] = v;
+    };
     for (int pi = 0; pi < P.np; ++pi)
         for (int e = 0; e < P.p[pi].k; ++e) {
             const long long j = P.p[pi].nbr[q * P.p[pi].k + e];
@@ -419,11 +432,9 @@ __global__ void k_scatter(Passes P, long long n, int kt, const int64_t* off, int
             cols[o] = j;
             vals[o] = v;
             ++o;
-            const long long slot = off[j] + kt +
-                                   (long long)atomicAdd((unsigned long long*)(fillc + j), 1ull);
-            cols[slot] = q;
-            vals[slot] = v;
+            put(j, q, v);
         }
+    if (!lists_itself(P, q)) put(q, q, 0.0);
 }
 
 // Order-preserving map of doubles to unsigned. A total order: NaN, which the
@@ -580,13 +591,14 @@ static long long search_elems(long long n) {
 // Scratch elements (int64) for pmb_launch_knn with n pixels, total
 // neighbours per pixel kt and passes np: features, neighbour lists, row
 // capacities / offsets / fill counters / unique counts, and the unmerged
-// W (2 n kt columns + values). The search's ordered points, boxes and buckets
-// share the space of W, which is filled after it.
+// W (2 n kt entries and at most n zeros on the diagonal, columns + values).
+// The search's ordered points, boxes and buckets share the space of W, which is
+// filled after it.
 int64_t pmb_launch_knn_scratch(long long n, int kt, int np) {
     if (n <= 0 || kt <= 0 || np <= 0 || np > 4) return -1;
     const long long feat = (n * kDims * np * 4 + 7) / 8;  // floats -> int64 slots
     return feat + n * kt + 4 * (n + 1) + ((n + 1) + 1023) / 1024 + 2 +
-           std::max(2 * (2 * n * kt), search_elems(n));
+           std::max(2 * (2 * n * kt + n), search_elems(n));
 }
 
 // Two calls on the same scratch and rowptr. First (cols / vals null): the
@@ -618,7 +630,7 @@ int pmb_launch_knn(const double* image, int h, int w, const int* ks, const doubl
     int64_t* chunk = s;
     s += ((n + 1) + 1023) / 1024 + 2;
     int64_t* wcols = s;
-    s += 2 * n * kt;
+    s += 2 * n * kt + n;
     double* wvals = (double*)s;
     const int blocks = (int)((n + 255) / 256);
     if (cols && vals) {
@@ -660,8 +672,7 @@ int pmb_launch_knn(const double* image, int h, int w, const int* ks, const doubl
         nb += n * ks[p];
     }
     if (cudaMemsetAsync(cap, 0, 3 * (n + 1) * sizeof(int64_t), st) != cudaSuccess) return 1;
-    k_indegree<<<blocks, 256, 0, st>>>(P, n, cap);
-    k_add_outdegree<<<blocks, 256, 0, st>>>(n, kt, cap);
+    k_degree<<<blocks, 256, 0, st>>>(P, n, kt, cap);
     cudaMemcpyAsync(off, cap, n * sizeof(int64_t), cudaMemcpyDeviceToDevice, st);
     if (pmb_scan_exclusive(off, n, chunk, off + n, st)) return 1;
     cudaMemsetAsync(fillc, 0, (n + 1) * sizeof(int64_t), st);
