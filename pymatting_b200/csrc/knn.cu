@@ -43,8 +43,15 @@ __device__ __forceinline__ float unordered(unsigned u) {
     return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u);
 }
 
-// Features, and their extent: ext[d] = smallest, ext[kDims + d] = largest
-// (ordered; the smallest inverted, so that both start at 0 and grow).
+__device__ __forceinline__ bool all_finite(const float (&f)[kDims]) {
+    bool ok = true;
+#pragma unroll
+    for (int d = 0; d < kDims; ++d) ok = ok && isfinite(f[d]);
+    return ok;
+}
+
+// Features, and the extent of the finite ones: ext[d] = smallest, ext[kDims + d]
+// = largest (ordered; the smallest inverted, so that both start at 0 and grow).
 __global__ void __launch_bounds__(256) k_features(const double* __restrict__ image, int h, int w, double dw,
                                                   float* __restrict__ f, unsigned* ext) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -68,7 +75,7 @@ __global__ void __launch_bounds__(256) k_features(const double* __restrict__ ima
     __syncthreads();
 #pragma unroll
     for (int d = 0; d < kDims; ++d) {
-        const bool ok = in && v[d] == v[d];
+        const bool ok = in && isfinite(v[d]);
         const unsigned o = ok ? ordered(v[d]) : 0u;
         const unsigned hi = __reduce_max_sync(0xffffffffu, o);
         const unsigned lo = __reduce_max_sync(0xffffffffu, ok ? ~o : 0u);
@@ -242,6 +249,17 @@ __global__ void __launch_bounds__(kKnnWarps * 32) k_knn(const float* __restrict_
         qlo[d] = box[d * ntiles + own];
         qhi[d] = box[(kDims + d) * ntiles + own];
     }
+    // A query with a feature that is not finite is infinitely far from every
+    // point, so its list is the first k. Its lane goes along with a finite one
+    // (a search of its own, which no tile can be left out of, kept the warp busy
+    // with all of 65536 points for 14 ms a pass).
+    const unsigned finite = __ballot_sync(0xffffffffu, all_finite(qf));
+    const int with = finite >> lane & 1 ? lane : max(__ffs(finite) - 1, 0);
+#pragma unroll
+    for (int d = 0; d < kDims; ++d) {
+        const float v = __shfl_sync(0xffffffffu, qf[d], with);
+        qf[d] = finite ? v : 0.f;
+    }
     int cnt = 0, maxpos = 0, maxI = 0;
     double maxD = 0.0;
     float thr = in ? __int_as_float(0x7f800000) : -1.f;     // bound of the k-th distance
@@ -367,7 +385,10 @@ __global__ void __launch_bounds__(kKnnWarps * 32) k_knn(const float* __restrict_
     drain();
     if (in) {
         const long long i = sidx[q];
-        for (int s = 0; s < k; ++s) nbr[i * k + s] = s < cnt ? I[s * 32] : i;
+#pragma unroll
+        for (int d = 0; d < kDims; ++d) qf[d] = sf[d * np + q];
+        const bool found = all_finite(qf);
+        for (int s = 0; s < k; ++s) nbr[i * k + s] = !found ? s : s < cnt ? I[s * 32] : i;
     }
 }
 
