@@ -691,12 +691,16 @@ k_vc_up(WorkList wl /* fine tiles */, const GridDesc* coarse, const CUtensorMap*
         const GridDesc gc = coarse[m.g];
         const int bx = m.x0 - kBOX, by = m.y0 - 2;
         const int cx0 = (m.x0 >> 1) - 4, cy0 = (m.y0 >> 1) - 2;
-        mbar_expect_tx(&pipe.bar[bb], ((kNH + 1 + (PRE > 1 ? 1 : 0)) * kBH * kBW + kCBH * kCBW) *
+        // A grid one pixel wide or high halves to an empty one, which has no
+        // descriptor (a load through it is an illegal instruction) and whose
+        // box the prolongation does not read.
+        const bool any = gc.h > 0 && gc.w > 0;
+        mbar_expect_tx(&pipe.bar[bb], ((kNH + 1 + (PRE > 1 ? 1 : 0)) * kBH * kBW + (any ? kCBH * kCBW : 0)) *
                                           sizeof(T));
         tma_load_3d(sP[bb], map_of(maps, gf, kMapPlF), bx, by, 0, &pipe.bar[bb]);
         tma_load_2d(sX[bb], map_of(maps, gf, kMapBF), bx, by, &pipe.bar[bb]);
         if (PRE > 1) tma_load_2d(sS[bb], map_of(maps, gf, xs_slot), bx, by, &pipe.bar[bb]);
-        tma_load_2d(sC[bb], map_of(maps, gc, kMapXC), cx0, cy0, &pipe.bar[bb]);
+        if (any) tma_load_2d(sC[bb], map_of(maps, gc, kMapXC), cx0, cy0, &pipe.bar[bb]);
     };
     auto body = [&](const Meta& m, const GridDesc& gf, int bb) {
         const GridDesc gc = coarse[m.g];
@@ -1392,20 +1396,23 @@ k_vc_tail(const TailDesc<T>* __restrict__ descs, const InstState* st, double ome
         }
         s_off[nlev] = off;
         mbar_init(&s_bar, 1);
-        // Planes of every level (one block each) and the first level's b.
+        // Planes of every level (one block each) and the first level's b; the
+        // coarsest level may have no rows.
         uint32_t bytes = 0;
         for (int l = 0; l < nlev; ++l) bytes += kNH * D.lev[l].g.pstride * sizeof(T);
         bytes += D.lev[0].g.pstride * sizeof(T);
         mbar_expect_tx(&s_bar, bytes);
         for (int l = 0; l < nlev; ++l) {
             const GridDesc g = D.lev[l].g;
-            bulk_load(sm + s_off[l], D.lev[l].P + g.poff,
-                      (uint32_t)(kNH * g.pstride * sizeof(T)), &s_bar);
+            if (g.pstride > 0)
+                bulk_load(sm + s_off[l], D.lev[l].P + g.poff,
+                          (uint32_t)(kNH * g.pstride * sizeof(T)), &s_bar);
         }
         grid_wait();
         const GridDesc g0 = D.lev[0].g;
-        bulk_load(sm + s_off[0] + kNH * g0.pstride, D.lev[0].b + g0.voff,
-                  (uint32_t)(g0.pstride * sizeof(T)), &s_bar);
+        if (g0.pstride > 0)
+            bulk_load(sm + s_off[0] + kNH * g0.pstride, D.lev[0].b + g0.voff,
+                      (uint32_t)(g0.pstride * sizeof(T)), &s_bar);
     }
     grid_wait();
     __syncthreads();
