@@ -694,8 +694,10 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
                 L[m] = pipe_quotient(a[m], sj, y);
             }
             if (__any_sync(all, odd)) {
+                // + 0.0: a quotient that underflows to -0.0 is an entry too
+                // (kept where the threshold is negative).
 #pragma unroll
-                for (int m = 0; m < M; ++m) L[m] = a[m] / sj;
+                for (int m = 0; m < M; ++m) L[m] = a[m] / sj + 0.0;
             }
 #pragma unroll
             for (int m = 0; m < M; ++m) {
