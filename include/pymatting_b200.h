@@ -411,6 +411,13 @@ int pmb_ichol_levels(const pmb_ichol* f);
  * would fill (1..8), 0 for more than 8 (bandwidth above 448), -1 before any
  * factor. */
 int pmb_ichol_cluster(const pmb_ichol* f);
+/* Kernel that made the last factor: 1 the pipeline of warps, 0 the band front in
+ * global memory (bandwidth above 1024), 3 the same after a wait of the pipeline
+ * ran out; -1 before any factor. */
+int pmb_ichol_kernel(const pmb_ichol* f);
+/* Polls after which the pipeline's waits give up (negative: the default, 2^22;
+ * 0: at once), for the tests. */
+int pmb_ichol_wait_limit(pmb_ichol* f, int64_t polls);
 /* Device time (CUDA events on the factor's stream) of the factorisation
  * kernel in the last pmb_ichol_factor, in milliseconds; -1 before any. */
 float pmb_ichol_factor_ms(const pmb_ichol* f);

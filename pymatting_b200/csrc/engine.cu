@@ -1866,6 +1866,8 @@ struct Ichol {
     int64_t nnz = -1;
     int nlevels = 0;
     int cluster = -1;     // size class of the last factorisation (ichol_cluster_size)
+    int kernel = -1;      // kIcholBy... of the last factorisation
+    uint32_t wait_limit = kPipeSpinLimit;
     cudaEvent_t ev_f0 = nullptr, ev_f1 = nullptr;   // around the factor kernel
     float factor_ms = -1.0f;
     // Streamed solves (n <= kStreamMaxRows): chunk blocks of both sweeps.
@@ -2083,11 +2085,14 @@ PMB_API int pmb_ichol_factor(pmb_ichol* p, const int64_t* Ap, const int64_t* Ar,
                                  I.at<int>(I.o_level), I.at<int64_t>(I.o_Lp), I.at<int64_t>(I.o_Lr),
                                  I.at<double>(I.o_Lv), I.at<double>(I.o_F), I.at<uint16_t>(I.o_Rc), I.cap,
                                  discard_threshold, max_nnz, relative_discard_threshold, diag_keep_discarded,
-                                 I.at<int64_t>(I.o_result), s)) {
+                                 I.at<int64_t>(I.o_result), I.wait_limit, s)) {
         PMB_CUDA(cudaGetLastError());
         PMB_CUDA(cudaEventRecord(I.ev_f1, s));
         PMB_CUDA(cudaMemcpyAsync(&res, I.ws + I.o_result, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
         PMB_CUDA(cudaStreamSynchronize(s));
+        I.kernel = res == kIcholRetry ? kIcholByRetry : kIcholByPipe;
+    } else {
+        I.kernel = kIcholByGlobal;
     }
     if (res == kIcholRetry) {
         PMB_CUDA(cudaMemsetAsync(I.ws + I.o_F, 0, sizeof(double) * W * W, s));
@@ -2141,6 +2146,12 @@ PMB_API int pmb_ichol_factor(pmb_ichol* p, const int64_t* Ap, const int64_t* Ar,
 PMB_API int pmb_ichol_levels(const pmb_ichol* p) { return p ? p->I.nlevels : -1; }
 
 PMB_API int pmb_ichol_cluster(const pmb_ichol* p) { return p ? p->I.cluster : -1; }
+PMB_API int pmb_ichol_kernel(const pmb_ichol* p) { return p ? p->I.kernel : -1; }
+PMB_API int pmb_ichol_wait_limit(pmb_ichol* p, int64_t polls) {
+    if (!p || polls > 0xffffffffll) return fail(kErrArg, "pmb_ichol_wait_limit: bad arguments");
+    p->I.wait_limit = polls < 0 ? kPipeSpinLimit : (uint32_t)polls;
+    return 0;
+}
 
 PMB_API float pmb_ichol_factor_ms(const pmb_ichol* p) { return p ? p->I.factor_ms : -1.0f; }
 

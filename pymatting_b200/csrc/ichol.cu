@@ -288,7 +288,6 @@ constexpr int kLag = 4;
 constexpr int kDense = 8;             // dense columns kept (a power of two above kLag)
 constexpr int kPipeMaxChunks = 32;    // 32-offset chunks of a column: W <= 1025
 constexpr int kBatch = 2;             // nodes whose entries a walker has in flight
-constexpr uint32_t kPipeSpinLimit = 1u << 22;
 constexpr int kPipeStop = 0x7fffffff;
 constexpr int64_t kPipeMax = (int64_t)1 << 30;
 
@@ -357,7 +356,7 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
                     const double* __restrict__ Av, const double* __restrict__ d0,
                     const double* __restrict__ rsum, int* level, int64_t* Lp, int64_t* Lr, double* Lv,
                     int2* list, uint16_t* offs, int64_t cap, double discard, int64_t max_nnz, double rel_discard,
-                    int diag_keep, int64_t* result) {
+                    int diag_keep, int64_t* result, uint32_t limit) {
     extern __shared__ __align__(16) unsigned char pipe_smem[];
     constexpr int kWalkers = pipe_walkers(kFin);
     __shared__ __align__(16) int s_count[2][kFin * M];  // candidates << 16 | kept, per chunk
@@ -415,7 +414,7 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
                 const int cnt_ = *(volatile int*)&rowcnt[slot];
                 const int done = __shfl_sync(all, done_, 0);
                 int cnt = __shfl_sync(all, cnt_, 0);
-                if (done == kPipeStop || spins >= kPipeSpinLimit) {
+                if (done == kPipeStop || spins >= limit) {
                     stop = true;
                     break;
                 }
@@ -507,7 +506,7 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
         int wk = 0;
         auto await = [&](int c) {             // accumulator of column c, c = ready
             bool ok = false;
-            for (uint32_t spins = 0; spins < kPipeSpinLimit; ++spins) {
+            for (uint32_t spins = 0; spins < limit; ++spins) {
                 if (__shfl_sync(all, *(volatile int*)&s_ready[wk], 0) >= c) {
                     ok = true;
                     break;
@@ -1213,13 +1212,13 @@ void ichol_launch_init(int64_t n, const int64_t* Ap, const int64_t* Ar, const do
     if (n > 0) k_ichol_init<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, Ap, Ar, Av, shift, d, rsum, level, band);
 }
 
-// The pipelined kernel, for the bandwidths that its shared memory takes.
-// False: not launched. `list` holds max(W, kPipeMinW)^2 doubles.
+// The pipelined kernel, for the bandwidths that its shared memory takes; limit:
+// polls after which a wait gives up. False: not launched. `list` holds max(W, kPipeMinW)^2 doubles.
 bool ichol_launch_factor_pipe(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
                               const double* Av, const double* d, const double* rsum, int* level,
                               int64_t* Lp, int64_t* Lr, double* Lv, double* list, uint16_t* offs, int64_t cap,
                               double discard, int64_t max_nnz, double rel, int diag_keep,
-                              int64_t* result, cudaStream_t s) {
+                              int64_t* result, uint32_t limit, cudaStream_t s) {
     W = W < kPipeMinW ? kPipeMinW : W;
     if (W > 32 * kPipeMaxChunks + 1 || n > kPipeMax || cap > kPipeMax) return false;
     const int chunks = (int)((W - 1 + 31) / 32);
@@ -1237,7 +1236,7 @@ bool ichol_launch_factor_pipe(int64_t n, int64_t W, const int64_t* Ap, const int
     }
     kern<<<1, 32 * pipe_warps(fin), L.bytes, s>>>((int)n, (int)W, Ap, Ar, Av, d, rsum, level, Lp, Lr, Lv,
                                           reinterpret_cast<int2*>(list), offs, cap, discard, max_nnz, rel,
-                                          diag_keep, result);
+                                          diag_keep, result, limit);
     return true;
 }
 

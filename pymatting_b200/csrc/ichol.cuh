@@ -61,12 +61,16 @@ void ichol_launch_init(int64_t n, const int64_t* Ap, const int64_t* Ar, const do
 // Result of the pipelined kernel when a wait ran out: the factor is made by
 // ichol_launch_factor.
 constexpr int64_t kIcholRetry = -100;
+constexpr uint32_t kPipeSpinLimit = 1u << 22;
+// Kernel that made a factor: the front in global memory (also after a retry),
+// or the pipeline.
+enum : int { kIcholByGlobal = 0, kIcholByPipe = 1, kIcholByRetry = 3 };
 constexpr int64_t kPipeMinW = 8;      // rows of its ring (narrower bands are padded)
 bool ichol_launch_factor_pipe(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
                               const double* Av, const double* d, const double* rsum, int* level,
                               int64_t* Lp, int64_t* Lr, double* Lv, double* list, uint16_t* offs, int64_t cap,
                               double discard, int64_t max_nnz, double rel, int diag_keep,
-                              int64_t* result, cudaStream_t s);
+                              int64_t* result, uint32_t limit, cudaStream_t s);
 // The global-front kernel: bands that the pipelined kernel does not take.
 void ichol_launch_factor(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
                         const double* Av, double* d, const double* rsum, int* level, double* F,

@@ -230,6 +230,9 @@ class CsrSystem:
         return SolveStats(it.value, st.value, nr.value, nb.value)
 
 
+_ICHOL_KERNELS = {-1: None, 0: "global", 1: "pipeline", 3: "global after a pipeline wait ran out"}
+
+
 class IcholFactor:
     """Device thresholded incomplete Cholesky factor (pmb_ichol)."""
 
@@ -274,6 +277,10 @@ class IcholFactor:
         """Size class of the last factorisation: the CTAs whose shared memory
         its band front would fill (0: more than 8)."""
         return int(_ffi.lib().pmb_ichol_cluster(self._h))
+
+    def kernel(self):
+        """Kernel that made the last factor (pmb_ichol_kernel)."""
+        return _ICHOL_KERNELS[int(_ffi.lib().pmb_ichol_kernel(self._h))]
 
     def apply(self, b):
         x = dev.empty(self.n, torch.float64)
