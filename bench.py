@@ -705,7 +705,7 @@ def run_hard(args, rank, world, local):
             "dtype": "f64", "data": "synthetic",
             "config": {"workload": "estimate_alpha_cf_hard_ichol_320x240", "image": "320x240x3",
                        "unknowns": n, "factor_nnz": nnz_l, "levels": M.factor.levels(),
-                       "cluster_ctas": M.factor.cluster(),
+                       "factor_kernel": M.factor.kernel(),
                        "l2": "flushed between steps (256 MB write)",
                        "parallelism": "weak: one image per GPU, no collective"},
             "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s",

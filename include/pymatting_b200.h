@@ -408,10 +408,10 @@ int pmb_ichol_factor(pmb_ichol* f, const int64_t* Ap, const int64_t* Ar, const d
 /* Dependency levels of the factor (length of the triangular-solve schedule). */
 int pmb_ichol_levels(const pmb_ichol* f);
 /* Size class of the last factor: the CTAs whose shared memory its band front
- * would fill (1..8), 0 for more than 8 (bandwidth above 448), -1 before any
- * factor. */
+ * fills (1..8), 0 for more than 8, -1 before any factor. */
 int pmb_ichol_cluster(const pmb_ichol* f);
-/* Kernel that made the last factor: 1 the pipeline of warps, 0 the band front in
+/* Kernel that made the last factor: 1 the pipeline of warps, 2 the band front in
+ * the shared memory of a cluster (wide bands with long columns), 0 the front in
  * global memory (bandwidth above 1024), 3 the same after a wait of the pipeline
  * ran out; -1 before any factor. */
 int pmb_ichol_kernel(const pmb_ichol* f);

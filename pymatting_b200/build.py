@@ -30,6 +30,7 @@ SOURCES = {
     "laplacians.cu": [],
     "knn.cu": [],
     "ichol.cu": ["-fmad=false"],
+    "ichol_cluster.cu": ["-fmad=false"],
     "engine.cu": [],
 }
 HEADERS = ["pm_common.cuh", "stencil.cuh", "csr.cuh", "ichol.cuh"]

@@ -2079,20 +2079,49 @@ PMB_API int pmb_ichol_factor(pmb_ichol* p, const int64_t* Ap, const int64_t* Ar,
         PMB_CUDA(cudaEventCreate(&I.ev_f1));
     }
     PMB_CUDA(cudaEventRecord(I.ev_f0, s));
-    int64_t res = kIcholRetry;
-    I.cluster = ichol_cluster_size(W);
-    if (ichol_launch_factor_pipe(n, W, Ap, Ar, Av, I.at<double>(I.o_d), I.at<double>(I.o_rsum),
-                                 I.at<int>(I.o_level), I.at<int64_t>(I.o_Lp), I.at<int64_t>(I.o_Lr),
-                                 I.at<double>(I.o_Lv), I.at<double>(I.o_F), I.at<uint16_t>(I.o_Rc), I.cap,
-                                 discard_threshold, max_nnz, relative_discard_threshold, diag_keep_discarded,
-                                 I.at<int64_t>(I.o_result), I.wait_limit, s)) {
+    auto outcome = [&](int64_t& r) -> int {
         PMB_CUDA(cudaGetLastError());
         PMB_CUDA(cudaEventRecord(I.ev_f1, s));
-        PMB_CUDA(cudaMemcpyAsync(&res, I.ws + I.o_result, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+        PMB_CUDA(cudaMemcpyAsync(&r, I.ws + I.o_result, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
         PMB_CUDA(cudaStreamSynchronize(s));
+        return 0;
+    };
+    // The pipeline, or the cluster where columns are longer than
+    // ichol_dense_columns says: the envelope tells if nothing is discarded, else
+    // the pipeline looks at every W columns in the first eighth (fill grows for
+    // several W; the pipeline is at most 1.8 times slower there, so a later
+    // start from the beginning would not pay).
+    int64_t res = kIcholRetry;
+    I.cluster = ichol_cluster_size(W);
+    const int64_t dense = ichol_dense_columns(W);
+    bool cluster = dense > 0 && !(discard_threshold > 0.0) && !(relative_discard_threshold > 0.0) &&
+                   std::min(I.cap / n, W - 1) > dense;
+    bool look = dense > 0 && n >= 16 * W;
+    I.kernel = kIcholByGlobal;
+    for (;;) {
+        if (cluster) {
+            if (ichol_launch_factor_cluster(n, W, Ap, Ar, Av, I.at<double>(I.o_d), I.at<double>(I.o_rsum),
+                                            I.at<int>(I.o_level), I.at<int64_t>(I.o_Lp), I.at<int64_t>(I.o_Lr),
+                                            I.at<double>(I.o_Lv), I.cap, discard_threshold, max_nnz,
+                                            relative_discard_threshold, diag_keep_discarded,
+                                            I.at<int64_t>(I.o_result), s)) {
+                if (int rc = outcome(res)) return rc;
+                I.kernel = kIcholByCluster;
+                break;
+            }
+            cluster = look = false;         // no room for a cluster: the pipeline to its end
+        }
+        if (!ichol_launch_factor_pipe(n, W, Ap, Ar, Av, I.at<double>(I.o_d), I.at<double>(I.o_rsum),
+                                      I.at<int>(I.o_level), I.at<int64_t>(I.o_Lp), I.at<int64_t>(I.o_Lr),
+                                      I.at<double>(I.o_Lv), I.at<double>(I.o_F), I.at<uint16_t>(I.o_Rc), I.cap,
+                                      discard_threshold, max_nnz, relative_discard_threshold,
+                                      diag_keep_discarded, I.at<int64_t>(I.o_result), I.wait_limit,
+                                      look ? (int)W : 0, n / 8, dense * W, s))
+            break;
+        if (int rc = outcome(res)) return rc;
         I.kernel = res == kIcholRetry ? kIcholByRetry : kIcholByPipe;
-    } else {
-        I.kernel = kIcholByGlobal;
+        if (res != kIcholDense) break;
+        cluster = true;
     }
     if (res == kIcholRetry) {
         PMB_CUDA(cudaMemsetAsync(I.ws + I.o_F, 0, sizeof(double) * W * W, s));
@@ -2103,10 +2132,7 @@ PMB_API int pmb_ichol_factor(pmb_ichol* p, const int64_t* Ap, const int64_t* Ar,
                             I.at<int64_t>(I.o_Lp), I.at<int64_t>(I.o_Lr), I.at<double>(I.o_Lv), I.cap,
                             discard_threshold, max_nnz, relative_discard_threshold, diag_keep_discarded,
                             I.at<int64_t>(I.o_result), s);
-        PMB_CUDA(cudaGetLastError());
-        PMB_CUDA(cudaEventRecord(I.ev_f1, s));
-        PMB_CUDA(cudaMemcpyAsync(&res, I.ws + I.o_result, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        PMB_CUDA(cudaStreamSynchronize(s));
+        if (int rc = outcome(res)) return rc;
     }
     PMB_CUDA(cudaEventElapsedTime(&I.factor_ms, I.ev_f0, I.ev_f1));
     *result = res;

@@ -233,20 +233,6 @@ k_ichol_factor(int64_t n, int64_t W, const int64_t* __restrict__ Ap,
     if (threadIdx.x == 0) *result = s_fail ? (int64_t)s_fail : s_nnz;
 }
 
-// CTAs of shared memory that the W x W band front of FP64 values, pattern and
-// lists would fill; 0 above 8, or wider than 449. A size class of the system
-// that callers can ask for; the pipeline below holds no front.
-int ichol_cluster_size(int64_t W) {
-    if (W < 1 || W - 1 > 32 * 14) return 0;
-    const int64_t Wp = (W + 7) & ~(int64_t)7;
-    for (int64_t C = 1; C <= 8; ++C) {
-        const int64_t S = (W + C - 1) / C;
-        const int64_t bytes = S * Wp * 9 + S * 12 + W * 32;
-        if (((bytes + 15) & ~(int64_t)15) <= (int64_t)kFactorSmem) return (int)C;
-    }
-    return 0;
-}
-
 // ---------------------------------------------------------------------------
 // The same factorisation, left-looking, as a pipeline of the warps of one CTA.
 //
@@ -356,7 +342,7 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
                     const double* __restrict__ Av, const double* __restrict__ d0,
                     const double* __restrict__ rsum, int* level, int64_t* Lp, int64_t* Lr, double* Lv,
                     int2* list, uint16_t* offs, int64_t cap, double discard, int64_t max_nnz, double rel_discard,
-                    int diag_keep, int64_t* result, uint32_t limit) {
+                    int diag_keep, int64_t* result, uint32_t limit, int look_cols, int look_end, int64_t dense_nnz) {
     extern __shared__ __align__(16) unsigned char pipe_smem[];
     constexpr int kWalkers = pipe_walkers(kFin);
     __shared__ __align__(16) int s_count[2][kFin * M];  // candidates << 16 | kept, per chunk
@@ -552,7 +538,8 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
         const int me = warp - kFin - 1;
         const bool first = me == 0 && lane == 0;
         int slot = 0;
-        int64_t nnz = 0;
+        int64_t nnz = 0, nnz_at = 0;
+        int look = look_cols > 0 ? look_cols : -1;      // column count of the next look
         double dnext = W < n ? d0[W] : 0.0;
         int psl[M], pcnt[M];                 // list lengths to publish for the column before
 #pragma unroll
@@ -635,6 +622,14 @@ k_ichol_factor_pipe(int n, int W, const int64_t* __restrict__ Ap, const int64_t*
                 }
                 nnz += 1 + kept;
                 slot = slot + 1 == W ? 0 : slot + 1;
+                if (j + 1 == look) {
+                    if (look > look_cols && nnz - nnz_at > dense_nnz && first) {
+                        s_result = kIcholDense;
+                        s_stop = 1;
+                    }
+                    nnz_at = nnz;
+                    look = look + look_cols <= look_end ? look + look_cols : -1;
+                }
             }
             pipe_barrier<kFin>(2);
         }
@@ -1213,12 +1208,15 @@ void ichol_launch_init(int64_t n, const int64_t* Ap, const int64_t* Ar, const do
 }
 
 // The pipelined kernel, for the bandwidths that its shared memory takes; limit:
-// polls after which a wait gives up. False: not launched. `list` holds max(W, kPipeMinW)^2 doubles.
+// polls after which a wait gives up; look_cols > 0: ends with kIcholDense if the
+// second look_cols columns, or any of the next up to column look_end, kept more
+// than dense_nnz entries. False: not launched. `list` holds max(W, kPipeMinW)^2 doubles.
 bool ichol_launch_factor_pipe(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
                               const double* Av, const double* d, const double* rsum, int* level,
                               int64_t* Lp, int64_t* Lr, double* Lv, double* list, uint16_t* offs, int64_t cap,
                               double discard, int64_t max_nnz, double rel, int diag_keep,
-                              int64_t* result, uint32_t limit, cudaStream_t s) {
+                              int64_t* result, uint32_t limit, int look_cols, int64_t look_end,
+                              int64_t dense_nnz, cudaStream_t s) {
     W = W < kPipeMinW ? kPipeMinW : W;
     if (W > 32 * kPipeMaxChunks + 1 || n > kPipeMax || cap > kPipeMax) return false;
     const int chunks = (int)((W - 1 + 31) / 32);
@@ -1236,7 +1234,7 @@ bool ichol_launch_factor_pipe(int64_t n, int64_t W, const int64_t* Ap, const int
     }
     kern<<<1, 32 * pipe_warps(fin), L.bytes, s>>>((int)n, (int)W, Ap, Ar, Av, d, rsum, level, Lp, Lr, Lv,
                                           reinterpret_cast<int2*>(list), offs, cap, discard, max_nnz, rel,
-                                          diag_keep, result, limit);
+                                          diag_keep, result, limit, look_cols, (int)look_end, dense_nnz);
     return true;
 }
 

@@ -61,16 +61,26 @@ void ichol_launch_init(int64_t n, const int64_t* Ap, const int64_t* Ar, const do
 // Result of the pipelined kernel when a wait ran out: the factor is made by
 // ichol_launch_factor.
 constexpr int64_t kIcholRetry = -100;
+// ... and when the columns are long: ichol_launch_factor_cluster makes it.
+constexpr int64_t kIcholDense = -101;
 constexpr uint32_t kPipeSpinLimit = 1u << 22;
 // Kernel that made a factor: the front in global memory (also after a retry),
-// or the pipeline.
-enum : int { kIcholByGlobal = 0, kIcholByPipe = 1, kIcholByRetry = 3 };
+// the pipeline, the front in a cluster's shared memory.
+enum : int { kIcholByGlobal = 0, kIcholByPipe = 1, kIcholByCluster = 2, kIcholByRetry = 3 };
 constexpr int64_t kPipeMinW = 8;      // rows of its ring (narrower bands are padded)
 bool ichol_launch_factor_pipe(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
                               const double* Av, const double* d, const double* rsum, int* level,
                               int64_t* Lp, int64_t* Lr, double* Lv, double* list, uint16_t* offs, int64_t cap,
                               double discard, int64_t max_nnz, double rel, int diag_keep,
-                              int64_t* result, uint32_t limit, cudaStream_t s);
+                              int64_t* result, uint32_t limit, int look_cols, int64_t look_end,
+                              int64_t dense_nnz, cudaStream_t s);
+// The front in a cluster's shared memory (ichol_cluster.cu). False: not launched.
+bool ichol_launch_factor_cluster(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
+                                 const double* Av, const double* d, const double* rsum, int* level,
+                                 int64_t* Lp, int64_t* Lr, double* Lv, int64_t cap, double discard,
+                                 int64_t max_nnz, double rel, int diag_keep, int64_t* result,
+                                 cudaStream_t s);
+int64_t ichol_dense_columns(int64_t W);
 // The global-front kernel: bands that the pipelined kernel does not take.
 void ichol_launch_factor(int64_t n, int64_t W, const int64_t* Ap, const int64_t* Ar,
                         const double* Av, double* d, const double* rsum, int* level, double* F,
@@ -85,7 +95,8 @@ void ichol_launch_rows(int64_t n, const int64_t* Lp, const int64_t* Lr, const do
 void ichol_launch_row_fill(int64_t n, const int64_t* Lp, const int64_t* Lr, const double* Lv,
                            int64_t* rfill, int64_t* Rc, double* Rv, const int64_t* Rp,
                            cudaStream_t s);
-// Size class of a band of W rows (see ichol.cu).
+// CTAs of the cluster whose shared memory the band front of W rows fills; 0 if
+// it has no room there.
 int ichol_cluster_size(int64_t W);
 void ichol_prepare();
 void ichol_launch_solve(int64_t n, int nlevels, const int64_t* lptr, const int* order,

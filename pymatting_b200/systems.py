@@ -230,7 +230,8 @@ class CsrSystem:
         return SolveStats(it.value, st.value, nr.value, nb.value)
 
 
-_ICHOL_KERNELS = {-1: None, 0: "global", 1: "pipeline", 3: "global after a pipeline wait ran out"}
+_ICHOL_KERNELS = {-1: None, 0: "global", 1: "pipeline", 2: "cluster",
+                  3: "global after a pipeline wait ran out"}
 
 
 class IcholFactor:
@@ -275,7 +276,7 @@ class IcholFactor:
 
     def cluster(self):
         """Size class of the last factorisation: the CTAs whose shared memory
-        its band front would fill (0: more than 8)."""
+        its band front fills (0: more than 8)."""
         return int(_ffi.lib().pmb_ichol_cluster(self._h))
 
     def kernel(self):

@@ -57,3 +57,35 @@ def test_failure_codes_after_a_wait_that_ran_out(gpu):
         assert _factor(A, polls, discard=0.0, max_nnz=A.shape[0] + 10)[1] == -2
         f, nnz = _factor(A, polls)
         assert nnz > 0
+
+
+# Bands around the first width with a cluster of 4 and the last that fits 8
+# CTAs, nothing discarded: columns of nearly the whole band.
+@pytest.mark.parametrize("w,kernel", [(250, "pipeline"), (290, "cluster"), (300, "cluster"), (400, "cluster"),
+                                      (430, "cluster"), (446, "pipeline")])
+@pytest.mark.parametrize("keep", [True, False])
+def test_long_columns(gpu, w, kernel, keep):
+    import pymatting_b200 as pm
+    A = grid_laplacian(8, w, 1e-2, w)
+    f, _nnz = _factor(A, discard=0.0, keep=keep)
+    assert f.kernel() == kernel
+    check_factor(pm, A, discard_threshold=0.0, diag_keep_discarded=keep)
+
+
+def test_long_columns_are_seen_by_the_pipeline(gpu):
+    """A small threshold: the pipeline's first columns tell, where there are
+    many more to come. The factors are the same."""
+    import pymatting_b200 as pm
+    w = 400
+    A = grid_laplacian(34, w, 1e-2, 3)
+    assert _factor(A, discard=1e-14)[0].kernel() == "cluster"
+    assert _factor(A, discard=1e-2)[0].kernel() == "pipeline"
+    assert _factor(grid_laplacian(15, w, 1e-2, 3), discard=1e-14)[0].kernel() == "pipeline"
+    check_factor(pm, A, discard_threshold=1e-14)
+
+
+def test_failure_codes_of_long_columns(gpu):
+    A = grid_laplacian(8, 300, 1e-2, 1)
+    assert _factor(A, discard=0.0)[0].kernel() == "cluster"
+    assert _factor(A, discard=0.0, shift=-50.0)[1] == -1
+    assert _factor(A, discard=0.0, max_nnz=3 * A.shape[0])[1] == -2
