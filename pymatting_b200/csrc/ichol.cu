@@ -979,7 +979,10 @@ k_ichol_solve_smem(int64_t n, int nlevels, const int64_t* __restrict__ lptr,
 // across the warp, as in k_ichol_solve_smem, and x_i = (x_i - sum) / L_ii as
 // the reference's back substitutions (ichol.py:116-145). 7,815 rows in 2,301
 // levels: 1.48 -> 1.21 ms for both sweeps, about 500 cycles per chunk, of
-// which the five shuffle steps of the reduction are the largest part.
+// which the five shuffle steps of the reduction are the largest part. Terms
+// beyond the 64 in registers go in groups whose loads are in flight together:
+// 7,200 rows of 289 entries 10.3 (two at a time, no registers) and 14.0 (one
+// at a time) -> 8.9 ms, 10,985 rows of 45 entries 3.01 -> 2.42 ms.
 // ---------------------------------------------------------------------------
 
 constexpr int kStreamWarps = 8;       // that take rows; one more for the copies
@@ -1038,6 +1041,29 @@ k_ichol_solve_stream(int64_t n, int total, StreamFirst first, const unsigned cha
         col = reinterpret_cast<const int*>(val + h->ents);
         return h->rows;
     };
+    // Terms e, e + 32, ... of a row, the loads of kTerms in flight.
+    auto terms = [&](const double* val, const int* col, int count, int e, double& acc) {
+        constexpr int kTerms = 4;
+        for (; e < count; e += 32 * kTerms) {
+            double v[kTerms];
+            int i[kTerms];
+#pragma unroll
+            for (int u = 0; u < kTerms; ++u) {
+                v[u] = 0.0;
+                i[u] = 0;
+                if (e + 32 * u < count) {
+                    v[u] = val[e + 32 * u];
+                    i[u] = col[e + 32 * u];
+                }
+            }
+            double x[kTerms];
+#pragma unroll
+            for (int u = 0; u < kTerms; ++u) x[u] = sx[i[u]];
+#pragma unroll
+            for (int u = 0; u < kTerms; ++u)
+                if (e + 32 * u < count) acc += v[u] * x[u];
+        }
+    };
     auto fetch = [&](int c) {
         const StreamRow* rec;
         const double* val;
@@ -1080,7 +1106,7 @@ k_ichol_solve_stream(int64_t n, int total, StreamFirst first, const unsigned cha
             if (have) {
                 if (lane < r.count) acc += w0 * x0;
                 if (two) acc += w1 * x1;
-                for (int e = lane + 64; e < r.count; e += 32) acc += val[r.start + e] * sx[col[r.start + e]];
+                if (r.count > 64) terms(val + r.start, col + r.start, r.count, lane + 64, acc);
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
                 if (lane == 0) sx[r.row] = stream_quotient(xr - acc, r);
@@ -1088,7 +1114,7 @@ k_ichol_solve_stream(int64_t n, int total, StreamFirst first, const unsigned cha
             for (int k = warp + kStreamWarps; k < rows; k += kStreamWarps) {
                 const StreamRow rk = rec[k];
                 acc = 0.0;
-                for (int e = lane; e < rk.count; e += 32) acc += val[rk.start + e] * sx[col[rk.start + e]];
+                terms(val + rk.start, col + rk.start, rk.count, lane, acc);
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
                 if (lane == 0) sx[rk.row] = stream_quotient(sx[rk.row] - acc, rk);
