@@ -1133,47 +1133,75 @@ static bool any_running(const InstState* st, int n) {
     return false;
 }
 
+// Iterations of a first solve that launch their kernels, before the solve goes
+// on by replaying a graph of them. A graph costs 70 to 110 us to capture and
+// instantiate and 75 to 100 us to drop; an iteration of it saves, B200 with its
+// host, 24x32 to 1280x720:
+//   FP64 without a V-cycle (two launches, 18 us at least)   0.7 to 1.1 us
+//   mixed without a V-cycle (four)                          1.5 to 3.9 us
+//   V-cycle (5 to 17 launches, 37 us at least)              2.5 to 6.5 us
+//   CSR systems (15 us at least)                            5 to 6.6 us
+// A solve that ends soon after its line has paid for both. V-cycle solves take
+// up to 60 iterations, those of a nearest-neighbour Laplacian about 30, of a
+// random-walk or window one 50 and more: the lines lie between. With an
+// incomplete Cholesky factor, whose solves take a millisecond, the host is ahead
+// anyway.
+static int graph_after(const Stencil& S) {
+    return S.precond != kPrecVcycle && S.precision == 0 ? 192 : 96;
+}
+constexpr int kCsrGraphAfter = 36;
+
+// The graph of `chunk` iterations, unless the one at hand is of the same.
+template <typename T>
+static int capture_chunk(Stencil& S, int reorth) {
+    const int chunk = S.chunk;
+    if (S.graph && S.graph_reorth == reorth && S.graph_iters == chunk && S.graph_delta == S.delta &&
+        S.graph_max_outer == S.max_outer)
+        return 0;
+    if (S.graph) {
+        cudaGraphExecDestroy(S.graph);
+        S.graph = nullptr;
+    }
+    cudaGraph_t g;
+    PMB_CUDA(cudaStreamBeginCapture(S.stream, cudaStreamCaptureModeThreadLocal));
+    S.pass = 0;
+    for (int i = 0; i < chunk; ++i) cg_iteration<T>(S, reorth);
+    PMB_CUDA(cudaStreamEndCapture(S.stream, &g));
+    size_t nodes = 0;
+    PMB_CUDA(cudaGraphGetNodes(g, nullptr, &nodes));
+    PMB_CUDA(cudaGraphInstantiate(&S.graph, g, 0));
+    cudaGraphDestroy(g);
+    S.graph_iters = chunk;
+    S.graph_reorth = reorth;
+    S.graph_delta = S.delta;
+    S.graph_max_outer = S.max_outer;
+    S.graph_kernels = (int64_t)nodes;
+    // Capture only recorded the launches; they did not run.
+    S.launches -= (int64_t)nodes;
+    return 0;
+}
+
 // Iterate until every image has left the running state, `chunk` iterations
 // between looks at the states; images that finish early turn the remaining
 // kernels of the chunk into no-ops. A system's first solve launches its kernels
-// (the GPU takes longer than the host does, 13 launches of 2.5 us against 70 us
-// and more an iteration); one that is solved again replays a CUDA graph of the
-// chunk, whose capture and instantiation (0.3 ms, and 0.13 ms to drop it) only
-// then pay.
+// for graph_after iterations; what follows, and later solves, replay a graph.
 template <typename T>
 static int iterate(Stencil& S, int reorth, int maxiter) {
     const int chunk = S.chunk;
-    const bool replay = S.solves++ > 0;
+    bool replay = S.solves++ > 0;
     S.stats_fresh = false;
-    if (!replay) S.pass = 0;
-    if (replay && (!S.graph || S.graph_reorth != reorth || S.graph_iters != chunk ||
-        S.graph_delta != S.delta || S.graph_max_outer != S.max_outer)) {
-        if (S.graph) {
-            cudaGraphExecDestroy(S.graph);
-            S.graph = nullptr;
-        }
-        cudaGraph_t g;
-        PMB_CUDA(cudaStreamBeginCapture(S.stream, cudaStreamCaptureModeThreadLocal));
-        S.pass = 0;
-        for (int i = 0; i < chunk; ++i) cg_iteration<T>(S, reorth);
-        PMB_CUDA(cudaStreamEndCapture(S.stream, &g));
-        size_t nodes = 0;
-        PMB_CUDA(cudaGraphGetNodes(g, nullptr, &nodes));
-        PMB_CUDA(cudaGraphInstantiate(&S.graph, g, 0));
-        cudaGraphDestroy(g);
-        S.graph_iters = chunk;
-        S.graph_reorth = reorth;
-        S.graph_delta = S.delta;
-        S.graph_max_outer = S.max_outer;
-        S.graph_kernels = (int64_t)nodes;
-        // Capture only recorded the launches; they did not run.
-        S.launches -= (int64_t)nodes;
-    }
+    S.pass = 0;
+    if (replay)
+        if (int rc = capture_chunk<T>(S, reorth)) return rc;
     int done_iters = 0;
     for (;;) {
         if (int rc = read_states(S)) return rc;
         if (!any_running(S.h_state, S.nimg)) break;
         if (done_iters > maxiter + chunk) return fail(kErrState, "iteration control lost");
+        if (!replay && done_iters >= graph_after(S)) {
+            if (int rc = capture_chunk<T>(S, reorth)) return rc;
+            replay = true;
+        }
         if (replay) {
             PMB_CUDA(cudaGraphLaunch(S.graph, S.stream));
             S.launches += S.graph_kernels;
@@ -2276,6 +2304,21 @@ static void csr_iteration(Csr& C, cudaStream_t s) {
     csr_internal_precond(C, s);
 }
 
+// The graph of `chunk` iterations, unless there is one of the same kind.
+static int csr_capture(Csr& C, int chunk, int reorth) {
+    if (C.graph && C.graph_reorth == reorth) return 0;
+    if (C.graph) cudaGraphExecDestroy(C.graph);
+    C.graph = nullptr;
+    cudaGraph_t g;
+    PMB_CUDA(cudaStreamBeginCapture(C.stream, cudaStreamCaptureModeThreadLocal));
+    for (int i = 0; i < chunk; ++i) csr_iteration(C, C.stream);
+    PMB_CUDA(cudaStreamEndCapture(C.stream, &g));
+    PMB_CUDA(cudaGraphInstantiate(&C.graph, g, 0));
+    cudaGraphDestroy(g);
+    C.graph_reorth = reorth;
+    return 0;
+}
+
 template <typename Fn>
 static int csr_on_stream(Csr& C, cudaStream_t caller, Fn fn) {
     PMB_CUDA(cudaEventRecord(C.res.ev_in, caller));
@@ -2380,23 +2423,18 @@ PMB_API int pmb_csr_solve(pmb_csr* p, const double* b, const double* x0, double*
     return csr_on_stream(C, (cudaStream_t)stream, [&]() -> int {
         if (int rc = csr_begin(C, b, x0, atol, rtol, maxiter, reorthogonalize)) return rc;
         const int chunk = 4;
-        const bool replay = C.solves++ > 0;       // as in iterate()
-        if (replay && (!C.graph || C.graph_reorth != reorthogonalize)) {
-            if (C.graph) cudaGraphExecDestroy(C.graph);
-            C.graph = nullptr;
-            cudaGraph_t g;
-            PMB_CUDA(cudaStreamBeginCapture(C.stream, cudaStreamCaptureModeThreadLocal));
-            for (int i = 0; i < chunk; ++i) csr_iteration(C, C.stream);
-            PMB_CUDA(cudaStreamEndCapture(C.stream, &g));
-            PMB_CUDA(cudaGraphInstantiate(&C.graph, g, 0));
-            cudaGraphDestroy(g);
-            C.graph_reorth = reorthogonalize;
-        }
+        bool replay = C.solves++ > 0;             // as in iterate()
+        if (replay)
+            if (int rc = csr_capture(C, chunk, reorthogonalize)) return rc;
         int done = 0;
         for (;;) {
             if (int rc = csr_read_state(C)) return rc;
             if (C.h_state->status != kRunning) break;
             if (done > maxiter + chunk) return fail(kErrState, "iteration control lost");
+            if (!replay && done >= kCsrGraphAfter && C.mkind != kMIchol) {
+                if (int rc = csr_capture(C, chunk, reorthogonalize)) return rc;
+                replay = true;
+            }
             if (replay) PMB_CUDA(cudaGraphLaunch(C.graph, C.stream));
             else
                 for (int i = 0; i < chunk; ++i) csr_iteration(C, C.stream);
