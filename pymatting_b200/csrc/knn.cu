@@ -243,22 +243,24 @@ __global__ void __launch_bounds__(kKnnWarps * 32) k_knn(const float* __restrict_
     const long long q = own * kTile + lane;
     const bool in = q < n;
     float qf[kDims], qlo[kDims], qhi[kDims];
-#pragma unroll
-    for (int d = 0; d < kDims; ++d) {
-        qf[d] = sf[d * np + (in ? q : n - 1)];
-        qlo[d] = box[d * ntiles + own];
-        qhi[d] = box[(kDims + d) * ntiles + own];
-    }
     // A query with a feature that is not finite is infinitely far from every
     // point, so its list is the first k. Its lane goes along with a finite one
     // (a search of its own, which no tile can be left out of, kept the warp busy
     // with all of 65536 points for 14 ms a pass).
+#pragma unroll
+    for (int d = 0; d < kDims; ++d) qf[d] = sf[d * np + min(q, n - 1)];
     const unsigned finite = __ballot_sync(0xffffffffu, all_finite(qf));
-    const int with = finite >> lane & 1 ? lane : max(__ffs(finite) - 1, 0);
+    if (!finite) {
+        if (in)
+            for (int s = 0; s < k; ++s) nbr[(long long)sidx[q] * k + s] = s;
+        return;
+    }
+    const long long with = min(finite >> lane & 1 ? q : own * kTile + __ffs(finite) - 1, n - 1);
 #pragma unroll
     for (int d = 0; d < kDims; ++d) {
-        const float v = __shfl_sync(0xffffffffu, qf[d], with);
-        qf[d] = finite ? v : 0.f;
+        qf[d] = sf[d * np + with];
+        qlo[d] = box[d * ntiles + own];
+        qhi[d] = box[(kDims + d) * ntiles + own];
     }
     int cnt = 0, maxpos = 0, maxI = 0;
     double maxD = 0.0;

@@ -85,3 +85,16 @@ def test_one_bad_pixel_leaves_the_others_alone(gpu, monkeypatch, at, bad, kernel
     fine[at] = False
     fine |= kernel == "binary"
     assert np.array_equal(dense[fine], Lr[fine])
+
+
+@pytest.mark.parametrize("n_bad", [31, 33, 100, 600])
+def test_tiles_of_bad_pixels(gpu, monkeypatch, n_bad):
+    """Whole tiles of 32 points without a finite one; the last has 24 points."""
+    import pymatting_b200 as pm
+    monkeypatch.setattr(oracle, "knn", _knn_nan_last)
+    img = np.random.default_rng(2).random((20, 30, 3))
+    img.reshape(-1, 3)[np.random.default_rng(3).permutation(600)[:n_bad]] = np.nan
+    kw = dict(n_neighbors=[7, 5], distance_weights=[1.0, 0.1])
+    with np.errstate(all="ignore"):
+        Lr = oracle.knn_laplacian(img, **kw).toarray()
+    assert np.array_equal(pm.knn_laplacian(img, **kw).toarray(), Lr)
