@@ -33,7 +33,12 @@ SOURCES = {
     "ichol_cluster.cu": ["-fmad=false"],
     "engine.cu": [],
 }
-HEADERS = ["pm_common.cuh", "stencil.cuh", "csr.cuh", "ichol.cuh"]
+
+
+def headers():
+    """Every header of the library: all objects depend on all of them."""
+    names = [os.path.join(CSRC, f) for f in sorted(os.listdir(CSRC)) if f.endswith(".cuh")]
+    return names + [os.path.join(INCLUDE, "pymatting_b200.h")]
 
 
 def _nvcc():
@@ -52,8 +57,7 @@ def build(force=False, verbose=False):
     os.makedirs(LIBDIR, exist_ok=True)
     objdir = os.path.join(LIBDIR, "obj")
     os.makedirs(objdir, exist_ok=True)
-    headers = [os.path.join(CSRC, h) for h in HEADERS]
-    headers += [os.path.join(INCLUDE, "pymatting_b200.h")]
+    deps = headers()
     objs = []
     relink = force or not os.path.exists(TARGET)
     for src, extra in SOURCES.items():
@@ -62,7 +66,7 @@ def build(force=False, verbose=False):
             continue
         obj = os.path.join(objdir, src.replace(".cu", ".o"))
         objs.append(obj)
-        if force or _stale(obj, [path] + headers):
+        if force or _stale(obj, [path] + deps):
             cmd = [_nvcc()] + ARCH + COMMON + extra + ["-c", path, "-o", obj]
             if verbose:
                 print(" ".join(cmd))
