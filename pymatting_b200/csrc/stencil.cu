@@ -694,7 +694,7 @@ k_vc_up(WorkList wl /* fine tiles */, const GridDesc* coarse, const CUtensorMap*
         // A grid one pixel wide or high halves to an empty one, which has no
         // descriptor (a load through it is an illegal instruction) and whose
         // box the prolongation does not read.
-        const bool any = gc.h > 0 && gc.w > 0;
+        const bool any = gf.h > 1 && gf.w > 1;
         mbar_expect_tx(&pipe.bar[bb], ((kNH + 1 + (PRE > 1 ? 1 : 0)) * kBH * kBW + (any ? kCBH * kCBW : 0)) *
                                           sizeof(T));
         tma_load_3d(sP[bb], map_of(maps, gf, kMapPlF), bx, by, 0, &pipe.bar[bb]);
@@ -776,8 +776,11 @@ k_vc_up(WorkList wl /* fine tiles */, const GridDesc* coarse, const CUtensorMap*
 
 // One weighted Jacobi sweep xout = xin + omega (b - A xin) / d, or the first
 // sweep from zero xout = omega b / d when xin_slot < 0 (vcycle.py:32-43).
+// Shared memory holds one CTA per SM in FP64, two in FP32: the registers are
+// asked for as many (left to itself the compiler took 32, and 70 us instead of
+// 60 for a sweep of 1920x1080 in FP64).
 template <typename T>
-__global__ void __launch_bounds__(kTileThreads)
+__global__ void __launch_bounds__(kTileThreads, sizeof(T) == 8 ? 1 : 2)
 k_vc_smooth(WorkList wl, const CUtensorMap* maps, int xin_slot, const T* __restrict__ P,
             const T* __restrict__ b, T* xout, double omega, const InstState* st, int* err) {
     __shared__ __align__(8) uint64_t s_bar[2];
