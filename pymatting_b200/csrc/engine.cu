@@ -2304,11 +2304,16 @@ static void csr_iteration(Csr& C, cudaStream_t s) {
     csr_internal_precond(C, s);
 }
 
+// The graph holds the pointers of the matrix and of the preconditioner.
+static void csr_drop_graph(Csr& C) {
+    if (C.graph) cudaGraphExecDestroy(C.graph);
+    C.graph = nullptr;
+}
+
 // The graph of `chunk` iterations, unless there is one of the same kind.
 static int csr_capture(Csr& C, int chunk, int reorth) {
     if (C.graph && C.graph_reorth == reorth) return 0;
-    if (C.graph) cudaGraphExecDestroy(C.graph);
-    C.graph = nullptr;
+    csr_drop_graph(C);
     cudaGraph_t g;
     PMB_CUDA(cudaStreamBeginCapture(C.stream, cudaStreamCaptureModeThreadLocal));
     for (int i = 0; i < chunk; ++i) csr_iteration(C, C.stream);
@@ -2385,10 +2390,7 @@ PMB_API int pmb_csr_bind(pmb_csr* p, void* workspace, double* vectors, const int
         C.stream = C.res.stream;
         C.h_state = reinterpret_cast<InstState*>(C.res.pin);
     }
-    if (C.graph) {
-        cudaGraphExecDestroy(C.graph);
-        C.graph = nullptr;
-    }
+    csr_drop_graph(C);
     // Reduction counters must start at zero.
     PMB_CUDA(cudaMemsetAsync(C.ws + C.o_state, 0, sizeof(InstState), C.stream));
     PMB_CUDA(cudaStreamSynchronize(C.stream));
@@ -2402,6 +2404,7 @@ PMB_API int pmb_csr_set_matrix_preconditioner(pmb_csr* p, int64_t nnz, const int
     (void)nnz;
     (void)stream;
     p->C.M = CsrMat{indptr, indices, data};
+    csr_drop_graph(p->C);
     return 0;
 }
 
@@ -2409,6 +2412,7 @@ PMB_API int pmb_csr_set_ichol(pmb_csr* p, pmb_ichol* f, void* stream) {
     if (!p || !f || f->I.n != p->C.n) return fail(kErrArg, "pmb_csr_set_ichol: size mismatch");
     (void)stream;
     p->C.ich = &f->I;
+    csr_drop_graph(p->C);
     return 0;
 }
 
@@ -2525,7 +2529,7 @@ PMB_API int pmb_csr_destroy(pmb_csr* p) {
     if (!p) return 0;
     Csr& C = p->C;
     release_res(C.res);
-    if (C.graph) cudaGraphExecDestroy(C.graph);
+    csr_drop_graph(C);
     delete p;
     return 0;
 }
