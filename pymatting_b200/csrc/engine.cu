@@ -2267,6 +2267,7 @@ struct Csr {
     SolverRes res;
     cudaStream_t stream = nullptr;   // res.stream
     InstState* h_state = nullptr;
+    bool begun = false;              // the workspace holds a solve's state
     int64_t solves = 0;
     cudaGraphExec_t graph = nullptr;
     int graph_reorth = -1;
@@ -2335,8 +2336,22 @@ static int csr_on_stream(Csr& C, cudaStream_t caller, Fn fn) {
 }
 
 static int csr_read_state(Csr& C) {
+    if (!C.begun) {
+        if (!C.h_state) return fail(kErrState, "CSR system: not bound");
+        std::memset(C.h_state, 0, sizeof(InstState));
+        return 0;
+    }
     PMB_CUDA(cudaMemcpyAsync(C.h_state, C.state(), sizeof(InstState), cudaMemcpyDeviceToHost, C.stream));
     PMB_CUDA(cudaStreamSynchronize(C.stream));
+    return 0;
+}
+
+// The state of a solve that begins: the reduction counters start at zero. Not
+// when the workspace is bound, which has no stream to come after: what the
+// workspace's memory was used for before may still be running.
+static int csr_clear_state(Csr& C) {
+    PMB_CUDA(cudaMemsetAsync(C.ws + C.o_state, 0, sizeof(InstState), C.stream));
+    C.begun = true;
     return 0;
 }
 
@@ -2344,6 +2359,7 @@ static int csr_begin(Csr& C, const double* b, const double* x0, double atol, dou
                      int maxiter, int reorth) {
     C.reorth = reorth;
     cudaStream_t s = C.stream;
+    if (int rc = csr_clear_state(C)) return rc;
     csr_launch_init(csr_prec_kind(C), C.A, C.n, b, x0, C.v(kVx), C.v(kVr), C.v(kVz), C.invd,
                     C.state(), C.partials(), atol, rtol, maxiter, s);
     csr_internal_precond(C, s);
@@ -2391,9 +2407,7 @@ PMB_API int pmb_csr_bind(pmb_csr* p, void* workspace, double* vectors, const int
         C.h_state = reinterpret_cast<InstState*>(C.res.pin);
     }
     csr_drop_graph(C);
-    // Reduction counters must start at zero.
-    PMB_CUDA(cudaMemsetAsync(C.ws + C.o_state, 0, sizeof(InstState), C.stream));
-    PMB_CUDA(cudaStreamSynchronize(C.stream));
+    C.begun = false;
     return 0;
 }
 
@@ -2460,6 +2474,7 @@ PMB_API int pmb_csr_begin(pmb_csr* p, const double* b, const double* x0, double 
         if (!C.A.indptr) {
             // x0 is applied by the caller: r = b - A x0 arrives as b.
             CsrMat none{};
+            if (int rc = csr_clear_state(C)) return rc;
             csr_launch_init(csr_prec_kind(C), none, C.n, b, nullptr, C.v(kVx), C.v(kVr), C.v(kVz),
                             C.invd, C.state(), C.partials(), atol, rtol, maxiter, C.stream);
             C.reorth = reorthogonalize;
