@@ -1037,7 +1037,7 @@ static void run_vcycle(Stencil& S, const T* b0, T* z0, InstState* st, const T* d
         ++S.launches;
         prof_mark(S, l == 0 ? kPkDown0 : kPkDown);
     }
-    // Small levels of the images that have a tail, in one clustered launch.
+    // Small levels of the images that have a tail, a CTA each, in one launch.
     if (!S.tail_images.empty()) {
         launch_vc_tail<T>(S.at<TailDesc<T>>(S.o_tail), (int)S.tail_images.size(), S.tail_smem, st,
                           om, S.err(), s);
@@ -2431,7 +2431,8 @@ PMB_API int pmb_csr_set_ichol(pmb_csr* p, pmb_ichol* f, void* stream) {
 }
 
 // Full solve on the device (A as a matrix, preconditioner none / Jacobi /
-// matrix / ichol). Iterations replay a CUDA graph of 4 iterations.
+// matrix / ichol). Iterations are launched, or replay a CUDA graph of four
+// (kCsrGraphAfter).
 PMB_API int pmb_csr_solve(pmb_csr* p, const double* b, const double* x0, double* x_out, double atol,
                           double rtol, int maxiter, int reorthogonalize, void* stream) {
     if (!p || !b || !x_out) return fail(kErrArg, "pmb_csr_solve: bad arguments");

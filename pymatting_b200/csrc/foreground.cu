@@ -276,7 +276,6 @@ __device__ __forceinline__ int src_index(int v, int n_dst, int n_src) {
     return (int)min(s, (unsigned)(n_src - 1));
 }
 
-// grid: (ceil(Sp * 32 / 256), S); one thread per diagonal entry (k, s, j).
 __device__ __forceinline__ Coef coef_at(const float* __restrict__ alpha, int h0, int w0, float reg,
                                         float gw, const Level& L, int y, int x) {
     Coef c;

@@ -8,16 +8,24 @@
 //   _backsub_L_csc_inplace  :116-129  and  _backsub_LT_csc_inplace :132-145.
 //
 // The factorisation is inherently sequential over columns (column j needs
-// every column k < j that has a kept entry in row j). Instead of the
-// reference's left-looking linked lists, one CTA runs it right-looking over
-// a dense band "front": when column k is final, its kept entries update the
-// pending columns k+1 .. k+B directly (B = bandwidth of A; fill never leaves
-// the envelope). Per column, warp 0 does the serial part with warp ballots
-// (candidate rows, pivot, thresholding, compaction), then the whole CTA does
-// the pair updates while the last warp recycles the column's front slot:
-// two block barriers per column. Diagonal
-// updates happen in the same column order as the reference; the off-
-// diagonal accumulations differ only in summation order.
+// every column k < j that has a kept entry in row j). Three kernels make it,
+// with the reference's keep and discard rules, every update of an entry in
+// ascending k and one rounding each for product and difference, so their
+// factors are identical:
+//   k_ichol_factor_pipe     left-looking, a pipeline of the warps of one CTA:
+//                           bandwidths up to 1024 (below);
+//   k_ichol_factor_cluster  right-looking, the band front in a cluster's shared
+//                           memory: wide bands with long columns
+//                           (ichol_cluster.cu);
+//   k_ichol_factor          right-looking, the front in global memory, one CTA:
+//                           the widest bands. When column k is final, its kept
+//                           entries update the pending columns k+1 .. k+B
+//                           directly (B = bandwidth of A; fill never leaves
+//                           the envelope). Per column, warp 0 does the serial
+//                           part with warp ballots (candidate rows, pivot,
+//                           thresholding, compaction), then the whole CTA does
+//                           the pair updates while the last warp recycles the
+//                           column's front slot: two block barriers a column.
 //
 // The factor's dependency levels (level[i] = 1 + max level of the columns
 // that update row i) fall out of the factorisation for free and drive the
@@ -77,7 +85,7 @@ __device__ __forceinline__ void load_column(int64_t j, int64_t W, const int64_t*
     }
 }
 
-// The factorisation. One CTA. Front F / pat: W x W (W = B + 1), slot of
+// The front in global memory. One CTA. Front F / pat: W x W (W = B + 1), slot of
 // column j = j % W, entry (i, j) at offset i - j. cand / kept: scratch of
 // at least W entries each.
 __global__ void __launch_bounds__(kIcholThreads)

@@ -192,7 +192,7 @@ __global__ void k_lkm_finish(const double* __restrict__ image, const double* __r
 //               that enters and the row that leaves are read again (the
 //               second time from L1 or L2) instead of being kept.
 //   horizontal  the vertical sums of kRows rows lie in shared memory; each
-//               thread slides over an eighth of a row of one of the four.
+//               thread slides over a sixteenth of a row of one of the four.
 //   finish      a thread per output: window coefficients (brought in by
 //               asynchronous copies while the sums are made) or the pixel.
 //
@@ -201,7 +201,8 @@ __global__ void k_lkm_finish(const double* __restrict__ image, const double* __r
 //
 // What the pass-by-pass form spent its time on was memory: seven launches
 // moved 47 values per pixel, these move 27, of which 15 have to come from or
-// go to HBM. 1280x720, radius 10: 142 -> 75 us; 1920x1080: 261 -> 147 us. Bound
+// go to HBM. L2 flushed before, 1280x720, radius 10: 144 -> 75 us; 1920x1080:
+// 263 -> 148 us (back to back 142 -> 62 and 259 -> 135). Bound
 // by the latency of the row loads (24 warps per SM, long-scoreboard stalls;
 // LSU and DRAM pipes under 40 % busy).
 // ---------------------------------------------------------------------------

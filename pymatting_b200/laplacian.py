@@ -347,7 +347,9 @@ def knn_laplacian(image, n_neighbors=[20, 10], distance_weights=[2.0, 0.1], kern
     space (r, g, b, weight x, weight y) are found by an exact search on the
     device with the reference k-d tree's distance, keeping the k smallest by
     (distance, index); the reference resolves equal distances in its tree
-    order. Candidate tiles are pruned by their bounding boxes. W = sum of
+    order. A pixel that is not finite is infinitely far from every other: it
+    is in no finite pixel's list, and its own is the first k pixels. Candidate
+    tiles are pruned by their bounding boxes. W = sum of
     B + B^T (binary or soft weights), L = I - D^-1 W as canonical CSR on the
     device.
     """
