@@ -418,8 +418,9 @@ int pmb_ichol_kernel(const pmb_ichol* f);
 /* Polls after which the pipeline's waits give up (negative: the default, 2^22;
  * 0: at once), for the tests. */
 int pmb_ichol_wait_limit(pmb_ichol* f, int64_t polls);
-/* Device time (CUDA events on the factor's stream) of the factorisation
- * kernel in the last pmb_ichol_factor, in milliseconds; -1 before any. */
+/* Device time (CUDA events on the factor's stream) of the factorisation in the
+ * last pmb_ichol_factor, in milliseconds, a kernel that was given up for another
+ * one included; -1 before any. */
 float pmb_ichol_factor_ms(const pmb_ichol* f);
 /* Device pointers of the CSC factor (values, row indices, column pointers). */
 int pmb_ichol_factor_arrays(pmb_ichol* f, void** Lv, void** Lr, void** Lp);
